@@ -12,7 +12,7 @@
 #include <cstring>
 #include <vector>
 
-#include "qgb_common.cuh"
+#include "pauli_tiles.cuh"
 
 namespace qgb {
 
@@ -671,6 +671,16 @@ int pauli_expect_impl(const void* sv, int dtype, int n, const char* paulis, cons
     // and each group's slots must be contiguous: process terms in an order where
     // each launch covers a contiguous run of slots with a common X mask.
     double* partials = (double*)scratch;
+    if (!dm && nterms > 1) {
+        // many terms: X masks share a read of the state as far as they fit a tile
+        std::vector<PauliTerm> terms(nterms);
+        for (int t = 0; t < nterms; ++t) terms[t] = {ps[t].x, ps[t].z, ps[t].ny, t, coeff ? coeff[t] : 1.0};
+        int nblk = 0;
+        rc = pauli_tiles_expect(sv, dtype, n, terms.data(), nterms, batch, stride, red_blocks(nbits), partials, &nblk,
+                                st);
+        if (rc == QGB_OK) return finish(partials, nblk, nterms, batch, nullptr, out, st);
+        if (rc != QGB_EDECLINE) return rc;
+    }
     int t = 0;
     while (t < nterms) {
         PauliGroup g{};
@@ -889,6 +899,10 @@ extern "C" int qgb_pauli_apply(const void* sv, void* out, int dtype, int n, cons
     if (nterms < 1 || nterms > 128) return set_error(QGB_EINVAL, "1..128 terms supported (got %d)", nterms);
     std::vector<ParsedPauli> ps;
     if ((rc = parse_paulis(paulis, n, nterms, ps))) return rc;
+    std::vector<PauliTerm> terms(nterms);
+    for (int t = 0; t < nterms; ++t) terms[t] = {ps[t].x, ps[t].z, ps[t].ny, t, coeff[t]};
+    rc = pauli_tiles_apply(sv, out, dtype, n, terms.data(), nterms, batch, sv_stride, (cudaStream_t)stream);
+    if (rc != QGB_EDECLINE) return rc;
     PauliApplyArgs a{};
     a.n = n;
     a.nterms = nterms;

@@ -151,6 +151,199 @@ __global__ void __launch_bounds__(kRedThreads) pauli_group_kernel(const cplx<T>*
     block_reduce_store<NT>(acc.d, dst, nblk, g.nterms);
 }
 
+// Many diagonal terms (no X or Y) of a complex64 state in one pass, bit for bit
+// the sums of pauli_group_kernel: the same elements per thread in the same
+// order (grid-stride), the same chunks. That kernel spent the pass on the signs
+// (a popcount, a test and selects per term and element) and on spilled
+// accumulators. Here the 32 lanes hold the terms' masks: the warp's 32
+// consecutive elements share every index bit above the lane's, so one ballot per
+// element and warp gives all terms' signs of those bits, the lane's own part is
+// a constant word, and a term costs a shift, a sign flip and an add. float64 sums
+// live in shared memory (touched once per 256 elements). A block is reduced by a
+// transposing butterfly (31 float64 adds for 32 terms instead of 160: the FP64
+// pipe is narrow). 26 terms over 27 qubits: 3.75 -> 0.55 ms; 39 terms of 1024
+// 20-qubit states 74.6 -> 20.3 ms (bound by the block reductions: 16 elements a thread).
+template <int NT>
+__device__ __forceinline__ double warp_sums(double (&v)[NT], int lane) {
+    // NT a power of two up to 32: lane l ends with the sum of term l / (32 / NT)
+    if constexpr (NT == 1) {
+        double x = v[0];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        return x;
+    } else {
+#pragma unroll
+        for (int h = NT / 2, o = 16; h >= 1; h >>= 1, o >>= 1) {
+            const bool up = lane & o;
+#pragma unroll
+            for (int j = 0; j < h; ++j) {
+                const double keep = up ? v[j + h] : v[j], send = up ? v[j] : v[j + h];
+                v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+        }
+        double x = v[0];
+#pragma unroll
+        for (int o = 16 / NT; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        return x;
+    }
+}
+
+constexpr int pow2_above(int v) { return v <= 1 ? 1 : 2 * pow2_above((v + 1) / 2); }
+
+template <int NT, typename I>
+__global__ void __launch_bounds__(kRedThreads) pauli_diag_kernel(const float2* __restrict__ sv, int n, int64_t sv_stride,
+                                                                 const __grid_constant__ PauliGroup g, int nslots,
+                                                                 double* __restrict__ partials) {
+    constexpr int NP = pow2_above(NT), U = 4;
+    extern __shared__ double dsm[];  // [NT][kRedThreads]
+    __shared__ double red[kRedThreads / 32][NP];
+    const int64_t b = blockIdx.y;
+    const float2* s = sv + b * sv_stride;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const I stride = I(gridDim.x) * kRedThreads, len = I(1) << n;
+    const I zl = lane < g.nterms ? I(g.zmask[lane]) : I(0);
+    uint32_t lw = 0;  // bit j: parity of the lane's index bits & z_j
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+        const uint32_t bit = __ballot_sync(0xffffffffu, (zl >> q) & 1);
+        if ((lane >> q) & 1) lw ^= bit;
+    }
+    float f[NT], h[NT];
+#pragma unroll
+    for (int j = 0; j < NT; ++j) f[j] = h[j] = 0.0f;
+    int cnt = 0, cnt2 = 0;
+    bool deep = false;  // dsm holds sums
+    const I first = I(blockIdx.x) * kRedThreads + tid;
+    for (I x0 = first; x0 - lane < len; x0 += U * stride) {  // uniform over a warp
+        float2 a[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) a[u] = x0 + u * stride < len ? s[x0 + u * stride] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const I x = x0 + u * stride;
+            if (x - lane >= len) break;
+            const uint32_t sw = __ballot_sync(0xffffffffu, popc_any(I((x - lane) & zl)) & 1) ^ lw;
+            const float p = a[u].x * a[u].x + a[u].y * a[u].y;
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+                f[j] += __uint_as_float(__float_as_uint(p) ^ ((sw << (31 - j)) & 0x80000000u));
+            if (++cnt == kChunk) {
+                cnt = 0;
+#pragma unroll
+                for (int j = 0; j < NT; ++j) {
+                    h[j] += f[j];
+                    f[j] = 0.0f;
+                }
+                if (++cnt2 == kChunk) {
+                    cnt2 = 0;
+#pragma unroll
+                    for (int j = 0; j < NT; ++j) {
+                        const double d = deep ? dsm[j * kRedThreads + tid] : 0.0;
+                        dsm[j * kRedThreads + tid] = d + double(h[j]);
+                        h[j] = 0.0f;
+                    }
+                    deep = true;
+                }
+            }
+        }
+    }
+    double v[NP];
+#pragma unroll
+    for (int j = 0; j < NP; ++j) {
+        if (j < NT) {
+            h[j] += f[j];
+            v[j] = double(h[j]);
+            if (deep) v[j] += dsm[j * kRedThreads + tid];
+        } else {
+            v[j] = 0.0;
+        }
+    }
+    const double mine = warp_sums<NP>(v, lane);
+    if (lane % (32 / NP) == 0) red[warp][lane / (32 / NP)] = mine;
+    __syncthreads();
+    if (tid < g.nterms) {
+        double x = 0.0;
+        for (int w = 0; w < kRedThreads / 32; ++w) x += red[w][tid];
+        partials[(b * nslots + g.slot0 + tid) * int64_t(gridDim.x) + blockIdx.x] = x * g.coeff[tid];
+    }
+}
+
+// Several X masks (each of up to NT terms) of a complex64 state in one launch,
+// bit for bit the sums of pauli_group_kernel. The blocks of one index range are
+// neighbours in the grid, one per mask, so the masks read the state's window
+// together and all but the first find it in L2 (and a small state costs one
+// launch instead of one per mask): 27 masks over 27 qubits 4.15 -> 1.88 ms. One
+// thread walking 9 neighbouring bits with one load per pair and mask took 3.28 ms. The two members of a pair contribute equally:
+// 2 Re or 2 Im of conj(psi[y]) psi[x], with x's sign.
+struct PauliMini {
+    uint64_t xmask;
+    int slot0, nterms;
+    uint64_t zmask[4];
+    int ny[4];
+    double coeff[4];
+};
+constexpr int kMiniGroups = 36;
+struct PauliMinis {
+    PauliMini g[kMiniGroups];
+};
+
+template <int NT>
+__global__ void __launch_bounds__(kRedThreads) pauli_multi_kernel(const float2* __restrict__ sv, int n, int64_t sv_stride,
+                                                                  const __grid_constant__ PauliMinis gs, int ngroups,
+                                                                  int nblk, int nslots, double* __restrict__ partials) {
+    const int grp = int(blockIdx.x) % ngroups, blk = int(blockIdx.x) / ngroups;
+    const PauliMini& g = gs.g[grp];
+    const int64_t b = blockIdx.y;
+    const float2* s = sv + b * sv_stride;
+    Acc<float, NT> acc;
+    const uint32_t stride = uint32_t(nblk) * kRedThreads;
+    uint32_t zm[NT];
+    bool im[NT];
+    uint32_t neg[NT];
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+        zm[j] = j < g.nterms ? uint32_t(g.zmask[j]) : 0u;
+        const int ny = j < g.nterms ? g.ny[j] & 3 : 0;
+        im[j] = ny & 1;
+        neg[j] = uint32_t(ny == 1 || ny == 2) << 31;  // Re(i^ny v): Re, -Im, -Re, Im
+    }
+    constexpr int U = 4;
+    const int top = 63 - __clzll(g.xmask);
+    const uint32_t xm = uint32_t(g.xmask), lowm = (1u << top) - 1u;
+    const uint32_t half = 1u << (n - 1);
+    for (uint32_t i0 = uint32_t(blk) * kRedThreads + threadIdx.x; i0 < half; i0 += U * stride) {
+        float2 a[U], c[U];
+        uint32_t xs[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint32_t i = i0 + u * stride;
+            xs[u] = i + (i & ~lowm);
+            a[u] = c[u] = make_float2(0.f, 0.f);
+            if (i < half) {
+                a[u] = s[xs[u]];
+                c[u] = s[xs[u] ^ xm];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (i0 + u * stride >= half) break;
+            const float vr = c[u].x * a[u].x + c[u].y * a[u].y;
+            const float vi = c[u].x * a[u].y - c[u].y * a[u].x;
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+                const float t = im[j] ? vi : vr;
+                const uint32_t sg = (uint32_t(__popc(xs[u] & zm[j])) << 31) ^ neg[j];
+                acc.f[j] = fmaf(2.0f, __uint_as_float(__float_as_uint(t) ^ sg), acc.f[j]);
+            }
+            acc.step();
+        }
+    }
+    acc.flush();
+#pragma unroll
+    for (int j = 0; j < NT; ++j) acc.d[j] *= g.coeff[j < g.nterms ? j : 0];
+    block_reduce_store<NT>(acc.d, partials + (int64_t(b) * nslots + g.slot0) * nblk + blk, nblk, g.nterms);
+}
+
 // out[b * nslots + t] = coeff[t] * sum_blk partials[(b * nslots + t) * nblk + blk]
 __global__ void finish_kernel(const double* __restrict__ partials, int nblk, int nslots, int64_t batch,
                               const double* __restrict__ coeff, double* __restrict__ out) {
@@ -549,32 +742,114 @@ struct PauliApplyArgs {
     double coeff[128];
 };
 
-template <typename T>
-__global__ void __launch_bounds__(256) pauli_apply_kernel(const cplx<T>* __restrict__ sv, cplx<T>* __restrict__ out,
+__global__ void __launch_bounds__(256) pauli_apply_kernel(const double2* __restrict__ sv, double2* __restrict__ out,
                                                           int64_t stride, const __grid_constant__ PauliApplyArgs a) {
     const int64_t b = blockIdx.y;
-    const cplx<T>* s = sv + b * stride;
-    cplx<T>* o = out + b * stride;
+    const double2* s = sv + b * stride;
+    double2* o = out + b * stride;
     const uint64_t len = uint64_t(1) << a.n, step = uint64_t(gridDim.x) * blockDim.x;
-    // computed in the state's own precision (the sum is rounded to it anyway)
     for (uint64_t y = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; y < len; y += step) {
-        T ar = T(0), ai = T(0);
+        double ar = 0.0, ai = 0.0;
         for (int t = 0; t < a.nterms; ++t) {
             const uint64_t x = y ^ a.xmask[t];
-            const cplx<T> v = s[x];
+            const double2 v = s[x];
             // P|x> = i^ny (-1)^{pop(x & z)} |x ^ xmask> ; contribution to out[y]
-            T cr = v.x, ci = v.y;
+            double cr = v.x, ci = v.y;
             switch (a.ny[t] & 3) {
-                case 1: { T t2 = cr; cr = -ci; ci = t2; } break;
+                case 1: { double t2 = cr; cr = -ci; ci = t2; } break;
                 case 2: cr = -cr; ci = -ci; break;
-                case 3: { T t2 = cr; cr = ci; ci = -t2; } break;
+                case 3: { double t2 = cr; cr = ci; ci = -t2; } break;
                 default: break;
             }
-            const T f = T((__popcll(x & a.zmask[t]) & 1) ? -a.coeff[t] : a.coeff[t]);
+            const double f = ((__popcll(x & a.zmask[t]) & 1) ? -a.coeff[t] : a.coeff[t]);
             ar += f * cr;
             ai += f * ci;
         }
-        o[y] = mk<T>(ar, ai);
+        o[y] = make_double2(ar, ai);
+    }
+}
+
+// The same for complex64, bit for bit: each entry's terms in the given order, one
+// rounding per term. The general kernel spends most of its instructions per term
+// on signs and phases; here a warp works on 128 consecutive entries, 4 per lane,
+// the signs of 32 terms come from one ballot per 128 entries (the lane's and the
+// entry's index bits from constant words), a diagonal term reads the entry kept in
+// registers, and the uniform per-term work serves 4 entries. 39 terms on 64
+// 20-qubit states: 9.21 -> 1.22 ms.
+template <typename I>
+__global__ void __launch_bounds__(256) pauli_apply_f32_kernel(const float2* __restrict__ sv, float2* __restrict__ out,
+                                                              int64_t stride, const __grid_constant__ PauliApplyArgs a) {
+    constexpr int U = 4;
+    const int64_t b = blockIdx.y;
+    const float2* s = sv + b * stride;
+    float2* o = out + b * stride;
+    const int lane = threadIdx.x & 31;
+    const I len = I(1) << a.n;
+    const I warps = I(gridDim.x) * 8;
+    for (I w = I(blockIdx.x) * 8 + (threadIdx.x >> 5); w < (len + 127) / 128; w += warps) {
+        const I base = w * 128;
+        float2 v[U];
+        float ar[U], ai[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const I y = base + u * 32 + lane;
+            v[u] = y < len ? s[y] : make_float2(0.f, 0.f);
+            ar[u] = ai[u] = 0.0f;
+        }
+        for (int t0 = 0; t0 < a.nterms; t0 += 32) {
+            // lane j: term t0 + j's Z mask, and the parity of its X and Z masks (x = y ^ xmask)
+            const bool has = t0 + lane < a.nterms;
+            const I z = has ? I(a.zmask[t0 + lane]) : I(0), xz = has ? I(a.xmask[t0 + lane]) & z : I(0);
+            uint32_t sw = __ballot_sync(0xffffffffu, (popc_any(I(base & z)) ^ popc_any(xz)) & 1);
+#pragma unroll
+            for (int q = 0; q < 5; ++q) {
+                const uint32_t bit = __ballot_sync(0xffffffffu, (z >> q) & 1);
+                if ((lane >> q) & 1) sw ^= bit;
+            }
+            const uint32_t b5 = __ballot_sync(0xffffffffu, (z >> 5) & 1), b6 = __ballot_sync(0xffffffffu, (z >> 6) & 1);
+            const uint32_t su[U] = {sw, sw ^ b5, sw ^ b6, sw ^ b5 ^ b6};
+            const int tn = a.nterms - t0 < 32 ? a.nterms - t0 : 32;
+            for (int t = 0; t < tn; ++t) {
+                const I xm = I(a.xmask[t0 + t]);
+                const int ny = a.ny[t0 + t] & 3;
+                const float c0 = float(a.coeff[t0 + t]);
+                float2 x[U];
+                if (xm == 0) {
+#pragma unroll
+                    for (int u = 0; u < U; ++u) x[u] = v[u];
+                } else {
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const I y = base + u * 32 + lane;
+                        x[u] = y < len ? s[y ^ xm] : make_float2(0.f, 0.f);
+                    }
+                }
+                if (ny & 1) {  // i^ny v: i v = (-Im, Re), -i v = (Im, -Re)
+                    const uint32_t ns = ny == 3 ? 0x80000000u : 0u;
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const uint32_t sg = ((su[u] >> t) << 31) ^ ns;
+                        const float f = __uint_as_float(__float_as_uint(c0) ^ sg);
+                        ar[u] = fmaf(f, -x[u].y, ar[u]);
+                        ai[u] = fmaf(f, x[u].x, ai[u]);
+                    }
+                } else {
+                    const uint32_t ns = ny == 2 ? 0x80000000u : 0u;
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const uint32_t sg = ((su[u] >> t) << 31) ^ ns;
+                        const float f = __uint_as_float(__float_as_uint(c0) ^ sg);
+                        ar[u] = fmaf(f, x[u].x, ar[u]);
+                        ai[u] = fmaf(f, x[u].y, ai[u]);
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const I y = base + u * 32 + lane;
+            if (y < len) o[y] = make_float2(ar[u], ai[u]);
+        }
     }
 }
 
@@ -655,6 +930,48 @@ void launch_group_nt(const void* sv, int n, int64_t stride, const PauliGroup& g,
     else launch_group<T, 32>(sv, n, stride, g, nslots, partials, batch, dm, st);
 }
 
+template <int NT>
+int launch_diag(const void* sv, int n, int64_t stride, const PauliGroup& g, int nslots, double* partials, int64_t batch,
+                cudaStream_t st) {
+    // the float64 sums are used from 256 elements per thread on
+    constexpr size_t most = sizeof(double) * NT * kRedThreads;
+    const uint64_t per = (uint64_t(1) << n) / (uint64_t(red_blocks(n)) * kRedThreads) + 1;
+    const size_t smem = per >= kChunk * kChunk ? most : 0;
+    if (cudaFuncSetAttribute(pauli_diag_kernel<NT, uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most)) !=
+        cudaSuccess)
+        return check_launch("pauli diagonal attribute");
+    pauli_diag_kernel<NT, uint32_t><<<dim3(red_blocks(n), unsigned(batch)), kRedThreads, smem, st>>>(
+        (const float2*)sv, n, stride, g, nslots, partials);
+    return check_launch("pauli diagonal terms");
+}
+
+int launch_diag_nt(const void* sv, int n, int64_t stride, const PauliGroup& g, int nslots, double* partials,
+                   int64_t batch, cudaStream_t st) {
+    switch ((g.nterms + 3) / 4) {
+        case 1: return launch_diag<4>(sv, n, stride, g, nslots, partials, batch, st);
+        case 2: return launch_diag<8>(sv, n, stride, g, nslots, partials, batch, st);
+        case 3: return launch_diag<12>(sv, n, stride, g, nslots, partials, batch, st);
+        case 4: return launch_diag<16>(sv, n, stride, g, nslots, partials, batch, st);
+        case 5: return launch_diag<20>(sv, n, stride, g, nslots, partials, batch, st);
+        case 6: return launch_diag<24>(sv, n, stride, g, nslots, partials, batch, st);
+        case 7: return launch_diag<28>(sv, n, stride, g, nslots, partials, batch, st);
+        default: return launch_diag<32>(sv, n, stride, g, nslots, partials, batch, st);
+    }
+}
+
+int launch_multi(const void* sv, int n, int64_t stride, const PauliMinis& gs, int ngroups, int nt, int nslots,
+                 double* partials, int64_t batch, cudaStream_t st) {
+    const int nblk = red_blocks(n);
+    const dim3 grid(unsigned(nblk) * unsigned(ngroups), unsigned(batch));
+    if (nt <= 1)
+        pauli_multi_kernel<1><<<grid, kRedThreads, 0, st>>>((const float2*)sv, n, stride, gs, ngroups, nblk, nslots,
+                                                            partials);
+    else
+        pauli_multi_kernel<4><<<grid, kRedThreads, 0, st>>>((const float2*)sv, n, stride, gs, ngroups, nblk, nslots,
+                                                            partials);
+    return check_launch("pauli masks");
+}
+
 int pauli_expect_impl(const void* sv, int dtype, int n, const char* paulis, const double* coeff, int nterms,
                       int64_t batch, int64_t stride, double* out, void* scratch, size_t scratch_bytes, bool dm,
                       cudaStream_t st) {
@@ -682,6 +999,11 @@ int pauli_expect_impl(const void* sv, int dtype, int n, const char* paulis, cons
         if (rc != QGB_EDECLINE) return rc;
     }
     int t = 0;
+    // complex64 statevectors with 32-bit indices: the diagonal terms of a group and the X masks of
+    // up to 4 terms have kernels of their own; single terms and wide groups run in the general one
+    const bool fast = dtype == QGB_C64 && !dm && n <= 31 && nterms > 1;
+    PauliMinis minis[2];  // masks of one term, of up to four
+    int nmini[2] = {0, 0};
     while (t < nterms) {
         PauliGroup g{};
         g.xmask = ps[t].x;
@@ -694,10 +1016,36 @@ int pauli_expect_impl(const void* sv, int dtype, int n, const char* paulis, cons
             ++g.nterms;
             ++t;
         }
+        if (fast && g.xmask == 0 && g.nterms > 1) {
+            if ((rc = launch_diag_nt(sv, n, stride, g, nterms, partials, batch, st))) return rc;
+            continue;
+        }
+        if (fast && g.xmask != 0 && g.nterms <= 4) {
+            const int c = g.nterms > 1;
+            PauliMini& m = minis[c].g[nmini[c]++];
+            m.xmask = g.xmask;
+            m.slot0 = g.slot0;
+            m.nterms = g.nterms;
+            for (int j = 0; j < g.nterms; ++j) {
+                m.zmask[j] = g.zmask[j];
+                m.ny[j] = g.ny[j];
+                m.coeff[j] = g.coeff[j];
+            }
+            if (nmini[c] == kMiniGroups) {
+                if ((rc = launch_multi(sv, n, stride, minis[c], nmini[c], c ? 4 : 1, nterms, partials, batch, st)))
+                    return rc;
+                nmini[c] = 0;
+            }
+            continue;
+        }
         if (dtype == QGB_C64) launch_group_nt<float>(sv, n, stride, g, nterms, partials, batch, dm, st);
         else launch_group_nt<double>(sv, n, stride, g, nterms, partials, batch, dm, st);
         if ((rc = check_launch("pauli expectation"))) return rc;
     }
+    for (int c = 0; c < 2; ++c)
+        if (nmini[c] &&
+            (rc = launch_multi(sv, n, stride, minis[c], nmini[c], c ? 4 : 1, nterms, partials, batch, st)))
+            return rc;
     return finish(partials, red_blocks(nbits), nterms, batch, nullptr, out, st);
 }
 
@@ -916,10 +1264,18 @@ extern "C" int qgb_pauli_apply(const void* sv, void* out, int dtype, int n, cons
     const uint64_t len = uint64_t(1) << n;
     uint64_t bx = (len + 255) / 256;
     const uint64_t cap = uint64_t(sm_count()) * 8;
+    if (dtype == QGB_C64) {  // a warp takes 128 entries
+        bx = (len + 1023) / 1024;
+        dim3 grid(unsigned(bx < cap ? bx : cap), (unsigned)batch);
+        if (n <= 31)
+            pauli_apply_f32_kernel<uint32_t><<<grid, 256, 0, st>>>((const float2*)sv, (float2*)out, sv_stride, a);
+        else
+            pauli_apply_f32_kernel<uint64_t><<<grid, 256, 0, st>>>((const float2*)sv, (float2*)out, sv_stride, a);
+        return check_launch("pauli apply");
+    }
     if (bx > cap) bx = cap;
     dim3 grid((unsigned)bx, (unsigned)batch);
-    if (dtype == QGB_C64) pauli_apply_kernel<float><<<grid, 256, 0, st>>>((const float2*)sv, (float2*)out, sv_stride, a);
-    else pauli_apply_kernel<double><<<grid, 256, 0, st>>>((const double2*)sv, (double2*)out, sv_stride, a);
+     pauli_apply_kernel<<<grid, 256, 0, st>>>((const double2*)sv, (double2*)out, sv_stride, a);
     return check_launch("pauli apply");
 }
 

@@ -165,5 +165,8 @@ int sweep_status_read_clear();
 // complex128 tile sweeps in double-float arithmetic (sweep_df.cu); c128_arith() is
 // 1 when they are selected (the default), 0 for the float64 kernels.
 int c128_arith();
+// vectors of few tiles, each tile over a thread-block cluster (sweep_cluster.cu;
+// complex128 in double-float); QGB_EDECLINE when there are tiles for every SM
+int launch_sweep_cluster(int dtype, void* sv, const void* mats, const qgb::SweepArgs& a, int kmax, cudaStream_t st);
 int launch_sweep_df(void* sv, const void* mats, const qgb::SweepArgs& a, int kmax, cudaStream_t st);
 }  // namespace qgb_host

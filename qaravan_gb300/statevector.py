@@ -100,11 +100,10 @@ class StatevectorSim:
         self.dtype = dtype
         # auto: the autotuner's choice for this size and dtype (a cached measurement, a
         # measurement now with QGB_AUTOTUNE=1, else the defaults measured on GB300:
-        # complex64 -> dense fused blocks, one HBM pass each: 6-qubit blocks on the tensor
-        # cores from 13 qubits up (half the passes of 4-qubit blocks at the same speed per
-        # pass, fastest measured on the 28-qubit brickwork), 4-qubit blocks on the CUDA cores
-        # below; complex128 -> 3-qubit blocks grouped into shared-memory tile sweeps (float64
-        # arithmetic dominates, so fewer passes win))
+        # complex64 -> dense fused blocks, one HBM pass each, 6-qubit blocks on the tensor cores
+        # from 13 qubits up (half the passes of 4-qubit blocks at the same speed per pass, fastest
+        # measured on the 28-qubit brickwork), 4-qubit blocks in one tile sweep below; complex128 -> 3-qubit blocks grouped into tile sweeps
+        # (arithmetic dominates, so fewer passes win))
         if mode == "auto":
             from . import autotune
             a_mode, a_width, a_tile = autotune.choose_sv(circ.num_sites, dtype)

@@ -216,6 +216,37 @@ int qgb_op_action_scaled(void* sv, int dtype, int n, const int* indices, int k, 
  * (tensorQ/density_matrix_sim.py:85-89), without the division. */
 int qgb_dm_trace_factor(const void* rho, int dtype, int n, double* chain, int start, void* stream);
 
+/* One launch of a compiled plan on one vector (batch 1), see qgb_run_calls. */
+enum {
+    QGB_CALL_OP = 0,    /* qgb_op_action                                      */
+    QGB_CALL_CHAIN = 1, /* qgb_op_action_unitary_chain, chain link `link`     */
+    QGB_CALL_ROWS = 2,  /* qgb_op_action_unitary                              */
+    QGB_CALL_SCALED = 3, /* qgb_op_action_scaled by trace[1]                  */
+    QGB_CALL_TRACE = 4, /* qgb_dm_trace_factor on n / 2 sites, start = `link` */
+    QGB_CALL_SWEEP = 5  /* qgb_apply_sweep with `sweep`                       */
+};
+typedef struct {
+    int32_t kind;
+    int32_t k;                  /* op calls: width                                */
+    int32_t sites[QGB_MAX_K];   /* op calls: sites, as qgb_op_action's indices    */
+    int32_t link;
+    int32_t pad;
+    int64_t mat;                /* op calls: element offset of the matrix in mats */
+    const qgb_sweep* sweep;     /* sweep calls                                    */
+} qgb_call;
+
+/* The calls of a plan in order, each as its own entry point would run it on the
+ * vector `sv` of n bits (one host call per plan instead of one per launch).
+ * Passes over the whole vector alternate between ascending and descending tile
+ * order, so that a pass begins with what the previous one left in L2. `chain`
+ * (6 doubles) and `trace` (3 doubles) may be null when no call uses them.
+ * Stops at the first failing call. Replaces the per-gate loop of BaseSim.run
+ * (core/base_sim.py:30-53). */
+int qgb_run_calls(void* sv, int dtype, int n, const qgb_call* calls, int ncalls, const void* mats, double* chain,
+                  double* trace, void* stream);
+size_t qgb_call_bytes(void);
+
+
 /* A fused pass (several gates per read+write of the state), planned by the
  * host compiler from a Circuit's gate list (core/base_sim.py:30-53 loop). */
 int qgb_apply_sweep(void* sv, int dtype, int n, const qgb_sweep* sweep, const void* mats,

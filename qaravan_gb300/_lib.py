@@ -69,6 +69,22 @@ class AdjointSweep(C.Structure):
     ]
 
 
+QGB_CALL_OP, QGB_CALL_CHAIN, QGB_CALL_ROWS, QGB_CALL_SCALED, QGB_CALL_TRACE, QGB_CALL_SWEEP = range(6)
+
+
+class Call(C.Structure):
+    """Mirror of ``qgb_call``."""
+    _fields_ = [
+        ("kind", C.c_int32),
+        ("k", C.c_int32),
+        ("sites", C.c_int32 * QGB_MAX_K),
+        ("link", C.c_int32),
+        ("pad", C.c_int32),
+        ("mat", C.c_int64),
+        ("sweep", C.POINTER(Sweep)),
+    ]
+
+
 _vp, _i, _i64, _u64, _sz, _dp, _cp, _ip = (C.c_void_p, C.c_int, C.c_int64, C.c_uint64, C.c_size_t,
                                            C.POINTER(C.c_double), C.c_char_p, C.POINTER(C.c_int))
 
@@ -83,6 +99,8 @@ SIGNATURES = {
     "qgb_op_action_unitary": (C.c_int, [_vp, _i, _i, _ip, _i, _vp, _i64, _i64, _i64, _vp]),
     "qgb_op_action_unitary_chain": (C.c_int, [_vp, _i, _i, _ip, _i, _vp, _i64, _i64, _i64, _vp, _i, _vp]),
     "qgb_op_action_scaled": (C.c_int, [_vp, _i, _i, _ip, _i, _vp, _vp, _vp]),
+    "qgb_run_calls": (C.c_int, [_vp, _i, _i, C.POINTER(Call), _i, _vp, _vp, _vp, _vp]),
+    "qgb_call_bytes": (C.c_size_t, []),
     "qgb_dm_trace_factor": (C.c_int, [_vp, _i, _i, _vp, _i, _vp]),
     "qgb_apply_sweep": (C.c_int, [_vp, _i, _i, C.POINTER(Sweep), _vp, _i64, _i64, _i64, _vp]),
     "qgb_set_sweep_impl": (C.c_int, [_i]),

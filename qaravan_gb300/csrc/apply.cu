@@ -235,7 +235,8 @@ namespace qgb_host {
 // j is out_bits[j] (same set of bits) to `batch` vectors of 2^nbits entries.
 int apply_dense_bits(void* sv, int dtype, int nbits, const int* in_bits, const int* out_bits, int k,
                      const void* op, int64_t op_stride, int64_t batch, int64_t sv_stride, cudaStream_t st,
-                     int unitary = 0, double* chain = nullptr, int link = 0, const double* scale = nullptr) {
+                     int unitary = 0, double* chain = nullptr, int link = 0, const double* scale = nullptr,
+                     int reverse = 0) {
     if (!sv || !op) return set_error(QGB_EINVAL, "null state or operator pointer");
     if (dtype != QGB_C64 && dtype != QGB_C128) return set_error(QGB_EINVAL, "dtype %d unknown", dtype);
     if (k < 1 || k > QGB_MAX_K) return set_error(QGB_EINVAL, "gate width k=%d not in [1, %d]", k, QGB_MAX_K);
@@ -277,7 +278,7 @@ int apply_dense_bits(void* sv, int dtype, int nbits, const int* in_bits, const i
     if (unitary == 2) {
         if (dtype == QGB_C64) {
             const int rc = try_dense_tc(sv, op, nbits, a.sorted, in_bits, out_bits, k, op_stride, batch, sv_stride, 2,
-                                        st, chain, link);
+                                        st, chain, link, nullptr, reverse);
             if (rc != QGB_EDECLINE) return rc;
         }
         // not on the chain kernel: clear the chain, so that the next pass starts a new one
@@ -286,7 +287,7 @@ int apply_dense_bits(void* sv, int dtype, int nbits, const int* in_bits, const i
     }
     if (dtype == QGB_C64) {
         const int rc = try_dense_tc(sv, op, nbits, a.sorted, in_bits, out_bits, k, op_stride, batch, sv_stride,
-                                    unitary, st, nullptr, 0, scale);
+                                    unitary, st, nullptr, 0, scale, reverse);
         if (rc != QGB_EDECLINE) return rc;
     }
     const int rc = dtype == QGB_C64 ? dispatch_dense<float>(sv, op, a, st) : dispatch_dense<double>(sv, op, a, st);
@@ -300,7 +301,8 @@ int apply_dense_bits(void* sv, int dtype, int nbits, const int* in_bits, const i
 namespace {
 
 int op_action(void* sv, int dtype, int n, const int* indices, int k, const void* op, int64_t op_stride,
-              int64_t batch, int64_t sv_stride, void* stream, int unitary, double* chain = nullptr, int link = 0) {
+              int64_t batch, int64_t sv_stride, void* stream, int unitary, double* chain = nullptr, int link = 0,
+              const double* scale = nullptr, int reverse = 0) {
     if (n < 1 || n > QGB_MAX_QUBITS) return set_error(QGB_EINVAL, "n=%d not in [1, %d]", n, QGB_MAX_QUBITS);
     if (!indices) return set_error(QGB_EINVAL, "null indices");
     if (k < 1 || k > QGB_MAX_K) return set_error(QGB_EINVAL, "gate width k=%d not in [1, %d]", k, QGB_MAX_K);
@@ -310,7 +312,7 @@ int op_action(void* sv, int dtype, int n, const int* indices, int k, const void*
         bits[j] = n - 1 - indices[j];
     }
     return apply_dense_bits(sv, dtype, n, bits, bits, k, op, op_stride, batch, sv_stride, (cudaStream_t)stream,
-                            unitary, chain, link);
+                            unitary, chain, link, scale, reverse);
 }
 
 }  // namespace
@@ -338,15 +340,51 @@ extern "C" int qgb_op_action_scaled(void* sv, int dtype, int n, const int* indic
                                     const double* factor, void* stream) {
     if (!factor || (reinterpret_cast<uintptr_t>(factor) % sizeof(double)))
         return set_error(QGB_EINVAL, "factor missing or not 8-byte aligned");
-    if (n < 1 || n > QGB_MAX_QUBITS) return set_error(QGB_EINVAL, "n=%d not in [1, %d]", n, QGB_MAX_QUBITS);
-    if (!indices) return set_error(QGB_EINVAL, "null indices");
-    if (k < 1 || k > QGB_MAX_K) return set_error(QGB_EINVAL, "gate width k=%d not in [1, %d]", k, QGB_MAX_K);
-    int bits[QGB_MAX_K];
-    for (int j = 0; j < k; ++j) {
-        if (indices[j] < 0 || indices[j] >= n) return set_error(QGB_EINVAL, "site %d out of range for n=%d", indices[j], n);
-        bits[j] = n - 1 - indices[j];
+    return op_action(sv, dtype, n, indices, k, op, 0, 1, 0, stream, 0, nullptr, 0, factor);
+}
+
+extern "C" size_t qgb_call_bytes(void) { return sizeof(qgb_call); }
+
+extern "C" int qgb_run_calls(void* sv, int dtype, int n, const qgb_call* calls, int ncalls, const void* mats,
+                             double* chain, double* trace, void* stream) {
+    if (ncalls < 0 || (ncalls > 0 && (!calls || !mats))) return set_error(QGB_EINVAL, "null calls or matrices");
+    if (dtype != QGB_C64 && dtype != QGB_C128) return set_error(QGB_EINVAL, "dtype %d unknown", dtype);
+    const size_t esz = dtype == QGB_C64 ? 8 : 16;
+    if ((reinterpret_cast<uintptr_t>(chain) | reinterpret_cast<uintptr_t>(trace)) % sizeof(double))
+        return set_error(QGB_EINVAL, "chain or trace buffer not 8-byte aligned");
+    int passes = 0;  // over the whole vector
+    for (int i = 0; i < ncalls; ++i) {
+        const qgb_call& c = calls[i];
+        const char* op = static_cast<const char*>(mats) + c.mat * int64_t(esz);
+        if (c.kind <= QGB_CALL_SCALED && c.mat < 0) return set_error(QGB_EINVAL, "call %d: negative matrix offset", i);
+        if (c.kind == QGB_CALL_CHAIN && (!chain || c.link < 0))
+            return set_error(QGB_EINVAL, "call %d: norm chain buffer missing or negative link", i);
+        if ((c.kind == QGB_CALL_SCALED || c.kind == QGB_CALL_TRACE) && !trace)
+            return set_error(QGB_EINVAL, "call %d: trace buffer missing", i);
+        int rc;
+        switch (c.kind) {
+            case QGB_CALL_OP:
+                rc = op_action(sv, dtype, n, c.sites, c.k, op, 0, 1, 0, stream, 0, nullptr, 0, nullptr, passes++ & 1);
+                break;
+            case QGB_CALL_CHAIN:
+                rc = op_action(sv, dtype, n, c.sites, c.k, op, 0, 1, 0, stream, 2, chain, c.link, nullptr, passes++ & 1);
+                break;
+            case QGB_CALL_ROWS:
+                rc = op_action(sv, dtype, n, c.sites, c.k, op, 0, 1, 0, stream, 1, nullptr, 0, nullptr, passes++ & 1);
+                break;
+            case QGB_CALL_SCALED:
+                rc = op_action(sv, dtype, n, c.sites, c.k, op, 0, 1, 0, stream, 0, nullptr, 0, trace + 1, passes++ & 1);
+                break;
+            case QGB_CALL_TRACE: rc = qgb_dm_trace_factor(sv, dtype, n / 2, trace, c.link, stream); break;
+            case QGB_CALL_SWEEP:
+                rc = qgb_apply_sweep(sv, dtype, n, c.sweep, mats, 0, 1, 0, stream);
+                ++passes;
+                break;
+            default: return set_error(QGB_EINVAL, "call %d: kind %d unknown", i, c.kind);
+        }
+        if (rc) return rc;
     }
-    return apply_dense_bits(sv, dtype, n, bits, bits, k, op, 0, 1, 0, (cudaStream_t)stream, 0, nullptr, 0, factor);
+    return QGB_OK;
 }
 
 extern "C" int qgb_dm_apply_superop(void* rho, int dtype, int n, const int* indices, int k, const void* superop,

@@ -99,6 +99,16 @@ __global__ void __launch_bounds__(kTcThreads, 1) dense_tc_kernel(float2* __restr
     __shared__ double chain_red[8][2];        // per data warp: squared norms of its inputs and outputs (MODE 2)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int q = warp & 3, h = (warp >> 2) & 1;
+    // Programmatic dependent launch: this grid may start while the previous pass still runs, its
+    // operator built and its tensor memory claimed by the time that pass has finished (64 tiles of
+    // 19 qubits: 11.7 -> 8.8 us a pass). Nothing that a previous kernel may write -- the state, the chain, the
+    // factor -- is touched before tc_grid_wait, and the next grid is let in only after it, so
+    // that everything before the previous pass (the kernel that wrote the operator) is complete.
+    const bool scalars = (MODE == 0 && (a.scale != nullptr || a.chain != nullptr)) || (MODE == 2 && a.c_head);
+    if (scalars) {
+        tc_grid_wait();
+        tc_grid_next();
+    }
     // MODE 2, the pass that opens an epoch: it starts the chain (measures its input)
     // unless the previous epoch left a reference and an output norm; its matrix is
     // scaled by 1 + gcorr = sqrt(ref / out_prev)
@@ -176,10 +186,16 @@ __global__ void __launch_bounds__(kTcThreads, 1) dense_tc_kernel(float2* __restr
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (!scalars) {
+        tc_grid_wait();
+        tc_grid_next();
+    }
     const uint32_t tmem = tmem_slot;
-    const uint64_t step = gridDim.x;
-    const uint64_t t0 = blockIdx.x;  // the grid never exceeds the tile count
-    const uint64_t ntiles = (a.tiles - t0 + step - 1) / step;
+    // tiles blockIdx.x + k * gridDim.x (the grid never exceeds the tile count), or as many from the end
+    const uint64_t ntiles = (a.tiles - blockIdx.x + gridDim.x - 1) / gridDim.x;
+    const uint64_t t0 = a.reverse ? a.tiles - 1 - blockIdx.x : blockIdx.x;
+    const uint64_t step = a.reverse ? 0 - uint64_t(gridDim.x) : uint64_t(gridDim.x);
+    const int per_state = __ffsll(a.tiles_per_state) - 1;  // a power of two
 
     if (warp == 8) {
         // ---- MMA warp: one thread issues, in tile order, on alternating buffer pairs.
@@ -231,7 +247,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) dense_tc_kernel(float2* __restr
         const uint32_t sctid = tile_swz(ctid);
         const uint64_t gctid = uint64_t(ctid & runmask) + a.hoff[ctid >> a.L];
         auto tile_base = [&](uint64_t t) -> float2* {
-            const uint64_t b = t / a.tiles_per_state, tt = t - b * a.tiles_per_state;
+            const uint64_t b = t >> per_state, tt = t & (a.tiles_per_state - 1);
             return sv + int64_t(b) * a.sv_stride + insert_zeros(tt, a.tile_bits, 13);
         };
         auto issue_load = [&](uint64_t t, int pb) {
@@ -347,6 +363,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) dense_tc_kernel(float2* __restr
                 const bool one = su >= 1.17549435e-38f && su <= 1.0e38f;
                 float y[D];
                 tmem_ld_row<D>(acc, y);
+                unsigned long long ss[4] = {0ull, 0ull, 0ull, 0ull};  // squares of the row, 8 interleaved sums
 #pragma unroll
                 for (int c0 = 0; c0 < D; c0 += 16) {
                     float* r = y + c0;
@@ -358,9 +375,20 @@ __global__ void __launch_bounds__(kTcThreads, 1) dense_tc_kernel(float2* __restr
 #pragma unroll
                         for (int e = 0; e < 16; ++e) r[e] = (r[e] * wunscale) * u;
                     }
-                    if constexpr (MODE == 2)
-                        if (a.c_tail) f_out += sumsq8<16>(r);
+                    if constexpr (MODE == 2) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            const unsigned long long v = f2pack(r[2 * e], r[2 * e + 1]);
+                            ss[e & 3] = f2fma(v, v, ss[e & 3]);
+                        }
+                    }
                     put16(p, c0, r);
+                }
+                if constexpr (MODE == 2) {
+                    float t[8];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) f2unpack(ss[j], t[2 * j], t[2 * j + 1]);
+                    f_out += ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
                 }
             }
             if constexpr (MODE == 2) {
@@ -541,6 +569,14 @@ using namespace qgb;
 
 namespace {
 
+// Programmatic launch up to this many tiles: us per pass with and without, 19 qubits (64 tiles) 8.8 /
+// 11.6, 20 qubits 11.1 / 11.9, 22 qubits (512) 19.6 / 20.4, 23 qubits 31.5 / 30.8, 24 qubits 61.0 / 54.9
+// (CTAs then start in the order the previous pass's leave, which costs L2 hits).
+constexpr uint64_t kPdlTiles = 512;
+// Descending passes up to this many tiles (states of up to 256 MB, twice L2): 24 qubits 57.1 -> 54.9 us
+// a pass; 28 qubits lose 0.7 %.
+constexpr uint64_t kReverseTiles = 4096;
+
 int g_dense_impl = -1;  // -1: not read yet; 0: CUDA cores only; 1: tensor cores for k = 5, 6; 2: also k = 4
 
 int dense_impl() {
@@ -570,7 +606,17 @@ int launch_tc(float2* sv, const float2* op, const TcArgs& a, cudaStream_t st) {
     }
     const uint64_t cap = uint64_t(qgb_host::sm_count()) * uint64_t(per_sm);
     const unsigned grid = unsigned(a.tiles < cap ? a.tiles : cap);
-    dense_tc_kernel<K, MODE><<<grid, kTcThreads, G::SMEM, st>>>(sv, op, a);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kTcThreads);
+    cfg.dynamicSmemBytes = G::SMEM;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = a.tiles <= kPdlTiles ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, dense_tc_kernel<K, MODE>, sv, op, a);
     return qgb_host::check_launch("dense_tc kernel");
 }
 
@@ -612,11 +658,17 @@ int build_tc_args(TcArgs& a, int nbits, const int* sorted, const int* in_bits, c
     }
     for (int j = 0; j < D / 2; ++j) a.off[j] = scat[j];
     a.hstride = uint64_t(1) << sorted[k - 1];
-    for (int c = 0; c < D; ++c) {
-        const uint64_t oi = matrix_offset(c, in_bits, k), oo = matrix_offset(c, out_bits, k);
-        for (int j = 0; j < D; ++j) {
-            if (scat[j] == oi) a.perm_in[j] = c;
-            if (scat[j] == oo) a.perm_out[j] = c;
+    // memory-order component j -> matrix column / row, bit by bit
+    a.perm_in[0] = a.perm_out[0] = 0;
+    for (int i = 0; i < k; ++i) {
+        int ci = 0, co = 0;
+        for (int j = 0; j < k; ++j) {
+            if (in_bits[j] == sorted[i]) ci = 1 << (k - 1 - j);
+            if (out_bits[j] == sorted[i]) co = 1 << (k - 1 - j);
+        }
+        for (int j = 0; j < (1 << i); ++j) {
+            a.perm_in[j | (1 << i)] = a.perm_in[j] | ci;
+            a.perm_out[j | (1 << i)] = a.perm_out[j] | co;
         }
     }
     a.vec2 = sorted[0] == 0 ? 1 : 0;
@@ -672,7 +724,7 @@ int build_tc_args(TcArgs& a, int nbits, const int* sorted, const int* in_bits, c
 // CUDA-core kernel instead.
 int try_dense_tc(void* sv, const void* op, int nbits, const int* sorted, const int* in_bits, const int* out_bits,
                  int k, int64_t op_stride, int64_t batch, int64_t sv_stride, int unitary, cudaStream_t st,
-                 double* chain, int link, const double* scale) {
+                 double* chain, int link, const double* scale, int reverse) {
     const int mode = dense_impl();
     if (scale && unitary != 0) return QGB_EDECLINE;  // a factor goes with plain (MODE 0) passes only
     if (unitary == 2 && (batch > 1 || !chain)) return QGB_EDECLINE;  // the chain follows one state
@@ -687,6 +739,7 @@ int try_dense_tc(void* sv, const void* op, int nbits, const int* sorted, const i
         if (rc != QGB_OK) return rc;
     }
     a.scale = scale;
+    a.reverse = reverse && a.tiles <= kReverseTiles;
     float2* s = static_cast<float2*>(sv);
     const float2* m = static_cast<const float2*>(op);
     if (unitary == 2) {

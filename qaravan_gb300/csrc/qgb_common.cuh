@@ -199,7 +199,7 @@ int sm_count();
 constexpr int QGB_EDECLINE = 1000;
 int try_dense_tc(void* sv, const void* op, int nbits, const int* sorted, const int* in_bits, const int* out_bits,
                  int k, int64_t op_stride, int64_t batch, int64_t sv_stride, int unitary, cudaStream_t st,
-                 double* chain = nullptr, int link = 0, const double* scale = nullptr);
+                 double* chain = nullptr, int link = 0, const double* scale = nullptr, int reverse = 0);
 int tc_status_read_clear();
 int tcs_status_read_clear();
 int dmb_status_read_clear();

@@ -39,6 +39,7 @@ struct TcArgs {
     const double* scale;                 // MODE 0: device factor f, the op applied is f * M (null: 1)
     int c_prev, c_cur, c_next;           // slots of the previous epoch, this epoch, the next epoch (-1: none)
     int c_head, c_tail;                  // this pass opens its epoch (corrects) / closes it (measures its output)
+    int reverse;                         // tiles in descending order
 };
 
 template <int K> struct TcGeom {
@@ -58,6 +59,12 @@ template <int K> struct TcGeom {
     static_assert(R >= 32 && R <= 256 && (R % 16) == 0, "MMA N out of range");
     static_assert(NCOLS == 512, "tensor memory holds 512 columns");
 };
+
+// Programmatic dependent launch: waits until the grids this one depends on have
+// finished and their writes are visible (returns at once in an ordinary launch);
+// lets the next grid in the stream begin.
+__device__ __forceinline__ void tc_grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void tc_grid_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t tc_smem_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
 

@@ -158,6 +158,7 @@ class Executor:
                     raise NotImplementedError("Pauli channels of more than 128 terms")
                 strings = "".join(t[1].lower() for t in s.terms).encode()
                 self._steps.append(("pauli_mix", strings, _lib.double_array([t[0] for t in s.terms]), len(s.terms)))
+        self._calls: dict = {}  # (norm mode, trace chain) -> the plan's launches for qgb_run_calls
         self.scratch = Scratch(self.device)
         self.norm = torch.empty(1, dtype=torch.float64, device=self.device)
         self.launches = 0
@@ -245,14 +246,14 @@ class Executor:
         nb = self.plan.nbits
         st = _lib.stream_ptr(state.device)
         ptr = state.data_ptr()
+        if batch == 1 and mats is None and events is None and all(s[0] in ("dense", "sweep") for s in self._steps):
+            return self._run_calls(state, L, ptr, st)
         mats = self.mats if mats is None else mats
         mptr = mats.data_ptr()
         launches = 0
         link = 0  # position in the current norm chain of consecutive unitary blocks
         # trace chain: one complex64 density matrix whose ops keep the trace
-        tchain = (_TRACE_CHAIN and self.normalize_kind == "dm" and self.code == _lib.QGB_C64 and batch == 1
-                  and mats is self.mats and self.plan.trace_kept
-                  and any(s[0] == "dense" and s[6] for s in self._steps))
+        tchain = batch == 1 and mats is self.mats and self._trace_chained()
         if tchain:
             if getattr(self, "_tchain", None) is None:
                 self._tchain = torch.zeros(4, dtype=torch.float64, device=self.device)
@@ -340,6 +341,71 @@ class Executor:
                 e1.record()
                 events.append((s[0], e0, e1))
         self.launches = launches
+        return state
+
+    def _trace_chained(self):
+        """Whether one vector of this plan runs the trace chain: a complex64 density
+        matrix whose ops keep the trace, with passes on the tensor cores."""
+        return (_TRACE_CHAIN and self.normalize_kind == "dm" and self.code == _lib.QGB_C64 and self.plan.trace_kept
+                and any(s[0] == "dense" and s[6] for s in self._steps))
+
+    def _call_list(self, mode, tchain):
+        """The plan's launches on one vector as one array for ``qgb_run_calls``: the
+        entries, chain links and trace measurements that ``run`` takes step by step."""
+        calls, link, t_since, t_pending = [], 0, 0, False
+        if tchain:
+            calls.append((_lib.QGB_CALL_TRACE, None, 0, 1, 0, None))
+        for s in self._steps:
+            if s[0] == "sweep":
+                calls.append((_lib.QGB_CALL_SWEEP, None, 0, 0, 0, s[1]))
+                link = 0
+                continue
+            _, sites, k, off, unitary, whole, on_tc = s
+            if tchain:
+                scaled = on_tc and t_pending
+                calls.append((_lib.QGB_CALL_SCALED if scaled else _lib.QGB_CALL_OP, sites, k, 0, off, None))
+                t_pending = t_pending and not scaled
+                t_since += int(on_tc)
+                if whole and t_since >= _TRACE_EPOCH:
+                    calls.append((_lib.QGB_CALL_TRACE, None, 0, 0, 0, None))
+                    t_since, t_pending = 0, True
+            elif unitary and mode == "chain":
+                calls.append((_lib.QGB_CALL_CHAIN, sites, k, link, off, None))
+                link += 1
+            else:
+                calls.append((_lib.QGB_CALL_ROWS if unitary and mode == "row" else _lib.QGB_CALL_OP, sites, k, 0, off,
+                              None))
+                link = 0
+        arr = (_lib.Call * max(len(calls), 1))()
+        for c, (kind, sites, k, ln, off, sweep) in zip(arr, calls):
+            c.kind, c.k, c.link, c.mat = kind, k, ln, off
+            for j in range(k):
+                c.sites[j] = sites[j]
+            if sweep is not None:
+                c.sweep = C.pointer(sweep)
+        return arr, len(calls)
+
+    def _run_calls(self, state, L, ptr, st):
+        tchain = self._trace_chained()
+        key = (_NORM_RESTORE, tchain)
+        hit = self._calls.get(key)
+        if hit is None:
+            if L.qgb_call_bytes() != C.sizeof(_lib.Call):
+                raise _lib.QgbError("call table layout mismatch with the library")
+            hit = self._calls[key] = self._call_list(*key)
+        arr, count = hit
+        chain = trace = None
+        if tchain:
+            if getattr(self, "_tchain", None) is None:
+                self._tchain = torch.zeros(4, dtype=torch.float64, device=self.device)
+            trace = self._tchain.data_ptr()
+        elif _NORM_RESTORE == "chain":
+            if getattr(self, "_chain", None) is None:
+                self._chain = torch.zeros(6, dtype=torch.float64, device=self.device)
+            chain = self._chain.data_ptr()
+        _lib.check(L.qgb_run_calls(ptr, self.code, self.plan.nbits, arr, count, self.mats.data_ptr(), chain, trace,
+                                   st), "run_calls")
+        self.launches = count
         return state
 
     def normalize(self, state, batch=1, stride=0):

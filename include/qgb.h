@@ -230,7 +230,9 @@ typedef struct {
     int32_t k;                  /* op calls: width                                */
     int32_t sites[QGB_MAX_K];   /* op calls: sites, as qgb_op_action's indices    */
     int32_t link;
-    int32_t pad;
+    int32_t first;              /* chain calls: passes of the chain's first epoch (0: 4), so
+                                   that a caller who knows the chain's length can let its last
+                                   pass open an epoch and correct the norm once more         */
     int64_t mat;                /* op calls: element offset of the matrix in mats */
     const qgb_sweep* sweep;     /* sweep calls                                    */
 } qgb_call;

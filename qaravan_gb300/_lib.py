@@ -79,7 +79,7 @@ class Call(C.Structure):
         ("k", C.c_int32),
         ("sites", C.c_int32 * QGB_MAX_K),
         ("link", C.c_int32),
-        ("pad", C.c_int32),
+        ("first", C.c_int32),
         ("mat", C.c_int64),
         ("sweep", C.POINTER(Sweep)),
     ]

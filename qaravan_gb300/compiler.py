@@ -250,6 +250,106 @@ def fuse_symbolic(ops, width):
     return [b for b in blocks if b is not None]
 
 
+def fuse_frontier(ops, width):
+    """Fusion into few blocks: while ops are left, every op whose predecessors are
+    all done grows a bit set up to ``width`` bits, each time by the bits of a next
+    op that let the set take the most further multi-bit ops per added bit, and the
+    best set becomes a block with every op it can take in order. A block of a
+    brickwork circuit is then a rhombus of 9 two-qubit gates on 6 bits, where the
+    order-driven :func:`fuse_symbolic` leaves staircases of 7 or 8. Same result type;
+    the blocks are a linear extension of the ops' order."""
+    N = len(ops)
+    obits = [tuple(op.bits) for op in ops]
+    queue: dict = {}  # bit -> its ops in order
+    for i, bits in enumerate(obits):
+        if len(bits) > width:
+            raise ValueError(f"op on {len(bits)} bits exceeds fusion width {width}")
+        for b in bits:
+            queue.setdefault(b, []).append(i)
+    for qb in queue.values():
+        qb.append(-1)  # no further op
+    head = dict.fromkeys(queue, 0)
+    weight = [1.0 if len(b) > 1 else 1e-3 for b in obits]
+
+    def take(bits, pos, got):
+        """Continues the in-order application on ``bits`` from ``pos`` (updated);
+        appends the ops taken to ``got`` and returns their weight."""
+        total, work = 0.0, list(bits)
+        while work:
+            b = work.pop()
+            while True:
+                i = queue[b][pos[b]]
+                if i < 0:
+                    break
+                ib = obits[i]
+                ok = True
+                for y in ib:
+                    if y not in pos or queue[y][pos[y]] != i:
+                        ok = False
+                        break
+                if not ok:
+                    break
+                got.append(i)
+                total += weight[i]
+                for y in ib:
+                    pos[y] += 1
+                    if y != b and y not in work:
+                        work.append(y)
+        return total
+
+    def grow(start):
+        pos = {b: head[b] for b in obits[start]}
+        got: list = []
+        total = take(obits[start], pos, got)
+        seen = set(pos)
+        while len(pos) < width:
+            best = None
+            tried = set()
+            for b in sorted(pos):
+                i = queue[b][pos[b]]
+                if i < 0:
+                    continue
+                ext = tuple(sorted(y for y in obits[i] if y not in pos))
+                if not ext or len(pos) + len(ext) > width or ext in tried:
+                    continue
+                tried.add(ext)
+                seen.update(ext)
+                p2 = dict(pos)
+                for y in ext:
+                    p2[y] = head[y]
+                g2: list = []
+                gain = take(list(p2), p2, g2) / len(ext)
+                if best is None or gain > best[0]:
+                    best = (gain, p2, g2)
+            if best is None:
+                break
+            total += best[0] * (len(best[1]) - len(pos))
+            pos = best[1]
+            got += best[2]
+        return total, pos, got, seen
+
+    cache: dict = {}  # start op -> its grown set, while nothing it looked at has moved
+    blocks, done = [], 0
+    while done < N:
+        best = None
+        for b in queue:
+            i = queue[b][head[b]]
+            if i < 0 or obits[i][0] != b or any(queue[y][head[y]] != i for y in obits[i]):
+                continue
+            hit = cache.get(i)
+            if hit is None:
+                hit = cache[i] = grow(i)
+            if best is None or hit[0] > best[0]:
+                best = hit
+        _, pos, got, _ = best
+        blocks.append(SymBlock(sorted(pos, reverse=True), got))
+        done += len(got)
+        head.update(pos)
+        moved = set(pos)
+        cache = {i: hit for i, hit in cache.items() if not (hit[3] & moved)}
+    return blocks
+
+
 def recipe_matrix(recipe, op_matrices):
     """Host (complex128) composition of a :class:`Recipe` -- what the device
     computes; used to check the device kernel and the symbolic fusion."""
@@ -410,7 +510,7 @@ def _remember_plan(key, plan):
 
 
 def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, max_sweep_k=5, itemsize=8,
-                device_fusion=False):
+                device_fusion=False, pack=False):
     """Compile an op sequence (with ``None`` marking a renormalisation point)
     into a :class:`Plan`.
 
@@ -420,7 +520,9 @@ def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, 
     (statevectors of at least 14 qubits; otherwise as ``"fused"``).
     ``itemsize`` (8 for complex64, 16 for complex128) caps the tile at 128 KiB
     of shared memory. ``device_fusion``: block matrices are left as
-    :class:`Recipe` objects for the executor to compose on the GPU.
+    :class:`Recipe` objects for the executor to compose on the GPU. ``pack``
+    (dense passes of device-fused blocks): the blocks of :func:`fuse_frontier`,
+    run from either end, when they are fewer -- fewer passes, the ops in another of their valid orders.
     """
     tile_bits = min(tile_bits, 14 if itemsize <= 8 else 13)
     # unitarity of every op with a matrix, batched once (the plan key, trace checks and fusion use it)
@@ -454,7 +556,7 @@ def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, 
     key = None
     if device_fusion and mode != "gate" and ops and not any(o is not None and o.kind == "pauli_mix" for o in ops):
         flags = [ucache[id(o)] for o in ops if o is not None]
-        key = (nbits, mode, width, tile_bits, low_bits, max_sweep_k, itemsize,
+        key = (nbits, mode, width, tile_bits, low_bits, max_sweep_k, itemsize, pack,
                tuple(None if o is None else tuple(o.bits) for o in ops), tuple(flags), tuple(_pair_offsets(ops)),
                tp_flags)
         plan = _cached_plan(key, ops)
@@ -493,6 +595,11 @@ def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, 
             base = len(plan.op_matrices)
             plan.op_matrices.extend(np.ascontiguousarray(o.matrix, dtype=np.complex128) for o in seg)
             sym = fuse_symbolic(seg, w)
+            if pack and mode == "fused":
+                n = len(seg)
+                back = [SymBlock(b.bits, [n - 1 - i for i in reversed(b.ops)])
+                        for b in reversed(fuse_frontier(seg[::-1], w))]
+                sym = min(sym, fuse_frontier(seg, w), back, key=len)  # the first of the shortest
             blocks = [Block(b.bits, Recipe(list(b.bits), [(base + i, list(seg[i].bits)) for i in b.ops]), b.n_ops)
                       for b in sym]
             bflags = [all(uflags[i] for i in b.ops) for b in sym]

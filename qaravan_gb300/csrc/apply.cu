@@ -235,8 +235,7 @@ namespace qgb_host {
 // j is out_bits[j] (same set of bits) to `batch` vectors of 2^nbits entries.
 int apply_dense_bits(void* sv, int dtype, int nbits, const int* in_bits, const int* out_bits, int k,
                      const void* op, int64_t op_stride, int64_t batch, int64_t sv_stride, cudaStream_t st,
-                     int unitary = 0, double* chain = nullptr, int link = 0, const double* scale = nullptr,
-                     int reverse = 0) {
+                     DensePass pass = {}) {
     if (!sv || !op) return set_error(QGB_EINVAL, "null state or operator pointer");
     if (dtype != QGB_C64 && dtype != QGB_C128) return set_error(QGB_EINVAL, "dtype %d unknown", dtype);
     if (k < 1 || k > QGB_MAX_K) return set_error(QGB_EINVAL, "gate width k=%d not in [1, %d]", k, QGB_MAX_K);
@@ -275,25 +274,27 @@ int apply_dense_bits(void* sv, int dtype, int nbits, const int* in_bits, const i
     a.batch = batch;
     a.sv_stride = sv_stride;
     a.groups = uint64_t(1) << (nbits - k);
-    if (unitary == 2) {
+    if (pass.unitary == 2) {
         if (dtype == QGB_C64) {
-            const int rc = try_dense_tc(sv, op, nbits, a.sorted, in_bits, out_bits, k, op_stride, batch, sv_stride, 2,
-                                        st, chain, link, nullptr, reverse);
+            const int rc = try_dense_tc(sv, op, nbits, a.sorted, in_bits, out_bits, k, op_stride, batch, sv_stride, st,
+                                        pass);
             if (rc != QGB_EDECLINE) return rc;
         }
         // not on the chain kernel: clear the chain, so that the next pass starts a new one
-        if (cudaMemsetAsync(chain, 0, 6 * sizeof(double), st) != cudaSuccess) return check_launch("norm chain reset");
-        unitary = 1;
+        if (cudaMemsetAsync(pass.chain, 0, 6 * sizeof(double), st) != cudaSuccess)
+            return check_launch("norm chain reset");
+        pass.unitary = 1;
+        pass.chain = nullptr;
     }
     if (dtype == QGB_C64) {
-        const int rc = try_dense_tc(sv, op, nbits, a.sorted, in_bits, out_bits, k, op_stride, batch, sv_stride,
-                                    unitary, st, nullptr, 0, scale, reverse);
+        const int rc = try_dense_tc(sv, op, nbits, a.sorted, in_bits, out_bits, k, op_stride, batch, sv_stride, st,
+                                    pass);
         if (rc != QGB_EDECLINE) return rc;
     }
     const int rc = dtype == QGB_C64 ? dispatch_dense<float>(sv, op, a, st) : dispatch_dense<double>(sv, op, a, st);
-    if (rc || !scale) return rc;
+    if (rc || !pass.scale) return rc;
     // the CUDA-core kernels take no factor: one more pass multiplies the result by it
-    return qgb_scale(sv, dtype, nbits, scale, 1, 0, st);
+    return qgb_scale(sv, dtype, nbits, pass.scale, 1, 0, st);
 }
 
 }  // namespace qgb_host
@@ -301,8 +302,7 @@ int apply_dense_bits(void* sv, int dtype, int nbits, const int* in_bits, const i
 namespace {
 
 int op_action(void* sv, int dtype, int n, const int* indices, int k, const void* op, int64_t op_stride,
-              int64_t batch, int64_t sv_stride, void* stream, int unitary, double* chain = nullptr, int link = 0,
-              const double* scale = nullptr, int reverse = 0) {
+              int64_t batch, int64_t sv_stride, void* stream, const DensePass& pass = {}) {
     if (n < 1 || n > QGB_MAX_QUBITS) return set_error(QGB_EINVAL, "n=%d not in [1, %d]", n, QGB_MAX_QUBITS);
     if (!indices) return set_error(QGB_EINVAL, "null indices");
     if (k < 1 || k > QGB_MAX_K) return set_error(QGB_EINVAL, "gate width k=%d not in [1, %d]", k, QGB_MAX_K);
@@ -312,19 +312,21 @@ int op_action(void* sv, int dtype, int n, const int* indices, int k, const void*
         bits[j] = n - 1 - indices[j];
     }
     return apply_dense_bits(sv, dtype, n, bits, bits, k, op, op_stride, batch, sv_stride, (cudaStream_t)stream,
-                            unitary, chain, link, scale, reverse);
+                            pass);
 }
 
 }  // namespace
 
 extern "C" int qgb_op_action(void* sv, int dtype, int n, const int* indices, int k, const void* op,
                              int64_t op_stride, int64_t batch, int64_t sv_stride, void* stream) {
-    return op_action(sv, dtype, n, indices, k, op, op_stride, batch, sv_stride, stream, 0);
+    return op_action(sv, dtype, n, indices, k, op, op_stride, batch, sv_stride, stream);
 }
 
 extern "C" int qgb_op_action_unitary(void* sv, int dtype, int n, const int* indices, int k, const void* op,
                                      int64_t op_stride, int64_t batch, int64_t sv_stride, void* stream) {
-    return op_action(sv, dtype, n, indices, k, op, op_stride, batch, sv_stride, stream, 1);
+    DensePass pass;
+    pass.unitary = 1;
+    return op_action(sv, dtype, n, indices, k, op, op_stride, batch, sv_stride, stream, pass);
 }
 
 extern "C" int qgb_op_action_unitary_chain(void* sv, int dtype, int n, const int* indices, int k, const void* op,
@@ -333,14 +335,20 @@ extern "C" int qgb_op_action_unitary_chain(void* sv, int dtype, int n, const int
     if (!chain || (reinterpret_cast<uintptr_t>(chain) % sizeof(double)))
         return set_error(QGB_EINVAL, "norm chain buffer missing or not 8-byte aligned");
     if (link < 0) return set_error(QGB_EINVAL, "negative chain link %d", link);
-    return op_action(sv, dtype, n, indices, k, op, op_stride, batch, sv_stride, stream, 2, chain, link);
+    DensePass pass;
+    pass.unitary = 2;
+    pass.chain = chain;
+    pass.link = link;
+    return op_action(sv, dtype, n, indices, k, op, op_stride, batch, sv_stride, stream, pass);
 }
 
 extern "C" int qgb_op_action_scaled(void* sv, int dtype, int n, const int* indices, int k, const void* op,
                                     const double* factor, void* stream) {
     if (!factor || (reinterpret_cast<uintptr_t>(factor) % sizeof(double)))
         return set_error(QGB_EINVAL, "factor missing or not 8-byte aligned");
-    return op_action(sv, dtype, n, indices, k, op, 0, 1, 0, stream, 0, nullptr, 0, factor);
+    DensePass pass;
+    pass.scale = factor;
+    return op_action(sv, dtype, n, indices, k, op, 0, 1, 0, stream, pass);
 }
 
 extern "C" size_t qgb_call_bytes(void) { return sizeof(qgb_call); }
@@ -357,29 +365,36 @@ extern "C" int qgb_run_calls(void* sv, int dtype, int n, const qgb_call* calls, 
         const qgb_call& c = calls[i];
         const char* op = static_cast<const char*>(mats) + c.mat * int64_t(esz);
         if (c.kind <= QGB_CALL_SCALED && c.mat < 0) return set_error(QGB_EINVAL, "call %d: negative matrix offset", i);
-        if (c.kind == QGB_CALL_CHAIN && (!chain || c.link < 0))
-            return set_error(QGB_EINVAL, "call %d: norm chain buffer missing or negative link", i);
+        if (c.kind == QGB_CALL_CHAIN && (!chain || c.link < 0 || c.first < 0))
+            return set_error(QGB_EINVAL, "call %d: norm chain buffer missing, negative link or epoch", i);
         if ((c.kind == QGB_CALL_SCALED || c.kind == QGB_CALL_TRACE) && !trace)
             return set_error(QGB_EINVAL, "call %d: trace buffer missing", i);
         int rc;
+        DensePass pass;
+        pass.reverse = passes++ & 1;
+        switch (c.kind) {
+            case QGB_CALL_CHAIN:
+                pass.unitary = 2;
+                pass.chain = chain;
+                pass.link = c.link;
+                pass.first = c.first;
+                break;
+            case QGB_CALL_ROWS: pass.unitary = 1; break;
+            case QGB_CALL_SCALED: pass.scale = trace + 1; break;
+            default: break;
+        }
         switch (c.kind) {
             case QGB_CALL_OP:
-                rc = op_action(sv, dtype, n, c.sites, c.k, op, 0, 1, 0, stream, 0, nullptr, 0, nullptr, passes++ & 1);
-                break;
             case QGB_CALL_CHAIN:
-                rc = op_action(sv, dtype, n, c.sites, c.k, op, 0, 1, 0, stream, 2, chain, c.link, nullptr, passes++ & 1);
-                break;
             case QGB_CALL_ROWS:
-                rc = op_action(sv, dtype, n, c.sites, c.k, op, 0, 1, 0, stream, 1, nullptr, 0, nullptr, passes++ & 1);
-                break;
             case QGB_CALL_SCALED:
-                rc = op_action(sv, dtype, n, c.sites, c.k, op, 0, 1, 0, stream, 0, nullptr, 0, trace + 1, passes++ & 1);
+                rc = op_action(sv, dtype, n, c.sites, c.k, op, 0, 1, 0, stream, pass);
                 break;
-            case QGB_CALL_TRACE: rc = qgb_dm_trace_factor(sv, dtype, n / 2, trace, c.link, stream); break;
-            case QGB_CALL_SWEEP:
-                rc = qgb_apply_sweep(sv, dtype, n, c.sweep, mats, 0, 1, 0, stream);
-                ++passes;
+            case QGB_CALL_TRACE:
+                rc = qgb_dm_trace_factor(sv, dtype, n / 2, trace, c.link, stream);
+                --passes;  // the diagonal only
                 break;
+            case QGB_CALL_SWEEP: rc = qgb_apply_sweep(sv, dtype, n, c.sweep, mats, 0, 1, 0, stream); break;
             default: return set_error(QGB_EINVAL, "call %d: kind %d unknown", i, c.kind);
         }
         if (rc) return rc;

@@ -723,10 +723,11 @@ int build_tc_args(TcArgs& a, int nbits, const int* sorted, const int* in_bits, c
 // nothing) when the op is not one it takes, so that the caller runs the
 // CUDA-core kernel instead.
 int try_dense_tc(void* sv, const void* op, int nbits, const int* sorted, const int* in_bits, const int* out_bits,
-                 int k, int64_t op_stride, int64_t batch, int64_t sv_stride, int unitary, cudaStream_t st,
-                 double* chain, int link, const double* scale, int reverse) {
+                 int k, int64_t op_stride, int64_t batch, int64_t sv_stride, cudaStream_t st, const DensePass& pass) {
     const int mode = dense_impl();
-    if (scale && unitary != 0) return QGB_EDECLINE;  // a factor goes with plain (MODE 0) passes only
+    int unitary = pass.unitary;
+    double* chain = pass.chain;
+    if (pass.scale && unitary != 0) return QGB_EDECLINE;  // a factor goes with plain (MODE 0) passes only
     if (unitary == 2 && (batch > 1 || !chain)) return QGB_EDECLINE;  // the chain follows one state
     if (mode == 0 || k < 4 || k > 6 || (k == 4 && mode < 2)) return QGB_EDECLINE;
     if (nbits < 13) return QGB_EDECLINE;              // fewer than one 8192-amplitude tile
@@ -738,19 +739,22 @@ int try_dense_tc(void* sv, const void* op, int nbits, const int* sorted, const i
         const int rc = build_tc_args(a, nbits, sorted, in_bits, out_bits, k, batch, sv_stride);
         if (rc != QGB_OK) return rc;
     }
-    a.scale = scale;
-    a.reverse = reverse && a.tiles <= kReverseTiles;
+    a.scale = pass.scale;
+    a.reverse = pass.reverse && a.tiles <= kReverseTiles;
     float2* s = static_cast<float2*>(sv);
     const float2* m = static_cast<const float2*>(op);
     if (unitary == 2) {
         // epochs of kChainEpoch passes: the first corrects (and starts the chain), the
         // last measures its output; the passes between run without norm control
-        if (link == 0 && cudaMemsetAsync(chain, 0, 6 * sizeof(double), st) != cudaSuccess)
+        if (pass.link == 0 && cudaMemsetAsync(chain, 0, 6 * sizeof(double), st) != cudaSuccess)
             return check_launch("norm chain reset");
-        const int e = link / kChainEpoch, pos = link % kChainEpoch;
+        const int first = pass.first > 0 ? pass.first : kChainEpoch;
+        const int later = pass.link - first;  // passes since the first epoch ended
+        const int e = later < 0 ? 0 : 1 + later / kChainEpoch;
+        const int pos = later < 0 ? pass.link : later % kChainEpoch;
         a.chain = chain;
         a.c_head = pos == 0;
-        a.c_tail = pos == kChainEpoch - 1;
+        a.c_tail = pos == (e == 0 ? first : kChainEpoch) - 1;
         a.c_prev = e > 0 ? (e - 1) % 3 : -1;
         a.c_cur = e % 3;
         a.c_next = (e + 1) % 3;

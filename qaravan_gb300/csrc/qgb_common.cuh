@@ -197,9 +197,17 @@ int sm_count();
 // Internal status (never returned through the C ABI): a specialised kernel
 // declines an op, and the caller runs the general kernel instead.
 constexpr int QGB_EDECLINE = 1000;
+// How a dense pass is run.
+struct DensePass {
+    int unitary = 0;                // 0: any op; 1: group norms restored; 2: link of a norm chain
+    double* chain = nullptr;        // unitary = 2: the chain's buffer (6 doubles),
+    int link = 0;                   //   this pass's number in the chain,
+    int first = 0;                  //   passes of its first epoch (0: as many as of the others)
+    const double* scale = nullptr;  // device factor of the operator (unitary = 0)
+    int reverse = 0;                // tiles in descending order
+};
 int try_dense_tc(void* sv, const void* op, int nbits, const int* sorted, const int* in_bits, const int* out_bits,
-                 int k, int64_t op_stride, int64_t batch, int64_t sv_stride, int unitary, cudaStream_t st,
-                 double* chain = nullptr, int link = 0, const double* scale = nullptr, int reverse = 0);
+                 int k, int64_t op_stride, int64_t batch, int64_t sv_stride, cudaStream_t st, const DensePass& pass);
 int tc_status_read_clear();
 int tcs_status_read_clear();
 int dmb_status_read_clear();

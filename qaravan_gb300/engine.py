@@ -29,6 +29,7 @@ from .compiler import DenseStep, NormalizeStep, PauliMixStep, Plan, Recipe, Swee
 # pass (qgb_op_action_unitary; also what batches use under "chain"), ~10 % of the
 # kernel's speed. "off": neither. QGB_NORM_RESTORE=chain|row|0 or set_norm_restore().
 _NORM_MODES = {"1": "chain", "chain": "chain", "row": "row", "0": "off", "off": "off"}
+_CHAIN_EPOCH = 4  # passes per epoch of the norm chain (the library's)
 _NORM_RESTORE = _NORM_MODES.get(os.environ.get("QGB_NORM_RESTORE", "chain"), "chain")
 
 
@@ -351,14 +352,17 @@ class Executor:
 
     def _call_list(self, mode, tchain):
         """The plan's launches on one vector as one array for ``qgb_run_calls``: the
-        entries, chain links and trace measurements that ``run`` takes step by step."""
-        calls, link, t_since, t_pending = [], 0, 0, False
+        entries and trace measurements that ``run`` takes step by step. The norm
+        chain knows its length here: its first epoch is cut so that the chain's last
+        pass opens an epoch and corrects the drift of every pass but its own, and
+        unitary blocks on the CUDA cores, which do not drift, leave it running."""
+        calls, chains, t_since, t_pending = [], [[]], 0, False
         if tchain:
             calls.append((_lib.QGB_CALL_TRACE, None, 0, 1, 0, None))
         for s in self._steps:
             if s[0] == "sweep":
                 calls.append((_lib.QGB_CALL_SWEEP, None, 0, 0, 0, s[1]))
-                link = 0
+                chains.append([])
                 continue
             _, sites, k, off, unitary, whole, on_tc = s
             if tchain:
@@ -369,20 +373,25 @@ class Executor:
                 if whole and t_since >= _TRACE_EPOCH:
                     calls.append((_lib.QGB_CALL_TRACE, None, 0, 0, 0, None))
                     t_since, t_pending = 0, True
-            elif unitary and mode == "chain":
-                calls.append((_lib.QGB_CALL_CHAIN, sites, k, link, off, None))
-                link += 1
+            elif unitary and mode == "chain" and on_tc:
+                chains[-1].append(len(calls))
+                calls.append((_lib.QGB_CALL_CHAIN, sites, k, len(chains[-1]) - 1, off, None))
+            elif unitary and mode != "off":
+                calls.append((_lib.QGB_CALL_ROWS, sites, k, 0, off, None))
             else:
-                calls.append((_lib.QGB_CALL_ROWS if unitary and mode == "row" else _lib.QGB_CALL_OP, sites, k, 0, off,
-                              None))
-                link = 0
+                calls.append((_lib.QGB_CALL_OP, sites, k, 0, off, None))
+                if not unitary:
+                    chains.append([])
         arr = (_lib.Call * max(len(calls), 1))()
-        for c, (kind, sites, k, ln, off, sweep) in zip(arr, calls):
-            c.kind, c.k, c.link, c.mat = kind, k, ln, off
+        for c, (kind, sites, k, link, off, sweep) in zip(arr, calls):
+            c.kind, c.k, c.link, c.mat = kind, k, link, off
             for j in range(k):
                 c.sites[j] = sites[j]
             if sweep is not None:
                 c.sweep = C.pointer(sweep)
+        for chain in chains:
+            for i in chain:
+                arr[i].first = (len(chain) - 1) % _CHAIN_EPOCH
         return arr, len(calls)
 
     def _run_calls(self, state, L, ptr, st):

@@ -44,12 +44,14 @@ struct AdjSweepArgs {
     // register runs: consecutive ops on at most `rbits` tile bits, applied to groups of
     // 2^rbits amplitudes of both tiles held in registers (0: one shared-memory pass per op)
     int rbits;
+    int n_runs;
     int run_len[QGB_SWEEP_MAX_OPS];     // at a run's first op: its op count (0 elsewhere)
     int run_pos[QGB_SWEEP_MAX_OPS][4];  // at a run's first op: the tile bit of each local bit of the run
     int op_lpos[QGB_SWEEP_MAX_OPS][2];  // every op's sites as local bits of its run
     int op_gcls[QGB_SWEEP_MAX_OPS];     // generator class of a wanted derivative (kGenNone: none)
-    uint64_t tiles;        // tiles per state
-    uint64_t chunk_tiles;  // tiles per chunk
+    uint64_t tiles;        // tiles per state, 2^tile_shift
+    uint64_t chunk_tiles;  // tiles per chunk, 2^chunk_shift
+    int tile_shift, chunk_shift;
     uint64_t chunks;       // chunks over all states
 };
 
@@ -248,7 +250,7 @@ __device__ __forceinline__ void adj_tile_run(cplx<T>* __restrict__ pt, cplx<T>* 
             T v = s[q];
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if ((tid & 31) == 0) wacc_add(red[(op0 + q) * kAdjMaxWarps + (tid >> 5)], v);
+            if ((tid & 31) == 0) wacc_add(red[op0 + q], v);
         }
     }
 }
@@ -269,6 +271,21 @@ constexpr int kAdjPermCX = 4, kAdjPermXC = 5, kAdjPermSwap = 6;
 // generator classes of a wanted derivative (host-classified Pauli-product rows): none, diagonal
 // (row r reads column r), flipped (one site: row r reads r ^ 1; two sites: 3 - r), any other
 constexpr int kGenNone = 0, kGenDiag = 1, kGenFlip = 2, kGenAny = 3;
+// one-site generators with real (Z, X) or imaginary (Y) entries need one component of each sum
+constexpr int kGenDiagRe = 4, kGenFlipRe = 5, kGenFlipIm = 6;
+
+// A staged one-site op uses 4 of its 16 slots; slots 4 and 5 repeat a real U^dagger's (a, b), (c, d)
+// or a diagonal one's entries, so that one 16-byte load fetches them (complex64), slot 6 holds
+// the two generator entries' nonzero components.
+__device__ __forceinline__ void adj_load2(const float2* u, float2& a, float2& b) {
+    const float4 q = *reinterpret_cast<const float4*>(u + 4);
+    a = make_float2(q.x, q.y);
+    b = make_float2(q.z, q.w);
+}
+__device__ __forceinline__ void adj_load2(const double2* u, double2& a, double2& b) {
+    a = u[4];
+    b = u[5];
+}
 
 // The derivative Im sum_r conj(l_r) (g_r p_{col r}) of one op over a group: complex sums
 // W_r = sum conj(l_r) q_r per generator row r, combined once per op as Im(g_r W_r) =
@@ -284,12 +301,36 @@ __device__ __forceinline__ void wacc<double, double2>(double2& w, const double2&
     w.y = fma(l.x, q.y, fma(-l.y, q.x, w.y));
 }
 
+// one component of wacc's sum
+template <bool IM, typename C, typename T>
+__device__ __forceinline__ void wacc1(T& w, const C& l, const C& q) {
+    if constexpr (IM) w = fma(l.x, q.y, fma(-l.y, q.x, w));
+    else w = fma(l.x, q.x, fma(l.y, q.y, w));
+}
+
 template <int R, int P, int MODE, int GEN, typename C, typename T>
 __device__ __forceinline__ void adj_reg1(C (&p)[1 << R], C (&l)[1 << R], const C* __restrict__ u,
                                          const float2* gv, T& s) {
     constexpr int D = 1 << R, bit = 1 << P;
-    const C u0 = u[0], u1 = u[1], u2 = u[2], u3 = u[3];
+    constexpr bool one = GEN == kGenDiagRe || GEN == kGenFlipRe || GEN == kGenFlipIm;
+    C u0, u1, u2, u3;
+    if constexpr (MODE == kAdjReal) {
+        C ab, cd;
+        adj_load2(u, ab, cd);
+        u0.x = ab.x;
+        u1.x = ab.y;
+        u2.x = cd.x;
+        u3.x = cd.y;
+    } else if constexpr (MODE == kAdjDiag) {
+        adj_load2(u, u0, u3);
+    } else if constexpr (MODE == kAdjDense) {
+        u0 = u[0];
+        u1 = u[1];
+        u2 = u[2];
+        u3 = u[3];
+    }
     C w0 = mk<T>(T(0), T(0)), w1 = mk<T>(T(0), T(0));
+    T v0 = T(0), v1 = T(0);
 #pragma unroll
     for (int c = 0; c < D; ++c) {
         if (c & bit) continue;
@@ -297,6 +338,12 @@ __device__ __forceinline__ void adj_reg1(C (&p)[1 << R], C (&l)[1 << R], const C
         if constexpr (GEN == kGenDiag) {
             wacc<T>(w0, l0, p0);
             wacc<T>(w1, l1, p1);
+        } else if constexpr (GEN == kGenDiagRe) {
+            wacc1<true>(v0, l0, p0);
+            wacc1<true>(v1, l1, p1);
+        } else if constexpr (GEN == kGenFlipRe || GEN == kGenFlipIm) {
+            wacc1<GEN == kGenFlipRe>(v0, l0, p1);
+            wacc1<GEN == kGenFlipRe>(v1, l1, p0);
         } else if constexpr (GEN != kGenNone) {  // one site: off-diagonal rows (X, Y)
             wacc<T>(w0, l0, p1);
             wacc<T>(w1, l1, p0);
@@ -338,7 +385,10 @@ __device__ __forceinline__ void adj_reg1(C (&p)[1 << R], C (&l)[1 << R], const C
             l[c | bit] = t;
         }
     }
-    if constexpr (GEN != kGenNone)
+    if constexpr (one) {
+        const C g = u[6];
+        s = fma(g.y, v1, g.x * v0);
+    } else if constexpr (GEN != kGenNone)
         s += T(gv[0].x) * w0.y + T(gv[0].y) * w0.x + T(gv[1].x) * w1.y + T(gv[1].y) * w1.x;
 }
 
@@ -436,28 +486,6 @@ __device__ __forceinline__ void adj_reg2(C (&p)[1 << R], C (&l)[1 << R], const C
     }
 }
 
-// the op's class and generator class, chosen once per op (each case its own unrolled code)
-template <int R, int P, int GEN, typename C, typename T>
-__device__ __forceinline__ void adj_reg1_mode(C (&p)[1 << R], C (&l)[1 << R], const C* u, int mode, const float2* gv,
-                                              T& s) {
-    switch (mode) {
-        case kAdjReal: adj_reg1<R, P, kAdjReal, GEN>(p, l, u, gv, s); break;
-        case kAdjDiag: adj_reg1<R, P, kAdjDiag, GEN>(p, l, u, gv, s); break;
-        case kAdjPerm: adj_reg1<R, P, kAdjPerm, GEN>(p, l, u, gv, s); break;
-        default: adj_reg1<R, P, kAdjDense, GEN>(p, l, u, gv, s); break;
-    }
-}
-
-template <int R, int P, typename C, typename T>
-__device__ __forceinline__ void adj_reg1_any(C (&p)[1 << R], C (&l)[1 << R], const C* u, int mode, int gen,
-                                             const float2* gv, T& s) {
-    switch (gen) {
-        case kGenNone: adj_reg1_mode<R, P, kGenNone>(p, l, u, mode, gv, s); break;
-        case kGenDiag: adj_reg1_mode<R, P, kGenDiag>(p, l, u, mode, gv, s); break;
-        default: adj_reg1_mode<R, P, kGenFlip>(p, l, u, mode, gv, s); break;
-    }
-}
-
 template <int R, int P0, int P1, int GEN, typename C, typename T>
 __device__ __forceinline__ void adj_reg2_mode(C (&p)[1 << R], C (&l)[1 << R], const C* u, int mode,
                                               const uint8_t* col, const float2* gv, const int* gc, T& s) {
@@ -479,17 +507,6 @@ __device__ __forceinline__ void adj_reg2_any(C (&p)[1 << R], C (&l)[1 << R], con
         case kGenDiag: adj_reg2_mode<R, P0, P1, kGenDiag>(p, l, u, mode, col, gv, gc, s); break;
         case kGenFlip: adj_reg2_mode<R, P0, P1, kGenFlip>(p, l, u, mode, col, gv, gc, s); break;
         default: adj_reg2_mode<R, P0, P1, kGenAny>(p, l, u, mode, col, gv, gc, s); break;
-    }
-}
-
-template <int R, typename C, typename T>
-__device__ __forceinline__ void adj_apply1(C (&p)[1 << R], C (&l)[1 << R], int P, const C* u, int mode, int gen,
-                                           const float2* gv, T& s) {
-    switch (P) {
-        case 0: adj_reg1_any<R, 0>(p, l, u, mode, gen, gv, s); break;
-        case 1: if constexpr (R > 1) adj_reg1_any<R, 1>(p, l, u, mode, gen, gv, s); break;
-        case 2: if constexpr (R > 2) adj_reg1_any<R, 2>(p, l, u, mode, gen, gv, s); break;
-        case 3: if constexpr (R > 3) adj_reg1_any<R, 3>(p, l, u, mode, gen, gv, s); break;
     }
 }
 
@@ -519,80 +536,344 @@ __device__ __forceinline__ void adj_apply2(C (&p)[1 << R], C (&l)[1 << R], int P
     }
 }
 
-// Every run of the pass on one staged pair of tiles: groups of 2^R amplitudes,
-// one group per thread at a time, a barrier after each run. umode / ucol: each
-// op's U^dagger class and, for a permutation, its source column per row.
-template <typename T, int R>
-__device__ __forceinline__ void adj_tile_runs(cplx<T>* __restrict__ pt, cplx<T>* __restrict__ lt, int m,
-                                              const AdjSweepArgs& a, const cplx<T>* __restrict__ ush,
+// Every op of a run is one case of one switch (its own unrolled code): a one-site op by its local bit,
+// U^dagger class and generator class, two consecutive one-site ops Z-like then Y-like on the same bit (the
+// RZ, RY pair of a reversed ansatz) as one, any two-site op through adj_apply2.
+constexpr int kCodeTwo = 0, kCodePair = 1, kCodeOne = 4;  // kCodePair + P; kCodeOne + (P * 4 + mode) * 6 + gen
+__device__ __forceinline__ int adj_gen_index(int gen) {  // kGenNone, DiagRe, FlipRe, FlipIm, Diag, Flip -> 0..5
+    return gen == kGenNone ? 0 : gen == kGenDiagRe ? 1 : gen == kGenFlipRe ? 2 : gen == kGenFlipIm ? 3
+           : gen == kGenDiag ? 4 : 5;
+}
+
+// The derivative sums of a tile's ops, reduced over a warp 32 ops at a time. Op t's 32 per-thread sums are
+// added by the xor tree 16, 8, 4, 2, 1, the additions of different ops sharing the lanes: two ops waiting at a
+// level are merged by one shuffle (the upper lanes go on with the later op), so an op costs one shuffle
+// instead of five and a level's latency is paid once for all. The sums of an op are added in the same
+// tree as one op at a time.
+__device__ __forceinline__ int adj_gen1(const AdjSweepArgs& a, int op) {  // a one-site op's generator class
+    const int cls = a.op_gcls[op];
+    if (cls == kGenNone) return kGenNone;
+    const float2 g0 = a.gval[op][0], g1 = a.gval[op][1];
+    const bool re = g0.y == 0.f && g1.y == 0.f, im = g0.x == 0.f && g1.x == 0.f;
+    if (cls == kGenDiag) return re ? kGenDiagRe : kGenDiag;
+    return re ? kGenFlipRe : (im ? kGenFlipIm : kGenFlip);
+}
+
+template <typename T>
+__device__ __forceinline__ T adj_merge(T a, T b, int o, int lane) {  // a: the earlier op
+    const bool up = lane & o;
+    const T keep = up ? b : a, send = up ? a : b;
+    return keep + __shfl_xor_sync(0xffffffffu, send, o);
+}
+
+template <typename T>
+struct AdjTree {
+    T s[5];
+    int t;
+    __device__ __forceinline__ void add_to(typename WAccOf<T>::type* red, const uint8_t* dlist, int nd, T x, int lane) {
+        const int at = (t & ~31) + int(__brev(uint32_t(lane)) >> 27);
+        if (at < nd) wacc_add(red[dlist[at]], x);
+    }
+    // the next derivative op's per-thread sum; red: this warp's accumulators, dlist: op of each derivative
+    __device__ __forceinline__ void push(T x, typename WAccOf<T>::type* red, const uint8_t* dlist, int nd, int lane) {
+        const int t0 = t;
+        bool out = true;
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            if (out) {
+                if ((t0 >> k) & 1) {
+                    x = adj_merge(s[k], x, 16 >> k, lane);
+                } else {
+                    s[k] = x;
+                    out = false;
+                }
+            }
+        }
+        if (out) add_to(red, dlist, nd, x, lane);
+        t = t0 + 1;
+    }
+    // two in a row
+    __device__ __forceinline__ void push2(T x, T y, typename WAccOf<T>::type* red, const uint8_t* dlist, int nd,
+                                          int lane) {
+        if (t & 1) {
+            push(x, red, dlist, nd, lane);
+            push(y, red, dlist, nd, lane);
+            return;
+        }
+        x = adj_merge(x, y, 16, lane);
+        const int t0 = t >> 1;
+        t += 2;
+        if (!(t0 & 1)) {
+            s[1] = x;
+            return;
+        }
+        x = adj_merge(s[1], x, 8, lane);
+        if (!(t0 & 2)) {
+            s[2] = x;
+            return;
+        }
+        x = adj_merge(s[2], x, 4, lane);
+        if (!(t0 & 4)) {
+            s[3] = x;
+            return;
+        }
+        x = adj_merge(s[3], x, 2, lane);
+        if (!(t0 & 8)) {
+            s[4] = x;
+            return;
+        }
+        x = adj_merge(s[4], x, 1, lane);
+        t -= 1;  // add_to names the block of the last op
+        add_to(red, dlist, nd, x, lane);
+        t += 1;
+    }
+    // the ops still waiting at the end of a tile
+    __device__ __forceinline__ void finish(typename WAccOf<T>::type* red, const uint8_t* dlist, int nd, int lane) {
+        if (t & 31) {
+            T x = T(0);
+            bool have = false;
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                if ((t >> k) & 1) {
+                    x = adj_merge(s[k], have ? x : T(0), 16 >> k, lane);
+                    have = true;
+                } else if (have) {
+                    x = adj_merge(x, T(0), 16 >> k, lane);
+                }
+            }
+            add_to(red, dlist, nd, x, lane);
+        }
+        t = 0;
+    }
+};
+
+// A run as the kernel executes it. Permutations without derivative at a run's start or end (the CNOT ladder of
+// an ansatz) move no data: the pass keeps the linear map from a tile's logical index to the place of
+// its amplitude in shared memory, and such an op only changes the map. A run's thread then addresses its group
+// through the images of the index bits: off[P] of the run's bits, base[j] of the j-th other bit, all XORed.
+constexpr int kAdjMaxTile = QGB_SWEEP_MAX_TILE_BITS;
+struct AdjRun {
+    uint32_t off[3];  // byte offsets
+    uint16_t base[kAdjMaxTile - 3];
+    uint16_t flip;   // image of 0 (X gates)
+    uint8_t first, count;  // its ops
+};
+struct AdjMap {  // of the whole tile, after the pass's last op
+    uint16_t bit[kAdjMaxTile];
+    uint16_t flip;
+    uint16_t nruns;
+};
+
+// Builds the runs and the final map from the ops' classes; called by one whole warp.
+template <typename T>
+__device__ void adj_build_runs(AdjRun* runs, AdjMap* map, const AdjSweepArgs& a, const uint8_t* umode, uint8_t* prog,
+                               const uint8_t* ucode, int lane) {
+    const int m = a.m;
+    uint32_t col = lane < m ? swz<T>(1u << lane) : 0u, flip = 0u;  // lane j: the image of index bit j
+    // each lane describes two ops (the loops below then wait for shuffles, not for tables): how the map
+    // moves (0: not at all, 1: X, 2, 3: CNOT either way, 4: SWAP), the sites, and at a run's first op its length
+    uint32_t info[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int op = lane + 32 * h;
+        info[h] = 0;
+        if (op < a.n_ops) {
+            const int mode = umode[op], p0 = a.op_pos[op][0], two = a.op_k[op] == 2;
+            uint32_t kind = 0;
+            if (a.op_gcls[op] == kGenNone) {
+                if (!two) kind = mode == kAdjPerm ? 1 : 0;
+                else kind = mode == kAdjPermCX ? 2 : mode == kAdjPermXC ? 3 : mode == kAdjPermSwap ? 4 : 0;
+            }
+            info[h] = kind | uint32_t(p0) << 4 | uint32_t(two ? a.op_pos[op][1] : p0) << 8 | uint32_t(a.run_len[op]) << 12;
+        }
+    }
+    auto info_of = [&](int op) { return __shfl_sync(0xffffffffu, op < 32 ? info[0] : info[1], op & 31); };
+    auto move = [&](uint32_t f) {  // new[x] = old[pi(x)]: the image of x becomes that of pi(x)
+        const int kind = f & 15, p0 = (f >> 4) & 15, p1 = (f >> 8) & 15;
+        const uint32_t c0 = __shfl_sync(0xffffffffu, col, p0), c1 = __shfl_sync(0xffffffffu, col, p1);
+        if (kind == 1) flip ^= c0;
+        else if (kind == 2) col ^= lane == p0 ? c1 : 0u;
+        else if (kind == 3) col ^= lane == p1 ? c0 : 0u;
+        else col = lane == p0 ? c1 : (lane == p1 ? c0 : col);
+    };
+    int nruns = 0;
+    for (int i0 = 0; i0 < a.n_ops;) {
+        const int end = i0 + int(info_of(i0) >> 12);
+        int b = i0, e = end;
+        for (; b < end; ++b) {
+            const uint32_t f = info_of(b);
+            if (!(f & 15)) break;
+            move(f);
+        }
+        while (e > b && (info_of(e - 1) & 15)) --e;
+        if (b < e) {
+            AdjRun& r = runs[nruns];
+            const int r0 = a.run_pos[i0][0], r1 = a.run_pos[i0][1], r2 = a.run_pos[i0][2];
+            const uint32_t own = 1u << r0 | 1u << r1 | 1u << r2;
+            if (lane == r0) r.off[0] = col * uint32_t(sizeof(cplx<T>));
+            if (lane == r1) r.off[1] = col * uint32_t(sizeof(cplx<T>));
+            if (lane == r2) r.off[2] = col * uint32_t(sizeof(cplx<T>));
+            if (lane < m && !((own >> lane) & 1u)) r.base[__popc(~own & ((1u << lane) - 1u))] = uint16_t(col);
+            if (lane == 0) {
+                r.flip = uint16_t(flip);
+                r.first = uint8_t(b);
+                r.count = uint8_t(e - b);
+                // only pairs, on bits 0, 1, .. in order: a program of its own (1 to 3 pairs)
+                int np = (e - b) % 2 == 0 && e - b <= 6 ? (e - b) / 2 : 0;
+                for (int j = 0; j < np; ++j)
+                    if (ucode[b + 2 * j] != kCodePair + j) np = 0;
+                prog[nruns] = uint8_t(np);
+            }
+            ++nruns;
+        }
+        for (; e < end; ++e) move(info_of(e));
+        i0 = end;
+    }
+    if (lane < m) map->bit[lane] = uint16_t(col);
+    if (lane == 0) {
+        map->flip = uint16_t(flip);
+        map->nruns = uint16_t(nruns);
+    }
+}
+
+// The pair Z-like then Y-like on bit P, straight-line.
+template <int P, typename C, typename T>
+__device__ __forceinline__ void adj_pair(C (&p)[8], C (&l)[8], const C* __restrict__ u, T& s0, T& s1) {
+    adj_reg1<3, P, kAdjDiag, kGenDiagRe>(p, l, u, nullptr, s0);
+    adj_reg1<3, P, kAdjReal, kGenFlipIm>(p, l, u + 16, nullptr, s1);
+}
+
+// Any run, an op at a time. one: a single group per thread (its sums join the tree).
+template <typename T>
+__device__ __forceinline__ void adj_run_ops(cplx<T> (&p)[8], cplx<T> (&l)[8], int first, int count, bool one,
+                                            const AdjSweepArgs& a, const cplx<T>* __restrict__ ush,
+                                            const uint8_t* __restrict__ ucode, const uint8_t* __restrict__ umode,
+                                            const uint8_t* __restrict__ ucol, AdjTree<T>& tree,
+                                            const uint8_t* __restrict__ dlist, int nd,
+                                            typename WAccOf<T>::type* __restrict__ red, int lane) {
+    using C = cplx<T>;
+    constexpr int R = 3;
+    for (int q = 0; q < count; ++q) {
+        const int op = first + q;
+        const C* u = ush + op * 16;
+        T sd = T(0), sd2 = T(0);
+        const int code = ucode[op];
+        switch (code) {
+#define QGB_ADJ_G(P, M, B)                                                                                  \
+    case kCodeOne + ((P) * 4 + (B)) * 6 + 0: adj_reg1<R, P, M, kGenNone>(p, l, u, a.gval[op], sd); break;   \
+    case kCodeOne + ((P) * 4 + (B)) * 6 + 1: adj_reg1<R, P, M, kGenDiagRe>(p, l, u, a.gval[op], sd); break; \
+    case kCodeOne + ((P) * 4 + (B)) * 6 + 2: adj_reg1<R, P, M, kGenFlipRe>(p, l, u, a.gval[op], sd); break; \
+    case kCodeOne + ((P) * 4 + (B)) * 6 + 3: adj_reg1<R, P, M, kGenFlipIm>(p, l, u, a.gval[op], sd); break; \
+    case kCodeOne + ((P) * 4 + (B)) * 6 + 4: adj_reg1<R, P, M, kGenDiag>(p, l, u, a.gval[op], sd); break;   \
+    case kCodeOne + ((P) * 4 + (B)) * 6 + 5: adj_reg1<R, P, M, kGenFlip>(p, l, u, a.gval[op], sd); break;
+#define QGB_ADJ_P(P)                                                        \
+    case kCodePair + (P): adj_pair<P>(p, l, u, sd, sd2); break;             \
+        QGB_ADJ_G(P, kAdjDense, 0) QGB_ADJ_G(P, kAdjDiag, 1) QGB_ADJ_G(P, kAdjPerm, 2) QGB_ADJ_G(P, kAdjReal, 3)
+            QGB_ADJ_P(0)
+            QGB_ADJ_P(1)
+            QGB_ADJ_P(2)
+#undef QGB_ADJ_P
+#undef QGB_ADJ_G
+            default:
+                adj_apply2<R>(p, l, a.op_lpos[op][0], a.op_lpos[op][1], u, umode[op], a.op_gcls[op], ucol + op * 4,
+                              a.gval[op], a.gcol[op], sd);
+                break;
+        }
+        const bool pair = code >= kCodePair && code < kCodeOne;
+        if (a.op_gcls[op] != kGenNone) {  // uniform over the CTA: every lane reaches the shuffles
+            if (one) {
+                if (pair) tree.push2(sd, sd2, red, dlist, nd, lane);
+                else tree.push(sd, red, dlist, nd, lane);
+            } else {  // several groups per thread: each is added by itself
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    sd += __shfl_xor_sync(0xffffffffu, sd, o);
+                    sd2 += __shfl_xor_sync(0xffffffffu, sd2, o);
+                }
+                if (lane == 0) {
+                    wacc_add(red[op], sd);
+                    if (pair) wacc_add(red[op + 1], sd2);
+                }
+            }
+        }
+        q += pair;
+    }
+}
+
+// Every run of the pass on one staged pair of tiles: groups of 8 amplitudes,
+// one group per thread at a time, a barrier after each run. ucode / umode / ucol:
+// each op's case, U^dagger class and, for a permutation, its source column per row.
+template <typename T>
+__device__ __forceinline__ void adj_tile_runs(uint32_t tile, int m, const AdjSweepArgs& a,
+                                              const cplx<T>* __restrict__ ush, const AdjRun* __restrict__ runs,
+                                              int nruns, const uint16_t* __restrict__ sbase,
+                                              const uint8_t* __restrict__ prog, const uint8_t* __restrict__ ucode,
                                               const uint8_t* __restrict__ umode, const uint8_t* __restrict__ ucol,
+                                              const uint8_t* __restrict__ dlist, int nd,
                                               typename WAccOf<T>::type* __restrict__ red, int tid, int nthr) {
     using C = cplx<T>;
-    constexpr int D = 1 << R;
-    const int warp = tid >> 5, lane = tid & 31;
-    for (int i0 = 0; i0 < a.n_ops;) {
-        const int nr = a.run_len[i0];
-        int rp[R], srt[R];
-#pragma unroll
-        for (int j = 0; j < R; ++j) rp[j] = srt[j] = a.run_pos[i0][j];
-#pragma unroll
-        for (int x = 1; x < R; ++x)
-#pragma unroll
-            for (int y = x; y > 0; --y)
-                if (srt[y - 1] > srt[y]) {
-                    const int t = srt[y];
-                    srt[y] = srt[y - 1];
-                    srt[y - 1] = t;
-                }
+    constexpr int D = 8;
+    const int lane = tid & 31;
+    const uint32_t groups = 1u << (m - 3);
+    const bool one = groups <= uint32_t(nthr);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const uint32_t lam = uint32_t(sizeof(C)) << m;  // the co-state's tile follows the state's
+    AdjTree<T> tree;
+    tree.t = 0;
+    for (int i = 0; i < nruns; ++i) {
+        const AdjRun& run = runs[i];
         uint32_t soff[D];
-#pragma unroll
-        for (int c = 0; c < D; ++c) {
-            uint32_t o = 0;
-#pragma unroll
-            for (int j = 0; j < R; ++j) o |= uint32_t((c >> j) & 1) << rp[j];
-            soff[c] = swz<T>(o);
-        }
-        const uint32_t groups = 1u << (m - R);
+        soff[0] = 0;
+        soff[1] = run.off[0];
+        soff[2] = run.off[1];
+        soff[4] = run.off[2];
+        soff[3] = soff[1] ^ soff[2];
+        soff[5] = soff[1] ^ soff[4];
+        soff[6] = soff[2] ^ soff[4];
+        soff[7] = soff[3] ^ soff[4];
         for (uint32_t gb = 0; gb < groups; gb += uint32_t(nthr)) {  // every thread the same trip count
             const uint32_t g = gb + uint32_t(tid);
             const bool ok = g < groups;
-            uint32_t base = ok ? g : 0u;
-#pragma unroll
-            for (int j = 0; j < R; ++j) base = ((base >> srt[j]) << (srt[j] + 1)) | (base & ((1u << srt[j]) - 1));
-            const uint32_t sb = swz<T>(base);
+            uint32_t sb = sbase[i * nthr + tid];
+            if (!one)  // the bits above the thread's
+                for (int j = 31 - __clz(nthr); j < m - 3; ++j) sb ^= (g >> j) & 1u ? uint32_t(run.base[j]) : 0u;
+            sb *= uint32_t(sizeof(C));
             C p[D], l[D];
 #pragma unroll
             for (int c = 0; c < D; ++c) {
-                p[c] = ok ? pt[sb ^ soff[c]] : mk<T>(T(0), T(0));
-                l[c] = ok ? lt[sb ^ soff[c]] : mk<T>(T(0), T(0));
+                const unsigned char* at = smem_raw + (tile + (sb ^ soff[c]));
+                p[c] = ok ? *reinterpret_cast<const C*>(at) : mk<T>(T(0), T(0));
+                l[c] = ok ? *reinterpret_cast<const C*>(at + lam) : mk<T>(T(0), T(0));
             }
-            for (int q = 0; q < nr; ++q) {
-                const int op = i0 + q;
-                const int gen = a.op_gcls[op];
-                const bool want = gen != kGenNone;
-                T sd = T(0);
-                if (a.op_k[op] == 1)
-                    adj_apply1<R>(p, l, a.op_lpos[op][0], ush + op * 16, umode[op], gen, a.gval[op], sd);
-                else
-                    adj_apply2<R>(p, l, a.op_lpos[op][0], a.op_lpos[op][1], ush + op * 16, umode[op], gen,
-                                  ucol + op * 4, a.gval[op], a.gcol[op], sd);
-                if (want) {  // uniform over the CTA: every lane reaches the shuffles
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) sd += __shfl_xor_sync(0xffffffffu, sd, o);
-                    if (lane == 0) wacc_add(red[op * kAdjMaxWarps + warp], sd);
+            const int np = one ? prog[i] : 0;
+            if (np > 0) {
+                const C* u = ush + int(run.first) * 16;
+                T s0, s1;
+                adj_pair<0>(p, l, u, s0, s1);
+                tree.push2(s0, s1, red, dlist, nd, lane);
+                if (np > 1) {
+                    adj_pair<1>(p, l, u + 32, s0, s1);
+                    tree.push2(s0, s1, red, dlist, nd, lane);
+                    if (np > 2) {
+                        adj_pair<2>(p, l, u + 64, s0, s1);
+                        tree.push2(s0, s1, red, dlist, nd, lane);
+                    }
                 }
+            } else {
+                adj_run_ops<T>(p, l, run.first, run.count, one, a, ush, ucode, umode, ucol, tree, dlist, nd, red, lane);
             }
             if (ok) {
 #pragma unroll
                 for (int c = 0; c < D; ++c) {
-                    pt[sb ^ soff[c]] = p[c];
-                    lt[sb ^ soff[c]] = l[c];
+                    unsigned char* at = smem_raw + (tile + (sb ^ soff[c]));
+                    *reinterpret_cast<C*>(at) = p[c];
+                    *reinterpret_cast<C*>(at + lam) = l[c];
                 }
             }
         }
         __syncthreads();
-        i0 += nr;
     }
+    tree.finish(red, dlist, nd, lane);
 }
 
 // Length of the run of ops starting at op0 on the same sites (same k and tile bits, in order).
@@ -618,11 +899,26 @@ __device__ __forceinline__ int adj_tile_ops(cplx<T>* pt, cplx<T>* lt, int m, con
     return r;
 }
 
-// complex64: 256 threads and 3 CTAs per SM (80 registers): the passes are latency-bound, and
-// the third CTA's warps outweigh the few register spills (64-set, 20-qubit gradient 0.42 ->
-// 0.36 s); complex128 keeps 128 registers (up to 512 threads when one CTA fits)
+// bytes of the kernel's shared memory before the runs, and in all
 template <typename T>
-__global__ void __launch_bounds__(sizeof(T) == 4 ? 256 : kAdjMaxThreads, sizeof(T) == 4 ? 3 : 1) adjoint_sweep_kernel(cplx<T>* __restrict__ phi,
+__host__ __device__ inline size_t adj_runs_offset(int m, int H, int n_ops, int nbuf) {
+    const size_t o = sizeof(cplx<T>) * ((size_t(2 * nbuf) << m) + size_t(n_ops) * 16) + sizeof(uint64_t) * (size_t(1) << H) +
+                     sizeof(double) * size_t(n_ops) * kAdjMaxWarps + size_t(n_ops) * 8;
+    return (o + 15) & ~size_t(15);
+}
+template <typename T>
+__host__ __device__ inline size_t adj_smem_bytes(int m, int H, int n_ops, int n_runs, int threads, int nbuf) {
+    return adj_runs_offset<T>(m, H, n_ops, nbuf) + (sizeof(AdjRun) + sizeof(uint16_t) * threads) * size_t(n_runs) +
+           sizeof(AdjMap);
+}
+
+// complex64: 256 threads and 2 CTAs per SM (128 registers): the straight-line programs spill at the 80
+// registers of a third CTA (64 sets of 20 qubits, 28 passes: 38.2 ms with three, 34.8 ms with two, 74.5 ms
+// before the map and the programs); complex128 keeps 128 registers (up to 512 threads when one CTA fits).
+// Bound by instruction issue: two thirds of it the two-by-two products and derivative sums, the rest
+// addresses, reductions and the copies; HBM is at a quarter.
+template <typename T>
+__global__ void __launch_bounds__(sizeof(T) == 4 ? 256 : kAdjMaxThreads, sizeof(T) == 4 ? 2 : 1) adjoint_sweep_kernel(cplx<T>* __restrict__ phi,
                                                                        cplx<T>* __restrict__ lam,
                                                                        const cplx<T>* __restrict__ mats,
                                                                        const __grid_constant__ AdjSweepArgs a,
@@ -632,13 +928,28 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 256 : kAdjMaxThreads, sizeof(
     const int L = a.L, H = a.H, m = a.m;
     const int nwarps = blockDim.x >> 5;
     // layout: nbuf x (phi tile, lam tile) | ush (n_ops x 16 complex: U^dagger of the current state) |
-    //         hoff (2^H uint64) | red (n_ops x kAdjMaxWarps accumulators, 8 bytes) | umode (n_ops) | ucol (n_ops x 4)
+    //         hoff (2^H uint64) | red (kAdjMaxWarps x n_ops accumulators, 8 bytes) | umode, ucode, dlist (n_ops each) | ucol (n_ops x 4) |
+    //         prog (n_ops) | runs (n_runs) | map | sbase (n_runs x threads)
     C* bufs = reinterpret_cast<C*>(smem_raw);
     C* ush = bufs + (size_t(2 * nbuf) << m);
     uint64_t* hoff = reinterpret_cast<uint64_t*>(ush + size_t(a.n_ops) * 16);
     auto* red = reinterpret_cast<typename WAccOf<T>::type*>(hoff + (size_t(1) << H));
     uint8_t* umode = reinterpret_cast<uint8_t*>(red + size_t(a.n_ops) * kAdjMaxWarps);
-    uint8_t* ucol = umode + a.n_ops;
+    uint8_t* ucode = umode + a.n_ops;
+    uint8_t* dlist = ucode + a.n_ops;
+    uint8_t* ucol = dlist + a.n_ops;
+    uint8_t* prog = ucol + 4 * a.n_ops;
+    AdjRun* runs = reinterpret_cast<AdjRun*>(smem_raw + adj_runs_offset<T>(m, H, a.n_ops, nbuf));
+    AdjMap* map = reinterpret_cast<AdjMap*>(runs + a.n_runs);
+    uint16_t* sbase = reinterpret_cast<uint16_t*>(map + 1);  // [run][thread]: the thread's group, images XORed
+    uint32_t out0 = 0;                                       // image of this thread's first amplitude at the end
+    auto* myred = red + size_t(threadIdx.x >> 5) * a.n_ops;  // this warp's accumulators
+    int nd = 0;                                              // derivatives, in order
+    for (int i = 0; i < a.n_ops; ++i)
+        if (a.op_gcls[i] != kGenNone) {
+            if (threadIdx.x == 0) dlist[nd] = uint8_t(i);
+            ++nd;
+        }
     int64_t staged = -1;  // state whose matrices sit in ush
     for (uint32_t h = threadIdx.x; h < (1u << H); h += blockDim.x) {
         uint64_t o = 0;
@@ -653,13 +964,21 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 256 : kAdjMaxThreads, sizeof(
     const uint64_t my_chunks = a.chunks > blockIdx.x ? (a.chunks - 1 - blockIdx.x) / gridDim.x + 1 : 0;
     const uint64_t my_tiles = my_chunks * a.chunk_tiles;
     auto tile_of = [&](uint64_t i) -> uint64_t {
-        return (uint64_t(blockIdx.x) + (i / a.chunk_tiles) * gridDim.x) * a.chunk_tiles + i % a.chunk_tiles;
+        return ((uint64_t(blockIdx.x) + (i >> a.chunk_shift) * gridDim.x) << a.chunk_shift) + (i & (a.chunk_tiles - 1));
     };
     auto base_of = [&](uint64_t w) -> uint64_t {
-        const uint64_t b = w / a.tiles, o = w - b * a.tiles;
-        uint64_t base = b * uint64_t(a.sv_stride);
-        for (int j = 0; j < a.n_outer; ++j) base |= ((o >> j) & 1ull) << a.outer_bits[j];
-        return base;
+        // the tile's bits at the outer positions, a bit per lane (called by whole warps)
+        const uint64_t b = w >> a.tile_shift, o = w & (a.tiles - 1);
+        uint32_t lo = 0, hi = 0;
+        for (int j = threadIdx.x & 31; j < a.n_outer; j += 32)
+            if ((o >> j) & 1ull) {
+                const int ob = a.outer_bits[j];
+                if (ob < 32) lo |= 1u << ob;
+                else hi |= 1u << (ob - 32);
+            }
+        lo = __reduce_or_sync(0xffffffffu, lo);
+        if (a.n > 32) hi = __reduce_or_sync(0xffffffffu, hi);
+        return b * uint64_t(a.sv_stride) + ((uint64_t(hi) << 32) | lo);
     };
     auto load_async = [&](uint64_t w, C* dp, C* dl) {
         const uint64_t base = base_of(w);
@@ -683,7 +1002,7 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 256 : kAdjMaxThreads, sizeof(
         } else {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
-        const int64_t b = int64_t(w / a.tiles);
+        const int64_t b = int64_t(w >> a.tile_shift);
         if (b != staged) {  // once per chunk: every op's U^dagger for this state (previous readers done: loop-end barrier)
             const C* mb = mats + b * a.mat_stride;
             for (int e = threadIdx.x; e < a.n_ops * 16; e += blockDim.x) {
@@ -725,35 +1044,88 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 256 : kAdjMaxThreads, sizeof(
                         else if (c4[0] == 0 && c4[1] == 2 && c4[2] == 1 && c4[3] == 3) mode = kAdjPermSwap;
                     }
                     umode[op] = uint8_t(mode);
+                    int code = kCodeTwo;
+                    if (d == 2) {
+                        C* w = ush + op * 16;
+                        const int gen = adj_gen1(a, op);
+                        if (mode == kAdjReal) {
+                            w[4] = mk<T>(u[0].x, u[1].x);
+                            w[5] = mk<T>(u[2].x, u[3].x);
+                        } else {
+                            w[4] = u[0];
+                            w[5] = u[3];
+                        }
+                        const bool im = gen == kGenFlipIm;
+                        w[6] = mk<T>(T(im ? a.gval[op][0].y : a.gval[op][0].x), T(im ? a.gval[op][1].y : a.gval[op][1].x));
+                        code = kCodeOne + (a.op_lpos[op][0] * 4 + mode) * 6 + adj_gen_index(gen);
+                    }
+                    ucode[op] = uint8_t(code);
                 }
+                __syncthreads();
+                // the Z-like, Y-like pairs: both ops of a pair in one run (each op looks at its successor only)
+                for (int op = threadIdx.x; op + 1 < a.n_ops; op += blockDim.x) {
+                    const int P = a.op_lpos[op][0];
+                    const int first = kCodeOne + (P * 4 + kAdjDiag) * 6 + 1, second = kCodeOne + (P * 4 + kAdjReal) * 6 + 3;
+                    if (a.run_len[op + 1] == 0 && ucode[op] == first && ucode[op + 1] == second)
+                        ucode[op] = uint8_t(kCodePair + P);
+                }
+                __syncthreads();
+                if (threadIdx.x < 32) adj_build_runs<T>(runs, map, a, umode, prog, ucode, threadIdx.x);
+                __syncthreads();
+                const int tb = min(m - 3, 31 - __clz(int(blockDim.x)));  // group bits that the thread number gives
+                for (int i = 0; i < map->nruns; ++i) {
+                    uint32_t sb = runs[i].flip;
+                    for (int j = 0; j < tb; ++j) sb ^= (threadIdx.x >> j) & 1u ? uint32_t(runs[i].base[j]) : 0u;
+                    sbase[i * int(blockDim.x) + int(threadIdx.x)] = uint16_t(sb);
+                }
+                out0 = map->flip;
+                for (int j = 0; j < m; ++j) out0 ^= ((per16 * threadIdx.x) >> j) & 1u ? uint32_t(map->bit[j]) : 0u;
             }
             staged = b;
         }
         __syncthreads();
         if (a.rbits == 3) {
-            adj_tile_runs<T, 3>(pt, lt, m, a, ush, umode, ucol, red, threadIdx.x, blockDim.x);
+            adj_tile_runs<T>(uint32_t(sizeof(C)) * (uint32_t(2 * slot) << m), m, a, ush, runs, map->nruns, sbase, prog, ucode, umode, ucol, dlist, nd, myred, threadIdx.x,
+                             blockDim.x);
         } else {
             for (int op = 0; op < a.n_ops;) {
-                op += a.op_k[op] == 1 ? adj_tile_ops<T, 1>(pt, lt, m, a, op, ush, red, threadIdx.x, blockDim.x)
-                                      : adj_tile_ops<T, 2>(pt, lt, m, a, op, ush, red, threadIdx.x, blockDim.x);
+                op += a.op_k[op] == 1 ? adj_tile_ops<T, 1>(pt, lt, m, a, op, ush, myred, threadIdx.x, blockDim.x)
+                                      : adj_tile_ops<T, 2>(pt, lt, m, a, op, ush, myred, threadIdx.x, blockDim.x);
                 __syncthreads();
             }
         }
         const uint64_t base = base_of(w);
-        for (uint32_t e = per16 * threadIdx.x; e < (1u << m); e += per16 * blockDim.x) {
+        if (a.rbits == 3) {  // through the map: the two amplitudes of a 16-byte store may lie apart
+            const int lg = 31 - __clz(int(per16 * blockDim.x));
+            uint32_t s1 = out0, it = 0;
+            for (uint32_t e = per16 * threadIdx.x; e < (1u << m); e += per16 * blockDim.x, ++it) {
+                const uint64_t dst = base + (hoff[e >> L] | (e & lmask));
+                for (uint32_t x = it & ~(it - 1), j = 0; it != 0 && (1u << j) <= x; ++j) s1 ^= map->bit[lg + j];
+                if constexpr (per16 == 2) {
+                    const uint32_t s2 = s1 ^ map->bit[0];
+                    const C a0 = pt[s1], a1 = pt[s2], b0 = lt[s1], b1 = lt[s2];
+                    *reinterpret_cast<float4*>(phi + dst) = make_float4(a0.x, a0.y, a1.x, a1.y);
+                    *reinterpret_cast<float4*>(lam + dst) = make_float4(b0.x, b0.y, b1.x, b1.y);
+                } else {
+                    phi[dst] = pt[s1];
+                    lam[dst] = lt[s1];
+                }
+            }
+        } else for (uint32_t e = per16 * threadIdx.x; e < (1u << m); e += per16 * blockDim.x) {
             const uint64_t dst = base + (hoff[e >> L] | (e & lmask));
             *reinterpret_cast<float4*>(phi + dst) = *reinterpret_cast<const float4*>(pt + swz<T>(e));
             *reinterpret_cast<float4*>(lam + dst) = *reinterpret_cast<const float4*>(lt + swz<T>(e));
         }
-        if (i % a.chunk_tiles == a.chunk_tiles - 1) {  // chunk done: one partial per op, accumulators reset
-            const uint64_t chunk = w / a.chunk_tiles;
+        if ((i & (a.chunk_tiles - 1)) == a.chunk_tiles - 1) {  // chunk done: one partial per op, accumulators reset
+            __syncthreads();  // every warp's sums of this tile are in
+            const uint64_t chunk = w >> a.chunk_shift;
             for (int op = threadIdx.x; op < a.n_ops; op += blockDim.x) {
                 if (a.op_out[op] < 0) continue;
-                auto* row = red + op * kAdjMaxWarps;
                 double t = 0.0;
                 for (int wp = 0; wp < nwarps; ++wp) {
-                    t += wacc_value(row[wp]);
-                    wacc_zero(row[wp]);
+                    auto& r = red[size_t(wp) * a.n_ops + op];
+                    t += wacc_value(r);
+                    wacc_zero(r);
                 }
                 partials[chunk * a.n_ops + op] = t;
             }
@@ -787,12 +1159,6 @@ using namespace qgb_host;
 namespace {
 
 template <typename T>
-size_t adj_smem_bytes(int m, int H, int n_ops, int nbuf) {
-    return sizeof(cplx<T>) * ((size_t(2 * nbuf) << m) + size_t(n_ops) * 16) + sizeof(uint64_t) * (size_t(1) << H) +
-           sizeof(double) * size_t(n_ops) * kAdjMaxWarps + size_t(n_ops) * 5;
-}
-
-template <typename T>
 int launch_adj(void* phi, void* lam, const void* mats, const AdjSweepArgs& a, double* partials, cudaStream_t st) {
     auto kern = adjoint_sweep_kernel<T>;
     static bool attr = false;
@@ -802,7 +1168,8 @@ int launch_adj(void* phi, void* lam, const void* mats, const AdjSweepArgs& a, do
         attr = true;
     }
     for (int nbuf = 2; nbuf >= 1; --nbuf) {
-        const size_t smem = adj_smem_bytes<T>(a.m, a.H, a.n_ops, nbuf);
+        // (the table for 512 threads where a block may get them)
+        const size_t smem = adj_smem_bytes<T>(a.m, a.H, a.n_ops, a.n_runs, sizeof(T) == 8 ? 512 : 256, nbuf);
         if (smem > 227 * 1024) continue;
         int per_sm = 0, threads = 256;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem) != cudaSuccess)
@@ -951,6 +1318,7 @@ extern "C" int qgb_adjoint_sweep_step(void* phi, void* lam, int dtype, int n, co
             for (int b = 0; b < m && nrp < a.rbits; ++b)
                 if (!((bits >> b) & 1u)) a.run_pos[i0][nrp++] = b;
             a.run_len[i0] = i - i0;
+            ++a.n_runs;
             for (int o = i0; o < i; ++o)
                 for (int j = 0; j < a.op_k[o]; ++j)
                     for (int r = 0; r < a.rbits; ++r)
@@ -967,6 +1335,8 @@ extern "C" int qgb_adjoint_sweep_step(void* phi, void* lam, int dtype, int n, co
     const int cps = adj_chunks_per_state(a.tiles, batch);
     a.chunk_tiles = a.tiles / uint64_t(cps);
     a.chunks = uint64_t(batch) * uint64_t(cps);
+    a.tile_shift = n - m;
+    a.chunk_shift = __builtin_ctzll(a.chunk_tiles);
     const size_t need = sizeof(double) * size_t(a.chunks) * size_t(a.n_ops);
     if (any_out && (!scratch || scratch_bytes < need))
         return set_error(QGB_ESCRATCH, "scratch of %zu bytes needed (qgb_adjoint_sweep_scratch_bytes)", need);

@@ -90,7 +90,8 @@ class _Runner:
                                device_fusion=True)
         else:
             plan = compile_ops(ops, n, mode=self.sim.mode, width=self.sim.fusion_width, tile_bits=self.sim.tile_bits,
-                               low_bits=self.sim.low_bits, max_sweep_k=kcap, itemsize=isz, device_fusion=True)
+                               low_bits=self.sim.low_bits, max_sweep_k=kcap, itemsize=isz, device_fusion=True, pack=True,
+                               pad=self.sim._pad())
         self.sim.initialize_state()  # |0..0>, a bitstring or a given array (copied), as the simulator starts
         psi = self.sim.state.detach().reshape(-1)
         self.sim.state = None  # psi is the only reference: no extra state-sized buffer

@@ -19,7 +19,8 @@ Three kinds of choice:
 seeded workload of that size the first time the size is seen and caches the
 fastest; otherwise it returns the defaults measured on GB300 (complex64
 statevectors: 6-qubit fused blocks on the tensor cores from 13 qubits, else
-4-qubit blocks in one tile sweep; complex128: 3-qubit blocks in 13-bit tile sweeps;
+4-qubit blocks in one tile sweep; complex128: 5-qubit blocks in fixed point on the
+tensor cores from 17 qubits, else 3-qubit blocks in 13-bit tile sweeps;
 trajectories: 13-bit tiles for complex64, 12 for complex128). The cache is a
 JSON file at ``$QGB_AUTOTUNE_CACHE`` (default
 ``~/.cache/qaravan_gb300/autotune.json``). ``select`` is the decision rule
@@ -36,7 +37,8 @@ import torch
 SV_CANDIDATES = {
     torch.complex64: [("fused", 6, 14), ("fused", 5, 14), ("fused", 4, 14), ("tcsweep", 5, 13), ("sweep", 4, 14),
                       ("sweep", 3, 12)],
-    torch.complex128: [("sweep", 3, 13), ("sweep", 2, 13), ("sweep", 4, 12), ("fused", 3, 13), ("fused", 2, 13)],
+    torch.complex128: [("sweep", 3, 13), ("sweep", 2, 13), ("sweep", 4, 12), ("fused", 5, 13), ("fused", 3, 13),
+                       ("fused", 2, 13)],
 }
 TRAJ_CANDIDATES = {torch.complex64: [11, 12, 13, 14], torch.complex128: [11, 12, 13]}
 SWEEP_CANDIDATES = [(12, 2), (12, 3), (12, 4), (13, 3), (13, 4), (14, 3), (14, 4)]
@@ -111,7 +113,15 @@ def default_sv(n, dtype):
         # (depth-20 brickwork: 12 qubits 156 us, 460 us with a launch per 4-qubit block)
         tc = n >= 13 and _lib.lib().qgb_get_dense_impl() >= 1
         return ("fused", 6, 14) if tc else ("sweep", 4, 14)
-    return ("sweep", 3, 13)
+    # depth-20 brickwork, 5-qubit blocks in fixed point on the tensor cores against double-float tile
+    # sweeps: 16 qubits 593 / 552 us, 17 qubits 595 / 1015 us, 20 qubits 1.51 / 3.51 ms
+    return ("fused", 5, 13) if n >= 17 and fixed_point() else ("sweep", 3, 13)
+
+
+def fixed_point() -> bool:
+    """Whether 5-qubit complex128 blocks may run in fixed point on the tensor cores."""
+    from . import _lib
+    return _lib.lib().qgb_get_dense_impl() >= 1 and _lib.lib().qgb_get_c128_arith() == 1
 
 
 def default_traj(n, dtype):

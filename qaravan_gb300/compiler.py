@@ -510,7 +510,7 @@ def _remember_plan(key, plan):
 
 
 def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, max_sweep_k=5, itemsize=8,
-                device_fusion=False, pack=False):
+                device_fusion=False, pack=False, pad=0):
     """Compile an op sequence (with ``None`` marking a renormalisation point)
     into a :class:`Plan`.
 
@@ -522,7 +522,10 @@ def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, 
     of shared memory. ``device_fusion``: block matrices are left as
     :class:`Recipe` objects for the executor to compose on the GPU. ``pack``
     (dense passes of device-fused blocks): the blocks of :func:`fuse_frontier`,
-    run from either end, when they are fewer -- fewer passes, the ops in another of their valid orders.
+    run from either end, when they are fewer; every block of fewer than ``pad`` bits
+    widened to ``pad`` (identity on the lowest free bits) -- fewer passes, the ops in another of their
+    valid orders. The kernel that ``pad`` serves takes unitary blocks of that width: a segment with
+    another op or a wider one runs as 3-bit blocks in tile sweeps.
     """
     tile_bits = min(tile_bits, 14 if itemsize <= 8 else 13)
     # unitarity of every op with a matrix, batched once (the plan key, trace checks and fusion use it)
@@ -556,7 +559,7 @@ def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, 
     key = None
     if device_fusion and mode != "gate" and ops and not any(o is not None and o.kind == "pauli_mix" for o in ops):
         flags = [ucache[id(o)] for o in ops if o is not None]
-        key = (nbits, mode, width, tile_bits, low_bits, max_sweep_k, itemsize, pack,
+        key = (nbits, mode, width, tile_bits, low_bits, max_sweep_k, itemsize, pack, pad,
                tuple(None if o is None else tuple(o.bits) for o in ops), tuple(flags), tuple(_pair_offsets(ops)),
                tp_flags)
         plan = _cached_plan(key, ops)
@@ -590,16 +593,22 @@ def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, 
         # qubits; density-matrix segments keep the trace chain of the dense passes instead
         tcs = (mode == "tcsweep" and nbits >= 14 and max(len(o.bits) for o in seg) <= 5
                and not any(o.pair is not None or o.kind == "channel" for o in seg))
-        w = 5 if tcs else max(width, max(len(o.bits) for o in seg))
+        widest = max(len(o.bits) for o in seg)
+        padded = bool(pad) and mode == "fused" and widest <= pad and all(uflags)
+        w = 5 if tcs else max(width if padded or not pad else 3, widest)
         if device_fusion:
             base = len(plan.op_matrices)
             plan.op_matrices.extend(np.ascontiguousarray(o.matrix, dtype=np.complex128) for o in seg)
             sym = fuse_symbolic(seg, w)
-            if pack and mode == "fused":
+            if pack and mode == "fused" and (padded or not pad):
                 n = len(seg)
                 back = [SymBlock(b.bits, [n - 1 - i for i in reversed(b.ops)])
                         for b in reversed(fuse_frontier(seg[::-1], w))]
                 sym = min(sym, fuse_frontier(seg, w), back, key=len)  # the first of the shortest
+                for b in sym:
+                    if padded and len(b.bits) < min(pad, nbits):
+                        free = [x for x in range(nbits) if x not in b.bits]
+                        b.bits = sorted(b.bits + free[:min(pad, nbits) - len(b.bits)], reverse=True)
             blocks = [Block(b.bits, Recipe(list(b.bits), [(base + i, list(seg[i].bits)) for i in b.ops]), b.n_ops)
                       for b in sym]
             bflags = [all(uflags[i] for i in b.ops) for b in sym]
@@ -612,7 +621,7 @@ def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, 
         if tcs:
             _plan_tc_sweeps(plan, blocks, bflags, nbits, low_bits)
             continue
-        if mode in ("fused", "tcsweep") or w > max_sweep_k or tile_bits <= 0:
+        if mode == "tcsweep" or (mode == "fused" and (padded or not pad)) or w > max_sweep_k or tile_bits <= 0:
             for b, u, w_ in zip(blocks, bflags, wflags):
                 plan.steps.append(DenseStep(list(b.bits), plan.add_matrix(b.matrix), u, w_))
             continue

@@ -291,6 +291,10 @@ int apply_dense_bits(void* sv, int dtype, int nbits, const int* in_bits, const i
                                     pass);
         if (rc != QGB_EDECLINE) return rc;
     }
+    if (dtype == QGB_C128 && pass.unitary && c128_arith() == 1) {
+        const int rc = try_dense_oz(sv, op, nbits, a.sorted, in_bits, out_bits, k, batch, st, pass);
+        if (rc != QGB_EDECLINE) return rc;
+    }
     const int rc = dtype == QGB_C64 ? dispatch_dense<float>(sv, op, a, st) : dispatch_dense<double>(sv, op, a, st);
     if (rc || !pass.scale) return rc;
     // the CUDA-core kernels take no factor: one more pass multiplies the result by it

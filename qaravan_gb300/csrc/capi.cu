@@ -160,6 +160,9 @@ extern "C" int qgb_check_status(void* stream) {
     const int tc = qgb_host::tc_status_read_clear();
     if (tc < 0) return qgb_host::set_error(QGB_ECUDA, "tensor-core status read failed");
     if (tc != 0) return qgb_host::set_error(QGB_ETIMEOUT, "a tensor-core completion wait gave up (code %d)", tc);
+    const int oz = qgb_host::oz_status_read_clear();
+    if (oz < 0) return qgb_host::set_error(QGB_ECUDA, "fixed-point block status read failed");
+    if (oz != 0) return qgb_host::set_error(QGB_ETIMEOUT, "a fixed-point block's completion wait gave up (code %d)", oz);
     const int tcs = qgb_host::tcs_status_read_clear();
     if (tcs < 0) return qgb_host::set_error(QGB_ECUDA, "tensor-core sweep status read failed");
     if (tcs != 0) return qgb_host::set_error(QGB_ETIMEOUT, "a tensor-core sweep wait gave up (code %d)", tcs);

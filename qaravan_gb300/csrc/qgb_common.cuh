@@ -208,6 +208,10 @@ struct DensePass {
 };
 int try_dense_tc(void* sv, const void* op, int nbits, const int* sorted, const int* in_bits, const int* out_bits,
                  int k, int64_t op_stride, int64_t batch, int64_t sv_stride, cudaStream_t st, const DensePass& pass);
+int try_dense_oz(void* sv, const void* op, int nbits, const int* sorted, const int* in_bits, const int* out_bits, int k,
+                 int64_t batch, cudaStream_t st, const DensePass& pass);
+int c128_arith();
+int oz_status_read_clear();
 int tc_status_read_clear();
 int tcs_status_read_clear();
 int dmb_status_read_clear();

@@ -293,7 +293,8 @@ class Executor:
                                "op_action")
                     link += 1
                 else:
-                    fn = L.qgb_op_action if mode == "off" else L.qgb_op_action_unitary
+                    c128 = unitary and mats is self.mats and self.code == _lib.QGB_C128  # fixed-point blocks
+                    fn = L.qgb_op_action if mode == "off" and not c128 else L.qgb_op_action_unitary
                     _lib.check(fn(ptr, self.code, nb, sites, k, mptr + off * self.itemsize,
                                   mat_stride if mat_stride else 0, batch, stride, st), "op_action")
                     link = 0
@@ -355,7 +356,8 @@ class Executor:
         entries and trace measurements that ``run`` takes step by step. The norm
         chain knows its length here: its first epoch is cut so that the chain's last
         pass opens an epoch and corrects the drift of every pass but its own, and
-        unitary blocks on the CUDA cores, which do not drift, leave it running."""
+        unitary blocks on the CUDA cores, which do not drift, leave it running. Unitary
+        complex128 blocks are marked in every mode: the mark picks the kernel, no factor."""
         calls, chains, t_since, t_pending = [], [[]], 0, False
         if tchain:
             calls.append((_lib.QGB_CALL_TRACE, None, 0, 1, 0, None))
@@ -376,7 +378,7 @@ class Executor:
             elif unitary and mode == "chain" and on_tc:
                 chains[-1].append(len(calls))
                 calls.append((_lib.QGB_CALL_CHAIN, sites, k, len(chains[-1]) - 1, off, None))
-            elif unitary and mode != "off":
+            elif unitary and (mode != "off" or self.code == _lib.QGB_C128):
                 calls.append((_lib.QGB_CALL_ROWS, sites, k, 0, off, None))
             else:
                 calls.append((_lib.QGB_CALL_OP, sites, k, 0, off, None))

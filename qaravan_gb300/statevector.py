@@ -102,8 +102,9 @@ class StatevectorSim:
         # measurement now with QGB_AUTOTUNE=1, else the defaults measured on GB300:
         # complex64 -> dense fused blocks, one HBM pass each, 6-qubit blocks on the tensor cores
         # from 13 qubits up (half the passes of 4-qubit blocks at the same speed per pass, fastest
-        # measured on the 28-qubit brickwork), 4-qubit blocks in one tile sweep below; complex128 -> 3-qubit blocks grouped into tile sweeps
-        # (arithmetic dominates, so fewer passes win))
+        # measured on the 28-qubit brickwork), 4-qubit blocks in one tile sweep below; complex128 ->
+        # 5-qubit blocks in fixed point on the tensor cores from 17 qubits up, below 3-qubit blocks
+        # grouped into tile sweeps (arithmetic dominates, so fewer passes win))
         if mode == "auto":
             from . import autotune
             a_mode, a_width, a_tile = autotune.choose_sv(circ.num_sites, dtype)
@@ -140,6 +141,13 @@ class StatevectorSim:
         else:
             raise ValueError("init_state must be a NumPy array, Torch tensor, or a bitstring")
 
+    def _pad(self):
+        """Width every fused block is widened to: complex128 blocks of 5 qubits run in
+        fixed point on the tensor cores (at least 12 qubits), narrower ones on the FP64 pipe."""
+        from . import autotune
+        return 5 if (self.dtype == torch.complex128 and self.mode == "fused" and self.fusion_width == 5
+                     and self.num_sites >= 12 and autotune.fixed_point()) else 0
+
     def compile(self):
         if self._exec is None:
             seq = circuit_ops(self.circ, build=True, nm=self.nm)
@@ -147,7 +155,8 @@ class StatevectorSim:
             kcap = 5 if self.dtype == torch.complex64 else 4
             plan = compile_ops(ops, self.num_sites, mode=self.mode, width=self.fusion_width,
                                tile_bits=self.tile_bits, low_bits=self.low_bits, max_sweep_k=kcap,
-                               itemsize=torch.empty(0, dtype=self.dtype).element_size(), device_fusion=True, pack=True)
+                               itemsize=torch.empty(0, dtype=self.dtype).element_size(), device_fusion=True, pack=True,
+                               pad=self._pad())
             self._exec = Executor(plan, self.dtype, self.device)
         return self._exec
 

@@ -29,6 +29,17 @@
 //    1 / sqrt(N_end). A last pass writes the normalised state to the
 //    trajectory's slot.
 //
+// What bounds it: instructions, on 16 warps an SM (one CTA; the tile buffers fill shared memory).
+// An op of a 16-amplitude group takes 96 to 128 FP32 instructions (op, K0, weights); the rest was
+// overhead, 400 instructions an op in all: a select per damped component for a jump that hardly
+// ever happens, a shuffle butterfly and a single lane's update per channel, moves of the group
+// where the switches on positions join, and index arithmetic per tile and run. Now one switch per
+// op into straight-line cases, jumps apart, weights summed 16 channels at a time through shared
+// memory in the butterfly's order, half the products for x rotations and real ops, diagonal ops by
+// a factor per local index, offsets from per-run tables: 230 instructions an op, and 152
+// trajectories of the 20-qubit Ising circuit, 3 Trotter steps, from 20.0 to 12.2 ms; every
+// rounding stays, so the states are the same bit for bit.
+//
 // Random numbers: Philox4x32-10 (philox.cuh). Pauli of site j after gate g:
 // counter (g, trajectory, 2j, 0), as the gate-by-gate kernel; jump threshold
 // number i of a trajectory: counter (i, trajectory, 0, 2).
@@ -41,8 +52,9 @@ using TrajSweepDesc = qgb_traj_sweep;
 using TrajOpDesc = qgb_traj_op;
 
 constexpr int kTrajMaxOps = 128;    // ops per sweep
+constexpr int kTrajMaxSmem = 222 * 1024;  // dynamic shared memory of a CTA
 constexpr int kTrajMaxJumps = 16;   // jumps inside one sweep of one trajectory
-constexpr int kTrajThreads = 512;  // 16 warps, one register group each at a time (98 registers): 15 % faster than
+constexpr int kTrajThreads = 512;  // 16 warps, one register group each at a time (100 registers): 15 % faster than
                                     // 8 warps with two groups each (215 registers), the latency-bound runs
 
 struct TrajRunArgs {
@@ -82,15 +94,35 @@ template <typename C> __device__ __forceinline__ C cmul(const C& a, const C& b) 
     return r;
 }
 
-template <int R, int P, typename C>
-__device__ __forceinline__ void reg_op1(C (&v)[1 << R], const C* __restrict__ m, bool diag) {
-    constexpr int D = 1 << R, bit = 1 << P;
-    const C m00 = m[0], m01 = m[1], m10 = m[2], m11 = m[3];
-    if (diag) {
+// A matrix entry pair in one 16-byte load (complex64).
+__device__ __forceinline__ void ld_pair(const float2* m, float2& a, float2& b) {
+    const float4 t = *reinterpret_cast<const float4*>(m);
+    a = make_float2(t.x, t.y);
+    b = make_float2(t.z, t.w);
+}
+__device__ __forceinline__ void ld_pair(const double2* m, double2& a, double2& b) {
+    a = m[0];
+    b = m[1];
+}
+
+// Diagonal op: m holds the factor of every local index, so no position is needed.
+template <int R, typename C>
+__device__ __forceinline__ void reg_diag(C (&v)[1 << R], const C* __restrict__ m) {
 #pragma unroll
-        for (int c = 0; c < D; ++c) v[c] = cmul(v[c], (c & bit) ? m11 : m00);
-        return;
+    for (int c = 0; c < (1 << R); c += 2) {
+        C a, b;
+        ld_pair(m + c, a, b);
+        v[c] = cmul(v[c], a);
+        v[c + 1] = cmul(v[c + 1], b);
     }
+}
+
+template <int R, int P, typename C>
+__device__ __forceinline__ void reg_op1(C (&v)[1 << R], const C* __restrict__ m) {
+    constexpr int D = 1 << R, bit = 1 << P;
+    C m00, m01, m10, m11;
+    ld_pair(m, m00, m01);
+    ld_pair(m + 2, m10, m11);
 #pragma unroll
     for (int c = 0; c < D; ++c) {
         if (c & bit) continue;
@@ -105,17 +137,11 @@ __device__ __forceinline__ void reg_op1(C (&v)[1 << R], const C* __restrict__ m,
 
 // matrix index bit 1 (most significant) <-> local position P0 (the op's first site), bit 0 <-> P1
 template <int R, int P0, int P1, typename C>
-__device__ __forceinline__ void reg_op2(C (&v)[1 << R], const C* __restrict__ m, bool diag) {
+__device__ __forceinline__ void reg_op2(C (&v)[1 << R], const C* __restrict__ m) {
     constexpr int D = 1 << R, b0 = 1 << P0, b1 = 1 << P1;
-    if (diag) {
-        const C d0 = m[0], d1 = m[5], d2 = m[10], d3 = m[15];
-#pragma unroll
-        for (int c = 0; c < D; ++c) v[c] = cmul(v[c], (c & b0) ? ((c & b1) ? d3 : d2) : ((c & b1) ? d1 : d0));
-        return;
-    }
     C mm[16];
 #pragma unroll
-    for (int e = 0; e < 16; ++e) mm[e] = m[e];
+    for (int e = 0; e < 16; e += 2) ld_pair(m + e, mm[e], mm[e + 1]);
 #pragma unroll
     for (int c = 0; c < D; ++c) {
         if ((c & b0) || (c & b1)) continue;
@@ -134,70 +160,150 @@ __device__ __forceinline__ void reg_op2(C (&v)[1 << R], const C* __restrict__ m,
     }
 }
 
+// One-site op whose entries are real on the diagonal and imaginary off it (ROT: x
+// rotations), or all real: half the products. The products left out are by an exact zero.
+template <int R, int P, bool ROT, typename C>
+__device__ __forceinline__ void reg_op1_half(C (&v)[1 << R], const C* __restrict__ m) {
+    constexpr int D = 1 << R, bit = 1 << P;
+    C m00, m01, m10, m11;
+    ld_pair(m, m00, m01);
+    ld_pair(m + 2, m10, m11);
+#pragma unroll
+    for (int c = 0; c < D; ++c) {
+        if (c & bit) continue;
+        const C a = v[c], b = v[c | bit];
+        if (ROT) {
+            v[c].x = fma(-m01.y, b.y, m00.x * a.x);
+            v[c].y = fma(m01.y, b.x, m00.x * a.y);
+            v[c | bit].x = fma(m11.x, b.x, -(m10.y * a.y));
+            v[c | bit].y = fma(m11.x, b.y, m10.y * a.x);
+        } else {
+            v[c].x = fma(m01.x, b.x, m00.x * a.x);
+            v[c].y = fma(m01.x, b.y, m00.x * a.y);
+            v[c | bit].x = fma(m11.x, b.x, m10.x * a.x);
+            v[c | bit].y = fma(m11.x, b.y, m10.x * a.y);
+        }
+    }
+}
+
+// Both components times s; complex64 in one packed instruction (each rounded as alone).
+__device__ __forceinline__ void scale2(float2& v, float s) {
+    asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %2};\n\tmul.rn.f32x2 a, a, b;\n\tmov.b64 {%0, %1}, a;\n\t}"
+        : "+f"(v.x), "+f"(v.y)
+        : "f"(s));
+}
+__device__ __forceinline__ void scale2(double2& v, double s) {
+    v.x *= s;
+    v.y *= s;
+}
+
 // Amplitude damping of the site at local position P: w += weight of its |1>
-// components; then K0 (mode 1: |1> components times s0) or the jump (mode 2:
-// the |1> components times sj move to |0>, |1> cleared).
-template <int R, int P, typename C, typename T>
-__device__ __forceinline__ void reg_damp(C (&v)[1 << R], int mode, T s0, T sj, T& w) {
+// components; then K0 (|1> components times s0) or a replayed jump (the |1>
+// components times sj move to |0>, |1> cleared).
+template <int R, int P, bool JUMP, typename C, typename T>
+__device__ __forceinline__ void reg_damp(C (&v)[1 << R], T s, T& w) {
     constexpr int D = 1 << R, bit = 1 << P;
 #pragma unroll
     for (int c = 0; c < D; ++c) {
         if (!(c & bit)) continue;
         w = fma(v[c].x, v[c].x, w);
         w = fma(v[c].y, v[c].y, w);
-        if (mode == 1) {
-            v[c].x *= s0;
-            v[c].y *= s0;
-        } else {
-            v[c ^ bit].x = sj * v[c].x;
-            v[c ^ bit].y = sj * v[c].y;
+        if (JUMP) {
+            v[c ^ bit].x = s * v[c].x;
+            v[c ^ bit].y = s * v[c].y;
             v[c].x = T(0);
             v[c].y = T(0);
+        } else {
+            scale2(v[c], s);
         }
     }
 }
 
-template <int R, typename C>
-__device__ __forceinline__ void reg_apply1(C (&v)[1 << R], int P, const C* m, bool diag) {
-    switch (P) {
-        case 0: reg_op1<R, 0>(v, m, diag); break;
-        case 1: if constexpr (R > 1) reg_op1<R, 1>(v, m, diag); break;
-        case 2: if constexpr (R > 2) reg_op1<R, 2>(v, m, diag); break;
-        case 3: if constexpr (R > 3) reg_op1<R, 3>(v, m, diag); break;
+// Kinds of ops: one site general / real diagonal and imaginary off it / real; diagonal on one
+// or two sites (a factor per local index); two sites general.
+enum TrajKind : int { kOp1 = 0, kRot1 = 1, kReal1 = 2, kDiag1 = 3, kDiag2 = 4, kOp2 = 5 };
+
+// Where an op's channels leave the lanes' weights: complex64 in the next rows of shared memory
+// (TrajSweepSmem::rows), complex128 straight in the accumulators.
+constexpr int kTrajRows = 16, kTrajRow = 36;
+
+template <typename T> struct WeightSink;
+template <> struct WeightSink<float> {
+    float* at;  // the lane's element of the next row
+    __device__ __forceinline__ void put(float w) {
+        *at = w;
+        at += kTrajRow;
+    }
+};
+template <> struct WeightSink<double> {
+    double* at;  // the next channel's accumulator
+    __device__ __forceinline__ void put(double w) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+        if ((threadIdx.x & 31) == 0) wacc_add(*at, w);
+        ++at;
+    }
+};
+
+// An op and the K0 damping of its sites, straight-line.
+template <int R, int KIND, int P0, int P1, bool DAMP, typename C, typename T>
+__device__ __forceinline__ void reg_case(C (&v)[1 << R], const C* m, T s0, WeightSink<T>& sink) {
+    constexpr bool two = KIND == kDiag2 || KIND == kOp2;
+    if constexpr (P0 < R && (!two || (P1 < R && P0 != P1))) {
+        if constexpr (KIND == kOp1) reg_op1<R, P0>(v, m);
+        else if constexpr (KIND == kRot1) reg_op1_half<R, P0, true>(v, m);
+        else if constexpr (KIND == kReal1) reg_op1_half<R, P0, false>(v, m);
+        else if constexpr (KIND == kOp2) reg_op2<R, P0, P1>(v, m);
+        else reg_diag<R>(v, m);
+        if constexpr (DAMP) {
+            T w = T(0);  // the state's precision: the jump and renormalisation factors come from these
+            reg_damp<R, P0, false>(v, s0, w);
+            sink.put(w);
+            if constexpr (two) {
+                w = T(0);
+                reg_damp<R, P1, false>(v, s0, w);
+                sink.put(w);
+            }
+        }
     }
 }
 
-template <int R, int CODE, typename C>
-__device__ __forceinline__ void reg_apply2_case(C (&v)[1 << R], const C* m, bool diag) {
-    constexpr int P0 = CODE / 4, P1 = CODE % 4;
-    if constexpr (P0 < R && P1 < R && P0 != P1) reg_op2<R, P0, P1>(v, m, diag);
-}
-
-template <int R, typename C>
-__device__ __forceinline__ void reg_apply2(C (&v)[1 << R], int P0, int P1, const C* m, bool diag) {
-    switch (P0 * 4 + P1) {
-        case 1: reg_apply2_case<R, 1>(v, m, diag); break;
-        case 2: reg_apply2_case<R, 2>(v, m, diag); break;
-        case 3: reg_apply2_case<R, 3>(v, m, diag); break;
-        case 4: reg_apply2_case<R, 4>(v, m, diag); break;
-        case 6: reg_apply2_case<R, 6>(v, m, diag); break;
-        case 7: reg_apply2_case<R, 7>(v, m, diag); break;
-        case 8: reg_apply2_case<R, 8>(v, m, diag); break;
-        case 9: reg_apply2_case<R, 9>(v, m, diag); break;
-        case 11: reg_apply2_case<R, 11>(v, m, diag); break;
-        case 12: reg_apply2_case<R, 12>(v, m, diag); break;
-        case 13: reg_apply2_case<R, 13>(v, m, diag); break;
-        case 14: reg_apply2_case<R, 14>(v, m, diag); break;
+// One switch per op: with one for the op and one per damped site the group changed
+// registers at each join.
+template <int R, bool DAMP, typename C, typename T>
+__device__ __forceinline__ void reg_op(C (&v)[1 << R], int code, const C* m, T s0, WeightSink<T>& sink) {
+#define QGB_ONE(K, P) case K * 16 + P * 4: reg_case<R, K, P, 0, DAMP>(v, m, s0, sink); break;
+#define QGB_ONES(K) QGB_ONE(K, 0) QGB_ONE(K, 1) QGB_ONE(K, 2) QGB_ONE(K, 3)
+#define QGB_TWO(K, P, Q) case K * 16 + P * 4 + Q: reg_case<R, K, P, Q, DAMP>(v, m, s0, sink); break;
+#define QGB_TWOS(K)                                                                                              \
+    QGB_TWO(K, 0, 1) QGB_TWO(K, 0, 2) QGB_TWO(K, 0, 3) QGB_TWO(K, 1, 0) QGB_TWO(K, 1, 2) QGB_TWO(K, 1, 3)       \
+    QGB_TWO(K, 2, 0) QGB_TWO(K, 2, 1) QGB_TWO(K, 2, 3) QGB_TWO(K, 3, 0) QGB_TWO(K, 3, 1) QGB_TWO(K, 3, 2)
+    switch (code) {
+        QGB_ONES(kOp1)
+        QGB_ONES(kRot1)
+        QGB_ONES(kReal1)
+        QGB_ONES(kDiag1)
+        QGB_TWOS(kDiag2)
+        QGB_TWOS(kOp2)
     }
+#undef QGB_ONE
+#undef QGB_ONES
+#undef QGB_TWO
+#undef QGB_TWOS
 }
 
+// Damping of one site, with or without a jump (only ops where a jump is replayed come here).
 template <int R, typename C, typename T>
-__device__ __forceinline__ void reg_damp_at(C (&v)[1 << R], int P, int mode, T s0, T sj, T& w) {
-    switch (P) {
-        case 0: reg_damp<R, 0>(v, mode, s0, sj, w); break;
-        case 1: if constexpr (R > 1) reg_damp<R, 1>(v, mode, s0, sj, w); break;
-        case 2: if constexpr (R > 2) reg_damp<R, 2>(v, mode, s0, sj, w); break;
-        case 3: if constexpr (R > 3) reg_damp<R, 3>(v, mode, s0, sj, w); break;
+__device__ __forceinline__ void reg_damp_at(C (&v)[1 << R], int P, bool jump, T s0, T sj, T& w) {
+    switch (P + (jump ? 4 : 0)) {
+        case 0: reg_damp<R, 0, false>(v, s0, w); break;
+        case 1: if constexpr (R > 1) reg_damp<R, 1, false>(v, s0, w); break;
+        case 2: if constexpr (R > 2) reg_damp<R, 2, false>(v, s0, w); break;
+        case 3: if constexpr (R > 3) reg_damp<R, 3, false>(v, s0, w); break;
+        case 4: reg_damp<R, 0, true>(v, sj, w); break;
+        case 5: if constexpr (R > 1) reg_damp<R, 1, true>(v, sj, w); break;
+        case 6: if constexpr (R > 2) reg_damp<R, 2, true>(v, sj, w); break;
+        case 7: if constexpr (R > 3) reg_damp<R, 3, true>(v, sj, w); break;
     }
 }
 
@@ -207,123 +313,142 @@ __device__ __forceinline__ void reg_damp_at(C (&v)[1 << R], int P, int mode, T s
 // Per-sweep, per-trajectory state in dynamic shared memory.
 template <typename T> struct TrajSweepSmem {
     cplx<T>* msh;     // [op][16]: the op's matrix with its sampled Paulis folded in (first op: times the prescale)
-    typename WAccOf<T>::type* chw_w;  // [warp][2 * kTrajMaxOps]: per-warp weights of |1> before each damping
+    typename WAccOf<T>::type* chw_w;  // [warp][2 * kTrajMaxOps]: per-warp weights of |1> before each damping, by channel
+    T* rows;          // [warp][kTrajRows][kTrajRow]: the lanes' weights of the last channels (complex64)
     T* djump;         // [op][2]: jump factor sqrt(gamma) / sqrt(gamma W) where a jump is replayed
-    uint8_t* dmode;   // [op][2]: 0 none, 1 K0, 2 jump
-    uint8_t* dflag;   // [op]: the folded matrix is diagonal
+    uint32_t* desc;   // [op]: kind, local positions, width, replayed jumps and first channel (TrajDesc)
+    uint4* runs;      // [op][2]: at a run's first op, the swizzled byte offset of every local position; the bits
+                      // below the run's ascending positions (16 bits each) and the run's length
 };
 
-// Every run of a sweep on one staged tile; G groups of 2^R amplitudes per
-// thread at a time, a barrier after each run.
-template <typename T, int R, int G>
-__device__ __forceinline__ void traj_tile_runs(cplx<T>* __restrict__ tile, int m, const TrajOpDesc* __restrict__ ops,
-                                               int nops, const TrajSweepSmem<T>& sm, bool damp, T s0, int tid,
-                                               int nthr) {
+// Op descriptor bits: the local positions of its sites and its kind (the case of reg_op), ...
+enum TrajDesc : uint32_t { kDescP0 = 2, kDescP1 = 0, kDescKind = 4, kDescCode = 127, kDescTwo = 1u << 7,
+                           kDescJump0 = 1u << 8, kDescJumps = 3u << 8, kDescChan = 10 };
+
+// A channel's weights of the 32 lanes wait in a row of shared memory; when kTrajRows channels have
+// one, lane j sums row j in the order of a shuffle butterfly and adds the sum to the channel's
+// accumulator: 31 additions and 8 loads for 16 channels, where a butterfly per channel took 5
+// shuffles, 5 additions and an update by a single lane each. The row pitch keeps the 16-byte loads
+// of different rows on different banks.
+__device__ __forceinline__ void traj_flush(const float* __restrict__ rows, int count, WAccF* __restrict__ acc, int lane) {
+    __syncwarp();
+    if (lane < count) {
+        float x[32];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float4 q = *reinterpret_cast<const float4*>(rows + lane * kTrajRow + 4 * j);
+            x[4 * j] = q.x;
+            x[4 * j + 1] = q.y;
+            x[4 * j + 2] = q.z;
+            x[4 * j + 3] = q.w;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int l = 0; l < o; ++l) x[l] = __fadd_rn(x[l], x[l + o]);
+        wacc_add(acc[lane], x[0]);
+    }
+    __syncwarp();
+}
+
+// Every run of a sweep on one staged tile, a group of 2^R amplitudes per thread
+// at a time, a barrier after each run.
+template <typename T, int R, bool DAMP>
+__device__ __forceinline__ void traj_tile_runs(cplx<T>* __restrict__ tile, int m, int nops,
+                                               const TrajSweepSmem<T>& sm, T s0, int tid, int nthr) {
     using C = cplx<T>;
     constexpr int D = 1 << R;
     const int warp = tid >> 5, lane = tid & 31;
     auto* myw = sm.chw_w + size_t(warp) * (2 * kTrajMaxOps);
+    T* rows = sm.rows + warp * (kTrajRows * kTrajRow);
     for (int i0 = 0; i0 < nops;) {
-        const int nr = ops[i0].run;
-        int rp[R], srt[R];
-#pragma unroll
-        for (int j = 0; j < R; ++j) rp[j] = srt[j] = ops[i0].run_pos[j];
-#pragma unroll
-        for (int x = 1; x < R; ++x)
-#pragma unroll
-            for (int y = x; y > 0; --y)
-                if (srt[y - 1] > srt[y]) {
-                    const int t = srt[y];
-                    srt[y] = srt[y - 1];
-                    srt[y - 1] = t;
-                }
-        uint32_t soff[D];
-#pragma unroll
-        for (int l = 0; l < D; ++l) {
-            uint32_t o = 0;
-#pragma unroll
-            for (int j = 0; j < R; ++j) o |= uint32_t((l >> j) & 1) << rp[j];
-            soff[l] = tswz<T>(o);
-        }
+        const uint4 r0 = sm.runs[2 * i0], r1 = sm.runs[2 * i0 + 1];
+        const uint32_t bit[4] = {r0.x, r0.y, r0.z, r0.w};
+        const uint32_t below[4] = {r1.x & 0xffffu, r1.x >> 16, r1.y & 0xffffu, r1.y >> 16};
+        const int nr = int(r1.z);
         const uint32_t groups = 1u << (m - R);
-        for (uint32_t gb = 0; gb < groups; gb += uint32_t(G * nthr)) {
-            C v[G][D];
-            uint32_t sb[G];
-            bool ok[G];
+        for (uint32_t gb = 0; gb < groups; gb += uint32_t(nthr)) {
+            C v[D];
+            const uint32_t g = gb + uint32_t(tid);
+            const bool ok = g < groups;
+            uint32_t base = ok ? g : 0u;
 #pragma unroll
-            for (int gi = 0; gi < G; ++gi) {
-                const uint32_t g = gb + uint32_t(gi * nthr + tid);
-                ok[gi] = g < groups;
-                uint32_t base = ok[gi] ? g : 0u;
+            for (int j = 0; j < R; ++j) base += base & ~below[j];  // a zero bit at the position
+            uint32_t at[D];  // byte offsets of the group; the swizzle is linear over XOR
+            at[0] = tswz<T>(base) * uint32_t(sizeof(C));
 #pragma unroll
-                for (int j = 0; j < R; ++j)
-                    base = ((base >> srt[j]) << (srt[j] + 1)) | (base & ((1u << srt[j]) - 1));
-                sb[gi] = tswz<T>(base);
+            for (int j = 0; j < R; ++j)
 #pragma unroll
-                for (int l = 0; l < D; ++l) v[gi][l] = ok[gi] ? tile[sb[gi] ^ soff[l]] : mk<T>(T(0), T(0));
-            }
-            for (int q = 0; q < nr; ++q) {
-                const int i = i0 + q;
-                const int k = ops[i].k, p0 = ops[i].lpos[0], p1 = ops[i].lpos[1];
-                const C* mm = sm.msh + size_t(i) * 16;
-                const bool dg = sm.dflag[i] != 0;
-                T w0 = T(0), w1 = T(0);  // the state's precision: the jump and renormalisation factors come from these
+                for (int l = 0; l < (1 << j); ++l) at[l + (1 << j)] = at[l] ^ bit[j];
 #pragma unroll
-                for (int gi = 0; gi < G; ++gi) {
-                    if (k == 1) reg_apply1<R>(v[gi], p0, mm, dg);
-                    else reg_apply2<R>(v[gi], p0, p1, mm, dg);
-                }
-                if (damp) {
-                    const int d0 = sm.dmode[2 * i], d1 = sm.dmode[2 * i + 1];
-                    const T j0 = sm.djump[2 * i], j1 = sm.djump[2 * i + 1];
-#pragma unroll
-                    for (int gi = 0; gi < G; ++gi) {
-                        reg_damp_at<R>(v[gi], p0, d0, s0, j0, w0);
-                        if (k == 2) reg_damp_at<R>(v[gi], p1, d1, s0, j1, w1);
-                    }
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) {
-                        w0 += __shfl_xor_sync(0xffffffffu, w0, o);
-                        w1 += __shfl_xor_sync(0xffffffffu, w1, o);
-                    }
-                    if (lane == 0) {
-                        wacc_add(myw[2 * i], w0);
-                        wacc_add(myw[2 * i + 1], w1);
+            for (int l = 0; l < D; ++l)
+                v[l] = ok ? *reinterpret_cast<const C*>(reinterpret_cast<const char*>(tile) + at[l]) : mk<T>(T(0), T(0));
+            auto* acc = myw + (sm.desc[i0] >> kDescChan);  // of the next channel without a sum
+            WeightSink<T> sink;
+            if constexpr (sizeof(T) == 4) sink.at = rows + lane;
+            else sink.at = acc;
+            const C* mm = sm.msh + size_t(i0) * 16;
+            const uint32_t* dp = sm.desc + i0;
+            uint32_t next = *dp;
+            for (int left = nr; left > 0; --left, mm += 16) {
+                const uint32_t d = next;
+                next = *++dp;  // one past the last op is the table after it
+                if (!DAMP || !(d & kDescJumps)) {
+                    reg_op<R, DAMP>(v, int(d & kDescCode), mm, s0, sink);
+                } else {
+                    const T* dj = sm.djump + 2 * (dp - 1 - sm.desc);
+                    reg_op<R, false>(v, int(d & kDescCode), mm, s0, sink);
+                    T w = T(0);
+                    reg_damp_at<R>(v, (d >> kDescP0) & 3, (d & kDescJump0) != 0, s0, dj[0], w);
+                    sink.put(w);
+                    if (d & kDescTwo) {
+                        w = T(0);
+                        reg_damp_at<R>(v, (d >> kDescP1) & 3, (d & (kDescJump0 << 1)) != 0, s0, dj[1], w);
+                        sink.put(w);
                     }
                 }
+                if constexpr (DAMP && sizeof(T) == 4) {
+                    if (left == 1 || sink.at > rows + lane + (kTrajRows - 2) * kTrajRow) {
+                        const int count = int(sink.at - (rows + lane)) / kTrajRow;
+                        traj_flush(rows, count, acc, lane);
+                        acc += count;
+                        sink.at = rows + lane;
+                    }
+                }
             }
+            if (ok)
 #pragma unroll
-            for (int gi = 0; gi < G; ++gi)
-                if (ok[gi])
-#pragma unroll
-                    for (int l = 0; l < D; ++l) tile[sb[gi] ^ soff[l]] = v[gi][l];
+                for (int l = 0; l < D; ++l) *reinterpret_cast<C*>(reinterpret_cast<char*>(tile) + at[l]) = v[l];
         }
         __syncthreads();
         i0 += nr;
     }
 }
 
-template <typename T, int RMAX>
-__device__ __forceinline__ void traj_tile_dispatch(cplx<T>* tile, int m, const TrajOpDesc* ops, int nops,
-                                                   const TrajSweepSmem<T>& sm, bool damp, T s0, int tid, int nthr) {
+template <typename T, int RMAX, bool DAMP>
+__device__ __forceinline__ void traj_tile_dispatch(cplx<T>* tile, int m, int nops, const TrajSweepSmem<T>& sm, T s0,
+                                                   int tid, int nthr) {
     const int R = m < RMAX ? m : RMAX;
     switch (R) {
-        case 1: traj_tile_runs<T, 1, 1>(tile, m, ops, nops, sm, damp, s0, tid, nthr); break;
-        case 2: traj_tile_runs<T, 2, 1>(tile, m, ops, nops, sm, damp, s0, tid, nthr); break;
-        case 3: traj_tile_runs<T, 3, 1>(tile, m, ops, nops, sm, damp, s0, tid, nthr); break;
-        default: if constexpr (RMAX >= 4) traj_tile_runs<T, 4, 1>(tile, m, ops, nops, sm, damp, s0, tid, nthr); break;
+        case 1: traj_tile_runs<T, 1, DAMP>(tile, m, nops, sm, s0, tid, nthr); break;
+        case 2: traj_tile_runs<T, 2, DAMP>(tile, m, nops, sm, s0, tid, nthr); break;
+        case 3: traj_tile_runs<T, 3, DAMP>(tile, m, nops, sm, s0, tid, nthr); break;
+        default: if constexpr (RMAX >= 4) traj_tile_runs<T, 4, DAMP>(tile, m, nops, sm, s0, tid, nthr); break;
     }
 }
 
 template <typename T> constexpr int traj_rmax() { return sizeof(T) == 4 ? 4 : 3; }
 
-// dynamic shared memory: tile buffers | high-bit offsets | folded matrices | per-warp weights | jump factors |
-// damping modes | diagonal flags
+template <typename T> constexpr size_t traj_row_elems() {
+    return sizeof(T) == 4 ? size_t(kTrajThreads / 32) * kTrajRows * kTrajRow : 0;
+}
+
+// dynamic shared memory: tile buffers | high-bit offsets | folded matrices | per-warp weights | lanes' weights |
+// jump factors | op descriptors | run positions
 template <typename T> __host__ __device__ constexpr size_t traj_aux_bytes() {
     return sizeof(uint32_t) * (size_t(1) << QGB_SWEEP_MAX_HIGH) + sizeof(cplx<T>) * kTrajMaxOps * 16 +
-           sizeof(typename WAccOf<T>::type) * (kTrajThreads / 32) * 2 * kTrajMaxOps + sizeof(T) * 2 * kTrajMaxOps +
-           2 * kTrajMaxOps +
-           kTrajMaxOps;
+           sizeof(typename WAccOf<T>::type) * (kTrajThreads / 32) * 2 * kTrajMaxOps + sizeof(T) * traj_row_elems<T>() +
+           sizeof(T) * 2 * kTrajMaxOps + (sizeof(uint32_t) + 2 * sizeof(uint4)) * kTrajMaxOps;
 }
 
 template <typename T>
@@ -341,9 +466,10 @@ __global__ void __launch_bounds__(kTrajThreads) traj_run_kernel(cplx<T>* __restr
     TrajSweepSmem<T> sm;
     sm.msh = reinterpret_cast<C*>(hoff + (size_t(1) << QGB_SWEEP_MAX_HIGH));
     sm.chw_w = reinterpret_cast<typename WAccOf<T>::type*>(sm.msh + kTrajMaxOps * 16);
-    sm.djump = reinterpret_cast<T*>(sm.chw_w + (kTrajThreads / 32) * 2 * kTrajMaxOps);
-    sm.dmode = reinterpret_cast<uint8_t*>(sm.djump + 2 * kTrajMaxOps);
-    sm.dflag = sm.dmode + 2 * kTrajMaxOps;
+    sm.rows = reinterpret_cast<T*>(sm.chw_w + (kTrajThreads / 32) * 2 * kTrajMaxOps);
+    sm.djump = sm.rows + traj_row_elems<T>();
+    sm.desc = reinterpret_cast<uint32_t*>(sm.djump + 2 * kTrajMaxOps);
+    sm.runs = reinterpret_cast<uint4*>(sm.desc + kTrajMaxOps);
     __shared__ double chw[2 * kTrajMaxOps];  // per (op, site): weight of |1> before damping, summed over the tiles
     __shared__ uint8_t pk[kTrajMaxOps][2];   // sampled Paulis
     __shared__ int jop[kTrajMaxJumps], jsite[kTrajMaxJumps];
@@ -381,14 +507,8 @@ __global__ void __launch_bounds__(kTrajThreads) traj_run_kernel(cplx<T>* __restr
                 for (int j = 0; j < H; ++j) o |= ((h >> j) & 1u) << sw.high_bits[j];
                 hoff[h] = o;
             }
-            uint32_t outer_bits[32];
-            int n_outer = 0;
-            {
-                uint32_t in_tile = lmask;
-                for (int j = 0; j < H; ++j) in_tile |= 1u << sw.high_bits[j];
-                for (int b = 0; b < a.n; ++b)
-                    if (!((in_tile >> b) & 1u)) outer_bits[n_outer++] = b;
-            }
+            uint32_t in_tile = lmask;
+            for (int j = 0; j < H; ++j) in_tile |= 1u << sw.high_bits[j];
             // the Paulis of the sweep's channels (state independent, the gate-by-gate kernel's counters)
             for (int c = tid; c < 2 * nops; c += nthr) {
                 const int i = c >> 1, j = c & 1;
@@ -434,20 +554,53 @@ __global__ void __launch_bounds__(kTrajThreads) traj_run_kernel(cplx<T>* __restr
                         }
                     }
                 }
-                for (int e = 0; e < D * D; ++e) sm.msh[size_t(i) * 16 + e] = M[e];
-                sm.dflag[i] = diag ? 1 : 0;
+                C* out = sm.msh + size_t(i) * 16;
+                if (diag) {  // the factor of every local index of the run's group
+                    const int r = m < traj_rmax<T>() ? m : traj_rmax<T>();
+                    for (int c = 0; c < (1 << r); ++c) {
+                        int e = (c >> op.lpos[0]) & 1;
+                        if (op.k == 2) e = 2 * e + ((c >> op.lpos[1]) & 1);
+                        out[c] = M[e * (D + 1)];
+                    }
+                } else {
+                    for (int e = 0; e < D * D; ++e) out[e] = M[e];
+                }
+                uint32_t chan = 0;
+                for (int x = 0; x < i; ++x) chan += uint32_t(sops[x].k);
+                int kind = op.k == 1 ? (diag ? kDiag1 : kOp1) : (diag ? kDiag2 : kOp2);
+                if (kind == kOp1) {
+                    if (M[0].y == T(0) && M[3].y == T(0) && M[1].x == T(0) && M[2].x == T(0)) kind = kRot1;
+                    else if (M[0].y == T(0) && M[3].y == T(0) && M[1].y == T(0) && M[2].y == T(0)) kind = kReal1;
+                }
+                sm.desc[i] = uint32_t(kind) << kDescKind | uint32_t(op.lpos[0]) << kDescP0 |
+                             (op.k == 2 ? uint32_t(op.lpos[1]) << kDescP1 | kDescTwo : 0u) | chan << kDescChan;
+                if (op.run > 0) {
+                    const int r = m < traj_rmax<T>() ? m : traj_rmax<T>();
+                    uint32_t b[4] = {0, 0, 0, 0}, low[4] = {0, 0, 0, 0};
+                    for (int x = 0; x < r; ++x) {
+                        int rank = 0;
+                        for (int y = 0; y < r; ++y) rank += op.run_pos[y] < op.run_pos[x];
+                        b[x] = tswz<T>(1u << op.run_pos[x]) * uint32_t(sizeof(C));
+                        low[rank] = (1u << op.run_pos[x]) - 1u;
+                    }
+                    sm.runs[2 * i] = make_uint4(b[0], b[1], b[2], b[3]);
+                    sm.runs[2 * i + 1] = make_uint4(low[0] | low[1] << 16, low[2] | low[3] << 16, uint32_t(op.run), 0u);
+                }
             }
             const uint64_t tiles = uint64_t(1) << (a.n - m);
-            auto base_of = [&](uint64_t w) -> uint32_t {
-                uint32_t b = 0;
-                for (int j = 0; j < n_outer; ++j) b |= uint32_t((w >> j) & 1ull) << outer_bits[j];
-                return b;
-            };
-            auto load = [&](uint64_t w, C* buf) {
-                const uint32_t base = base_of(w);
+            // bases of successive tiles: a count over the bits outside the tile
+            auto after = [&](uint32_t base) -> uint32_t { return ((base | in_tile) + 1u) & ~in_tile; };
+            // Offsets of the thread's 16-byte pieces: offset and swizzle are linear over disjoint bits, so a
+            // piece's are the thread's, once a sweep, and the step's, the same for all threads.
+            const uint32_t step = per16 * nthr, e_t = per16 * tid;
+            uint32_t off_t = e_t & lmask;
+            for (int j = 0; j < H; ++j) off_t |= (((e_t & ((1u << m) - 1u)) >> (L + j)) & 1u) << sw.high_bits[j];
+            const uint32_t sw_t = tswz<T>(e_t);
+            auto load = [&](uint32_t base, C* buf) {
                 if (src) {
-                    for (uint32_t e = per16 * tid; e < (1u << m); e += per16 * nthr)
-                        traj_cp16(buf + tswz<T>(e), src + (base + hoff[e >> L] + (e & lmask)));
+#pragma unroll 4
+                    for (uint32_t e = 0; e + e_t < (1u << m); e += step)
+                        traj_cp16(buf + (sw_t ^ tswz<T>(e)), src + (base + off_t + hoff[e >> L] + (e & lmask)));
                 } else {
                     for (uint32_t e = tid; e < (1u << m); e += nthr) {
                         const uint32_t gi = base + hoff[e >> L] + (e & lmask);
@@ -458,41 +611,45 @@ __global__ void __launch_bounds__(kTrajThreads) traj_run_kernel(cplx<T>* __restr
             };
             for (int pass = 0; pass <= kTrajMaxJumps; ++pass) {
                 // damping of every (op, site): K0, or the replayed jumps of this sweep
-                for (int c = tid; c < 2 * nops; c += nthr) {
-                    sm.dmode[c] = damp ? 1 : 0;
-                    sm.djump[c] = T(0);
-                }
+                for (int c = tid; c < 2 * nops; c += nthr) sm.djump[c] = T(0);
                 for (int c = tid; c < nwarps * 2 * nops; c += nthr)
                     wacc_zero(sm.chw_w[size_t(c / (2 * nops)) * (2 * kTrajMaxOps) + (c % (2 * nops))]);
                 __syncthreads();
                 if (tid == 0)
                     for (int q = 0; q < s_njump; ++q) {
-                        sm.dmode[2 * jop[q] + jsite[q]] = 2;
+                        sm.desc[jop[q]] |= kDescJump0 << jsite[q];
                         sm.djump[2 * jop[q] + jsite[q]] = T(sqrt(a.gamma) * jscale[q]);
                     }
                 __syncthreads();
+                uint32_t base = 0, base_next = after(0);
                 load(0, bufs);
                 for (uint64_t w = 0; w < tiles; ++w) {
                     C* cur = bufs + (size_t(a.nbuf == 2 ? (w & 1) : 0) << m);
                     if (a.nbuf == 2 && w + 1 < tiles) {
-                        load(w + 1, bufs + (size_t((w + 1) & 1) << m));
+                        load(base_next, bufs + (size_t((w + 1) & 1) << m));
                         asm volatile("cp.async.wait_group 1;" ::: "memory");
                     } else {
                         asm volatile("cp.async.wait_group 0;" ::: "memory");
                     }
                     __syncthreads();
-                    traj_tile_dispatch<T, traj_rmax<T>()>(cur, m, sops, nops, sm, damp, s0, tid, nthr);
-                    const uint32_t base = base_of(w);
-                    for (uint32_t e = per16 * tid; e < (1u << m); e += per16 * nthr)
-                        *reinterpret_cast<float4*>(dst + (base + hoff[e >> L] + (e & lmask))) =
-                            *reinterpret_cast<const float4*>(cur + tswz<T>(e));
+                    if (damp) traj_tile_dispatch<T, traj_rmax<T>(), true>(cur, m, nops, sm, s0, tid, nthr);
+                    else traj_tile_dispatch<T, traj_rmax<T>(), false>(cur, m, nops, sm, s0, tid, nthr);
+#pragma unroll 4
+                    for (uint32_t e = 0; e + e_t < (1u << m); e += step)
+                        *reinterpret_cast<float4*>(dst + (base + off_t + hoff[e >> L] + (e & lmask))) =
+                            *reinterpret_cast<const float4*>(cur + (sw_t ^ tswz<T>(e)));
                     __syncthreads();  // the buffer is free for the copy issued two tiles later
-                    if (a.nbuf == 1 && w + 1 < tiles) load(w + 1, bufs);
+                    if (a.nbuf == 1 && w + 1 < tiles) load(base_next, bufs);
+                    base = base_next;
+                    base_next = after(base);
                 }
                 // the weights, summed over the warps in a fixed order
                 for (int c = tid; c < 2 * nops; c += nthr) {
+                    const uint32_t d = sm.desc[c >> 1];
+                    if ((c & 1) && !(d & kDescTwo)) continue;
+                    const size_t ch = (d >> kDescChan) + (c & 1);
                     double x = 0.0;
-                    for (int wp = 0; wp < nwarps; ++wp) x += wacc_value(sm.chw_w[size_t(wp) * (2 * kTrajMaxOps) + c]);
+                    for (int wp = 0; wp < nwarps; ++wp) x += wacc_value(sm.chw_w[size_t(wp) * (2 * kTrajMaxOps) + ch]);
                     chw[c] = x;
                 }
                 __syncthreads();
@@ -551,9 +708,15 @@ __global__ void __launch_bounds__(kTrajThreads) traj_run_kernel(cplx<T>* __restr
         {
             const T sc = T(s_prescale);
             if (src) {
-                for (uint64_t e = tid; e < dim; e += nthr) {
-                    const C v = src[e];
-                    own[e] = mk<T>(v.x * sc, v.y * sc);
+                {
+#pragma unroll 4
+                    for (uint64_t e = uint64_t(per16) * tid; e < dim; e += per16 * nthr) {
+                        float4 q = *reinterpret_cast<const float4*>(src + e);
+                        T* x = reinterpret_cast<T*>(&q);
+#pragma unroll
+                        for (int j = 0; j < int(2 * per16); ++j) x[j] *= sc;
+                        *reinterpret_cast<float4*>(own + e) = q;
+                    }
                 }
             } else {
                 for (uint64_t e = tid; e < dim; e += nthr) own[e] = mk<T>(e == 0 ? T(1) : T(0), T(0));
@@ -582,13 +745,13 @@ int traj_grid(int mmax, int hmax, int64_t ntraj, int* nbuf_out, size_t* smem_out
     auto kern = traj_run_kernel<T>;
     static bool attr = false;
     if (!attr) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrajMaxSmem) != cudaSuccess)
             return check_launch("trajectory kernel attribute");
         attr = true;
     }
     for (int nbuf = 2; nbuf >= 1; --nbuf) {
         const size_t smem = traj_smem_bytes<T>(mmax, hmax, nbuf);
-        if (smem > 200 * 1024) continue;
+        if (smem > kTrajMaxSmem) continue;
         int per_sm = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTrajThreads, smem) != cudaSuccess)
             return check_launch("trajectory kernel occupancy");

@@ -13,7 +13,8 @@
 //    copied with cp.async two ahead, split-fp16 operands staged into tensor
 //    memory, one MMA warp, the drain straight to HBM);
 //  * items are ordered pass by pass across circuits (round r holds the r-th
-//    pass of every circuit that has one), and an item waits until every item
+//    pass of every circuit that has one, dealt so that it is one wave of items),
+//    and an item waits until every item
 //    of its circuit's previous pass is done (a per-circuit counter, read with
 //    a bounded spin). Every item's dependencies have smaller tickets and were
 //    taken by running CTAs, so the smallest unfinished ticket can always
@@ -30,11 +31,18 @@
 //    Tr(rho^2) from the slots. Every sum runs in a fixed order (per thread,
 //    then a fixed shuffle tree, then warp by warp), so results are bitwise
 //    reproducible whichever CTA takes which item.
+// What bounds it: the data warps (two a scheduler) between the copies: reading and splitting a
+// tile, issuing its copies and draining it took 8200 cycles where the memory takes 5900. Offsets
+// in 32 bits by one masked addition a tile instead of 13 bit insertions in 64, and the rows a lane
+// stores shuffled once a tile instead of as pointers 16 times: 10.9 to 9.5 ms (16 noisy circuits of
+// 7 to 12 qubits, depth 10 to 20, with the small ones); items of one wave a round 11.3 to 10.9;
+// small circuits beside it on a stream of their own 9.5 to 8.6.
 // Every wait is bounded (about 2 s); a wait that runs out sets a status word
 // (qgb_check_status -> QGB_ETIMEOUT) and the CTA stops taking work.
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 #include <vector>
 
 #include "tc_common.cuh"
@@ -231,7 +239,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) dm_batch_tc_kernel(const __grid
             __syncthreads();
         }
         const uint64_t ntiles = it.ntiles;
-        const uint64_t tstr = it.tstride;
 
         if (warp == 8) {
             // ---- MMA warp
@@ -265,25 +272,25 @@ __global__ void __launch_bounds__(kTcThreads, 1) dm_batch_tc_kernel(const __grid
             const uint32_t row = tmem + (uint32_t(32 * q) << 16);
             const uint32_t runmask = (1u << sA.L) - 1u;
             const int n = C.n;
-            const uint64_t dmask = (uint64_t(1) << n) - 1;
+            const uint32_t dmask = (1u << n) - 1;  // vec(rho) has at most 28 bits: flat offsets fit 32 bits
             uint32_t sug;
-            uint64_t gg;
+            uint32_t gg;
             {
                 const uint32_t r = uint32_t(32 * q + lane);
                 uint32_t u = 0;
 #pragma unroll
                 for (int i = 0; i < 13 - K; ++i) u |= ((r >> i) & 1u) << sA.pos_g[i];
                 sug = tile_swz(u | (h ? sA.ut_h : 0u));
-                gg = uint64_t(u & runmask) + sA.hoff[u >> sA.L] + (h ? sA.hstride : 0);
+                gg = uint32_t((u & runmask) + sA.hoff[u >> sA.L] + (h ? sA.hstride : 0));
             }
             const uint32_t ctid = 2u * uint32_t(tid);
             const uint32_t sctid = tile_swz(ctid);
-            const uint64_t gctid = uint64_t(ctid & runmask) + sA.hoff[ctid >> sA.L];
+            const uint32_t gctid = uint32_t((ctid & runmask) + sA.hoff[ctid >> sA.L]);
             const bool first = (flags & kDmbFirst) != 0;
             // component offsets from their single-bit basis, in registers (both maps are
             // linear: swizzled tile offsets over XOR, flat offsets over OR), instead of a
             // shared-memory table read per component
-            uint32_t ub[K - 1], ob[K - 1];  // vec(rho) has at most 28 bits: flat offsets fit 32 bits
+            uint32_t ub[K - 1], ob[K - 1];
 #pragma unroll
             for (int i = 0; i < K - 1; ++i) {
                 ub[i] = sA.uts[1 << i];
@@ -303,8 +310,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) dm_batch_tc_kernel(const __grid
                     if ((j >> i) & 1) o |= ob[i];
                 return o;
             };
-            auto tile_off = [&](uint64_t t) -> uint64_t { return insert_zeros(t, sA.tile_bits, 13); };
-            auto issue_load = [&](uint64_t t, int pb) {
+            // offsets of the item's tiles: t0's, then one masked addition a tile (the tile's bits set, so
+            // that a carry passes them), where 13 bit insertions a tile took a tenth of the tile's time
+            uint32_t in_tile = 0;
+#pragma unroll
+            for (int i = 0; i < 13; ++i) in_tile |= 1u << sA.tile_bits[i];
+            const uint32_t off_stride = uint32_t(insert_zeros(it.tstride, sA.tile_bits, 13));
+            auto after = [&](uint32_t off) -> uint32_t { return ((off | in_tile) + off_stride) & ~in_tile; };
+            auto issue_load = [&](uint32_t off, int pb) {
                 const uint32_t dst0 = tc_smem_u32(tiles_smem + pb * G::TILE_BYTES);
                 if (first) {
                     // |0...0><0...0|: zeros, and 1 at flat index 0 (tile 0, tile index 0)
@@ -312,13 +325,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) dm_batch_tc_kernel(const __grid
 #pragma unroll
                     for (int m = 0; m < 4096 / kTcDataThreads; ++m)
                         d4[(sctid ^ tile_swz(512u * uint32_t(m))) >> 1] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (t == 0 && tid == 0) d4[0] = make_float4(1.f, 0.f, 0.f, 0.f);
+                    if (off == 0 && tid == 0) d4[0] = make_float4(1.f, 0.f, 0.f, 0.f);
                     return;
                 }
-                const float2* base = C.state + tile_off(t) + gctid;
+                const float2* base = C.state + (off + gctid);
 #pragma unroll
                 for (int m = 0; m < 4096 / kTcDataThreads; ++m)
-                    cp_async16(dst0 + 8u * (sctid ^ tile_swz(512u * uint32_t(m))), base + sA.g512[m]);
+                    cp_async16(dst0 + 8u * (sctid ^ tile_swz(512u * uint32_t(m))), base + uint32_t(sA.g512[m]));
             };
             // stage this thread's half row of the tile in pair pb; returns 2^-s of the row
             auto store_x = [&](int pb) -> float {
@@ -360,7 +373,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) dm_batch_tc_kernel(const __grid
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 return exp2i(-se);
             };
-            auto put16 = [&](float2* p, int c0, const float* r) {
+            // rho4: this lane's rows of the staged stores (vec4), as offsets from the state
+            auto put16 = [&](float2* p, const uint32_t (&rho4)[4], int c0, const float* r) {
                 if (sA.vec4) {
                     float4* st4 = reinterpret_cast<float4*>(stage_smem + warp * 2048);
 #pragma unroll
@@ -374,9 +388,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) dm_batch_tc_kernel(const __grid
                     for (int i = 0; i < 4; ++i) {
                         const int rho = 8 * i + (lane >> 2);
                         const float4 x = st4[rho * 4 + (pc ^ ((rho >> 1) & 3))];
-                        float2* pr = reinterpret_cast<float2*>(
-                            __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(p), rho));
-                        *reinterpret_cast<float4*>(pr + (off_of(c0 / 2) | opc)) = x;
+                        *reinterpret_cast<float4*>(C.state + (rho4[i] | off_of(c0 / 2) | opc)) = x;
                     }
                     __syncwarp();
                 } else if (sA.vec2) {
@@ -392,16 +404,19 @@ __global__ void __launch_bounds__(kTcThreads, 1) dm_batch_tc_kernel(const __grid
             const bool tail = (flags & kDmbTail) != 0, last = (flags & kDmbLast) != 0;
             // diagonal entries (ket bits == bra bits): a row can hold one only if its fixed
             // (non-target) bits agree on every ket/bra pair that has no target bit
-            uint64_t tbits = sA.hstride;
+            uint32_t tbits = uint32_t(sA.hstride);
 #pragma unroll
             for (int i = 0; i < K - 1; ++i) tbits |= ob[i];
-            const uint64_t freepair = dmask & ~((tbits | (tbits >> n)) & dmask);
+            const uint32_t freepair = dmask & ~((tbits | (tbits >> n)) & dmask);
             float f_pur = 0.f;
             double acc_pur = 0.0, acc_tr = 0.0;  // this thread's sums, in tile order
-            // the result of tile t (pair pb) to HBM, with the trace / purity / Z sums this pass needs
-            auto drain = [&](uint64_t t, int pb, float us) {
-                const uint64_t ridx = tile_off(t) + gg;  // flat index of this thread's row
+            // the result of the tile at off (pair pb) to HBM, with the trace / purity / Z sums this pass needs
+            auto drain = [&](uint32_t off, int pb, float us) {
+                const uint32_t ridx = off + gg;  // flat index of this thread's row
                 float2* p = C.state + ridx;
+                uint32_t rho4[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) rho4[i] = __shfl_sync(0xffffffffu, ridx, 8 * i + (lane >> 2));
                 const uint32_t acc = row + uint32_t(2 * R + pb * R + h * D);
                 const float wun = wunscale_s;
                 const float su = us * wun;
@@ -423,11 +438,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) dm_batch_tc_kernel(const __grid
                     if (tail && ((((ridx >> n) ^ ridx) & freepair) == 0)) {
 #pragma unroll
                         for (int e = 0; e < 8; ++e) {
-                            const uint64_t idx = ridx + off_of(c0 / 2 + e);
+                            const uint32_t idx = ridx + off_of(c0 / 2 + e);
                             if ((((idx >> n) ^ idx) & dmask) == 0) acc_tr += double(r[2 * e]);
                         }
                     }
-                    put16(p, c0, r);
+                    put16(p, rho4, c0, r);
                 }
                 if (last) {
                     acc_pur += double(f_pur);
@@ -436,9 +451,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) dm_batch_tc_kernel(const __grid
             };
 
             // the dense_tc pipeline over this item's tiles (units ubase + k)
-            issue_load(it.t0, int(ubase & 1));
+            uint32_t off_out = uint32_t(insert_zeros(it.t0, sA.tile_bits, 13)), off_in = after(off_out);
+            issue_load(off_out, int(ubase & 1));
             cp_async_commit();
-            if (ntiles > 1) issue_load(it.t0 + tstr, int((ubase + 1) & 1));
+            if (ntiles > 1) issue_load(off_in, int((ubase + 1) & 1));
             cp_async_commit();
             bool fail = false;
             float usA = 1.f, usB = 1.f;
@@ -457,7 +473,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) dm_batch_tc_kernel(const __grid
                 __syncwarp();
                 if (lane == 0) mbar_arrive(tc_smem_u32(&x_full[pc]));
                 data_bar();  // every read of buffer pc is done
-                if (k + 2 < ntiles) issue_load(it.t0 + (k + 2) * tstr, pc);
+                off_in = after(off_in);
+                if (k + 2 < ntiles) issue_load(off_in, pc);
                 cp_async_commit();
                 if (k >= 1) {
                     if (!tc_wait_bounded(tc_smem_u32(&mma_done[pn]), uint32_t(((u - 1) >> 1) & 1))) {
@@ -465,7 +482,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) dm_batch_tc_kernel(const __grid
                         if (tid == 0) atomicExch(&g_dmb_status, 2);
                     } else {
                         tc_fence_after();
-                        drain(it.t0 + (k - 1) * tstr, pn, pn ? usB : usA);
+                        drain(off_out, pn, pn ? usB : usA);
+                        off_out = after(off_out);
                     }
                 }
             }
@@ -474,7 +492,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) dm_batch_tc_kernel(const __grid
                 const int pl = int(u & 1);
                 if (tc_wait_bounded(tc_smem_u32(&mma_done[pl]), uint32_t((u >> 1) & 1))) {
                     tc_fence_after();
-                    drain(it.t0 + (ntiles - 1) * tstr, pl, pl ? usB : usA);
+                    drain(off_out, pl, pl ? usB : usA);
                 } else {
                     fail = true;
                     if (tid == 0) atomicExch(&g_dmb_status, 2);
@@ -515,6 +533,7 @@ using namespace qgb;
 
 namespace {
 
+constexpr uint64_t kDmbMinTiles = 8;
 constexpr size_t kDmbSmem = 2 * size_t(TcGeom<6>::B_BYTES) + 2 * size_t(TcGeom<6>::TILE_BYTES) +
                             TcGeom<6>::STAGE_BYTES + 128;
 
@@ -552,16 +571,26 @@ int dmb_status_read_clear() {
 extern "C" size_t qgb_dm_batch_circuit_bytes(void) { return sizeof(qgb_dm_circuit); }
 extern "C" size_t qgb_dm_batch_pass_bytes(void) { return sizeof(qgb_dm_pass); }
 
-// Items of a circuit's pass: its tiles of 8192 entries dealt round-robin to
-// min(items_per_pass, tiles / 16) items (at least one): a pass of a large
-// circuit is one wave of items_per_pass (the SM count) items, and no item has
-// fewer than 16 tiles unless the whole pass has.
-constexpr int64_t kDmbMinTiles = 16;
-static int64_t items_of(int n, int items_per_pass) {
-    const int64_t tiles = int64_t(1) << (2 * n - 13);
-    const int64_t by_size = tiles / kDmbMinTiles > 0 ? tiles / kDmbMinTiles : 1;
-    return by_size < items_per_pass ? by_size : items_per_pass;
+// Items of a circuit's pass in round r: its tiles of 8192 entries dealt round-robin, so many a
+// item that the round (the r-th passes of all circuits that have one) is one wave of
+// items_per_pass (the SM count) items, at least kDmbMinTiles (an item builds its operand and
+// fills and drains the pipeline).
+static uint64_t tiles_of(int n) { return uint64_t(1) << (2 * n - 13); }
+
+static std::vector<uint64_t> item_tiles(const qgb_dm_circuit* circs, int ncirc, int items_per_pass) {
+    int rounds = 0;
+    for (int c = 0; c < ncirc; ++c) rounds = circs[c].n_passes > rounds ? circs[c].n_passes : rounds;
+    std::vector<uint64_t> q(size_t(rounds), 0);
+    for (int c = 0; c < ncirc; ++c)
+        for (int r = 0; r < circs[c].n_passes; ++r) q[size_t(r)] += tiles_of(circs[c].n);
+    for (uint64_t& x : q) {
+        x = (x + uint64_t(items_per_pass) - 1) / uint64_t(items_per_pass);
+        if (x < kDmbMinTiles) x = kDmbMinTiles;
+    }
+    return q;
 }
+
+static int64_t items_of(int n, uint64_t q) { return int64_t((tiles_of(n) + q - 1) / q); }
 
 static int check_tables(const qgb_dm_circuit* circs, int ncirc, const qgb_dm_pass* passes, int npasses,
                         int items_per_pass) {
@@ -604,12 +633,17 @@ static int check_tables(const qgb_dm_circuit* circs, int ncirc, const qgb_dm_pas
 
 extern "C" int64_t qgb_dm_batch_items(const qgb_dm_circuit* circs, int ncirc, int items_per_pass) {
     if (!circs || ncirc < 1 || items_per_pass < 1) return -1;
-    int64_t total = ncirc;  // a finishing item per circuit
-    for (int c = 0; c < ncirc; ++c) {
-        if (circs[c].n < 7 || circs[c].n > 14) return -1;
-        total += items_of(circs[c].n, items_per_pass) * circs[c].n_passes;
+    for (int c = 0; c < ncirc; ++c)
+        if (circs[c].n < 7 || circs[c].n > 14 || circs[c].n_passes < 0) return -1;
+    try {
+        const std::vector<uint64_t> q = item_tiles(circs, ncirc, items_per_pass);
+        int64_t total = ncirc;  // a finishing item per circuit
+        for (int c = 0; c < ncirc; ++c)
+            for (int r = 0; r < circs[c].n_passes; ++r) total += items_of(circs[c].n, q[size_t(r)]);
+        return total;
+    } catch (const std::bad_alloc&) {
+        return -1;
     }
-    return total;
 }
 
 extern "C" size_t qgb_dm_batch_table_bytes(int ncirc, int npasses, int64_t nitems) {
@@ -654,40 +688,42 @@ extern "C" int qgb_dm_batch_build(void* table, size_t table_bytes, const qgb_dm_
     }
     // rounds: the r-th pass of every circuit that has one, in circuit order; items of a pass
     // wait for all items of the circuit's previous pass
-    int maxp = 0;
-    for (int c = 0; c < ncirc; ++c) maxp = circs[c].n_passes > maxp ? circs[c].n_passes : maxp;
-    std::vector<int64_t> item0(size_t(npasses), 0);  // first item of each pass
+    const std::vector<uint64_t> q = item_tiles(circs, ncirc, items_per_pass);
+    std::vector<int64_t> item0(size_t(npasses), 0);    // first item of each pass
+    std::vector<int> count(size_t(npasses), 0);        // its items
+    std::vector<uint32_t> before(size_t(ncirc), 0);    // the circuit's items so far
     int64_t w = 0;
-    for (int r = 0; r < maxp; ++r)
+    for (int r = 0; r < int(q.size()); ++r)
         for (int c = 0; c < ncirc; ++c) {
             if (r >= circs[c].n_passes) continue;
-            const int64_t per = items_of(circs[c].n, items_per_pass);
-            const uint64_t tiles = uint64_t(1) << (2 * circs[c].n - 13);
+            const int64_t per = items_of(circs[c].n, q[size_t(r)]);
+            const uint64_t tiles = tiles_of(circs[c].n);
             item0[size_t(circs[c].first_pass + r)] = w;
+            count[size_t(circs[c].first_pass + r)] = int(per);
             for (int64_t j = 0; j < per; ++j) {
                 I[w].pass = circs[c].first_pass + r;
-                I[w].need = uint32_t(per * r);
+                I[w].need = before[size_t(c)];
                 I[w].t0 = uint32_t(j);
                 I[w].tstride = uint32_t(per);
                 I[w].ntiles = uint32_t((tiles - uint64_t(j) + uint64_t(per) - 1) / uint64_t(per));
                 ++w;
             }
+            before[size_t(c)] += uint32_t(per);
         }
     for (int c = 0; c < ncirc; ++c) {  // finishing items, after every pass of the circuit
-        const int64_t per = items_of(circs[c].n, items_per_pass);
         const int lastp = circs[c].first_pass + circs[c].n_passes - 1;
         I[w].pass = lastp;
-        I[w].need = uint32_t(per * circs[c].n_passes);
+        I[w].need = before[size_t(c)];
         I[w].t0 = I[w].ntiles = 0;
         I[w].tstride = 1;
         I[w].last0 = item0[size_t(lastp)];
-        I[w].last_items = int(per);
+        I[w].last_items = count[size_t(lastp)];
         ++w;
     }
     for (int p = 0; p < npasses; ++p)
         if (passes[p].flags & kDmbHead) {
             P[p].tail_item0 = item0[size_t(passes[p].tslot)];
-            P[p].tail_items = int(items_of(circs[passes[p].circ].n, items_per_pass));
+            P[p].tail_items = count[size_t(passes[p].tslot)];
         }
     return w == nitems ? QGB_OK : set_error(QGB_EINVAL, "item count mismatch");
 }

@@ -1145,6 +1145,7 @@ __global__ void adjoint_sweep_finish_kernel(const double* __restrict__ partials,
     const int op = int(item - b * n_ops);
     if (a.op_out[op] < 0) return;
     double s = 0.0;
+#pragma unroll 16  // loads ahead of the (ordered) additions: 24 qubits 20.7 us a sweep one after the other, 11.9 so
     for (int j = lane; j < cps; j += 32) s += partials[(b * cps + j) * n_ops + op];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);

@@ -317,10 +317,10 @@ class _Inputs:
     back through ``matrix_exp``. Every other gate contributes its matrix."""
 
     def __init__(self, gates, closed_form=False):
-        self.mats, self.flat = _matrices(gates, closed_form)
+        of_gate = [_rotation_angle(g) for g in gates]
+        self.mats, self.flat = _matrices(gates, closed_form, of_gate)
         self.rot, angles = [], []
-        for i, g in enumerate(gates):
-            a = _rotation_angle(g)
+        for i, a in enumerate(of_gate):
             if a is not None:
                 self.rot.append(i)
                 angles.append(a)
@@ -403,14 +403,15 @@ class _EnergyFn(torch.autograd.Function):
 _GEN_T = {k: torch.from_numpy(m) for k, m in _GEN.items()}
 
 
-def _matrices(gates, closed_form=False):
+def _matrices(gates, closed_form=False, angles=None):
     """Every gate's matrix as a torch tensor, and all of them flattened into one
     complex128 host array (row-major, gate after gate). With ``closed_form``,
     rotation gates whose matrix has not been built yet (torch angles, see
     ``ParamGate``) get cos(theta) I - i sin(theta) P from their construction-time
     angles, all of a kind in one vectorised step, instead of one ``matrix_exp``
     each; the two differ by the series truncation of ``matrix_exp`` (about
-    2e-10), far below complex64 rounding, so the complex64 paths use it."""
+    2e-10), far below complex64 rounding, so the complex64 paths use it.
+    ``angles``: :func:`_rotation_angle` of every gate where the caller has them."""
     mats = [None] * len(gates)
     sizes = np.array([4 ** len(g.indices) for g in gates], dtype=np.int64)
     offs = np.concatenate([[0], np.cumsum(sizes)])
@@ -419,7 +420,8 @@ def _matrices(gates, closed_form=False):
         by_kind = {}
         for i, g in enumerate(gates):
             kind = _KIND.get(getattr(g, "name", None))
-            if kind is not None and getattr(g, "matrix_pending", lambda: False)() and _rotation_angle(g) is not None:
+            if kind is not None and getattr(g, "matrix_pending", lambda: False)() and (
+                    angles[i] if angles is not None else _rotation_angle(g)) is not None:
                 by_kind.setdefault(kind, []).append(i)
         for kind, idx in by_kind.items():
             if all(gates[i].angles_unchanged() for i in idx):

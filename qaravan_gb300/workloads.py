@@ -22,6 +22,7 @@ circuit families from a ``numpy.random.default_rng(seed)`` stream so every run
 from __future__ import annotations
 
 import numpy as np
+import torch
 
 from .circuits import Circuit, brickwall_skeleton
 from .gates import Gate, RY, RZ, CNOT
@@ -65,11 +66,22 @@ def hea_params(n, layers, seed):
 
 def hea_circuit(n, layers, params):
     """``params[l, q] = (theta, phi)``; NumPy floats or a torch tensor (keeps autograd)."""
+    if torch.is_tensor(params) and params.dim() == 3 and params.is_contiguous():
+        # one view an angle instead of three, each an autograd node (12 us an angle)
+        flat, (s0, s1, _) = params.view(-1), params.stride()
+
+        def angle(l, q, j):
+            return flat[l * s0 + q * s1 + j]
+        if layers > 0 and n > 0 and (params.shape[0] < layers or params.shape[1] < n or params.shape[2] < 2):
+            raise IndexError(f"parameters of shape {tuple(params.shape)} for {layers} layers of {n} sites")
+    else:
+        def angle(l, q, j):
+            return params[l][q][j]
     gl = []
     for l in range(layers):
         for q in range(n):
-            gl.append(RY([q], params[l][q][0]))
-            gl.append(RZ([q], params[l][q][1]))
+            gl.append(RY([q], angle(l, q, 0)))
+            gl.append(RZ([q], angle(l, q, 1)))
         for q in range(n - 1):
             gl.append(CNOT([q + 1, q], n))
     return Circuit(gl, n=n)

@@ -533,7 +533,7 @@ using namespace qgb;
 
 namespace {
 
-constexpr uint64_t kDmbMinTiles = 8;
+constexpr uint64_t kDmbMinTiles = 8, kDmbMaxTiles = 32;
 constexpr size_t kDmbSmem = 2 * size_t(TcGeom<6>::B_BYTES) + 2 * size_t(TcGeom<6>::TILE_BYTES) +
                             TcGeom<6>::STAGE_BYTES + 128;
 
@@ -574,7 +574,8 @@ extern "C" size_t qgb_dm_batch_pass_bytes(void) { return sizeof(qgb_dm_pass); }
 // Items of a circuit's pass in round r: its tiles of 8192 entries dealt round-robin, so many a
 // item that the round (the r-th passes of all circuits that have one) is one wave of
 // items_per_pass (the SM count) items, at least kDmbMinTiles (an item builds its operand and
-// fills and drains the pipeline).
+// fills and drains the pipeline) and, in rounds of many circuits, at most kDmbMaxTiles or one
+// wave of the pass alone: the circuit's next pass waits for all of them.
 static uint64_t tiles_of(int n) { return uint64_t(1) << (2 * n - 13); }
 
 static std::vector<uint64_t> item_tiles(const qgb_dm_circuit* circs, int ncirc, int items_per_pass) {
@@ -590,7 +591,12 @@ static std::vector<uint64_t> item_tiles(const qgb_dm_circuit* circs, int ncirc, 
     return q;
 }
 
-static int64_t items_of(int n, uint64_t q) { return int64_t((tiles_of(n) + q - 1) / q); }
+static int64_t items_of(int n, uint64_t q, int items_per_pass) {
+    uint64_t most = (tiles_of(n) + uint64_t(items_per_pass) - 1) / uint64_t(items_per_pass);
+    if (most < kDmbMaxTiles) most = kDmbMaxTiles;
+    if (q > most) q = most;
+    return int64_t((tiles_of(n) + q - 1) / q);
+}
 
 static int check_tables(const qgb_dm_circuit* circs, int ncirc, const qgb_dm_pass* passes, int npasses,
                         int items_per_pass) {
@@ -639,7 +645,7 @@ extern "C" int64_t qgb_dm_batch_items(const qgb_dm_circuit* circs, int ncirc, in
         const std::vector<uint64_t> q = item_tiles(circs, ncirc, items_per_pass);
         int64_t total = ncirc;  // a finishing item per circuit
         for (int c = 0; c < ncirc; ++c)
-            for (int r = 0; r < circs[c].n_passes; ++r) total += items_of(circs[c].n, q[size_t(r)]);
+            for (int r = 0; r < circs[c].n_passes; ++r) total += items_of(circs[c].n, q[size_t(r)], items_per_pass);
         return total;
     } catch (const std::bad_alloc&) {
         return -1;
@@ -696,7 +702,7 @@ extern "C" int qgb_dm_batch_build(void* table, size_t table_bytes, const qgb_dm_
     for (int r = 0; r < int(q.size()); ++r)
         for (int c = 0; c < ncirc; ++c) {
             if (r >= circs[c].n_passes) continue;
-            const int64_t per = items_of(circs[c].n, q[size_t(r)]);
+            const int64_t per = items_of(circs[c].n, q[size_t(r)], items_per_pass);
             const uint64_t tiles = tiles_of(circs[c].n);
             item0[size_t(circs[c].first_pass + r)] = w;
             count[size_t(circs[c].first_pass + r)] = int(per);

@@ -1,7 +1,8 @@
 """Items of the persistent density-matrix batch (host code): every pass's tiles are
-dealt exactly once, a round is one wave of items where its circuits have the tiles
-for it, no item is smaller than 8 tiles unless its pass is, and an item waits for
-exactly the items of its circuit's earlier passes."""
+dealt exactly once, a round is one wave of items unless that takes items of more
+than 32 tiles and more than one wave of the pass alone, no item is smaller than 8
+tiles unless its pass is, and an item waits for exactly the items of its circuit's
+earlier passes."""
 import numpy as np
 import pytest
 
@@ -48,8 +49,10 @@ def test_items(lib, circuits, sms):
             assert np.array_equal(np.sort(got), np.arange(tiles))
             assert np.all(mine["need"] == before)
             assert len(mine) == 1 or mine["ntiles"].max() >= 8
-            rounds.setdefault(j, []).append(len(mine))
+            most = max(32, -(-tiles // sms))
+            assert mine["ntiles"].max() <= most
+            rounds.setdefault(j, []).append((len(mine), mine["ntiles"].max() == most or len(mine) == -(-tiles // most)))
             before += len(mine)
         assert fin[i]["need"] == before and fin[i]["last_items"] == len(mine)
     for r, counts in rounds.items():  # a wave: at most one item a pass beyond the SMs (the rounding up)
-        assert sum(counts) <= sms + len(counts)
+        assert sum(k for k, _ in counts) <= sms + len(counts) or any(capped for _, capped in counts)

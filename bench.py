@@ -216,7 +216,8 @@ def fma_peaks():
 
 
 def c128_roofline(plan, n, ms, double_float, peaks):
-    """Roofline of a complex128 sweep plan: float64 kernels against the measured
+    """Roofline of a complex128 plan: dense passes (5-qubit blocks in fixed point on
+    the tensor cores) against the HBM copy rate; sweeps with float64 kernels against the measured
     FP64 FMA rate (8 flops per complex multiply-add); double-float kernels
     against the measured FP32 rate, counting the FP32 pipe's work -- one
     double-float complex multiply-add is 4 real terms of 1 multiply, 3 FMAs and
@@ -225,7 +226,13 @@ def c128_roofline(plan, n, ms, double_float, peaks):
     from qaravan_gb300.compiler import plan_flops
     flops64 = plan_flops(plan)[1] * 2 ** n  # 8 per complex multiply-add
     out = {"tflops_fp64_equivalent": round(flops64 / (ms / 1e3) / 1e12, 3)}
-    if double_float:
+    if plan.steps and all(type(s).__name__ == "DenseStep" and len(s.bits) == 5 for s in plan.steps):
+        peak, kind = _peaks()
+        achieved = 2 * 16 * 2 ** n * len(plan.steps) / (ms / 1e3) / 1e9
+        out["arithmetic"] = "fixed point, 9-bit digits on the tensor cores"
+        out["roofline"] = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
+                           "frac": round(achieved / peak, 3), "peak_source": f"hbm_gbs of {kind}"}
+    elif double_float:
         achieved = 2 * 48 * (flops64 / 8) / (ms / 1e3) / 1e12
         out["roofline"] = {"bound": "fp32", "achieved": round(achieved, 2), "peak": peaks["fp32_tflops"],
                            "unit": "TFLOP/s", "frac": round(achieved / peaks["fp32_tflops"], 3),
@@ -241,7 +248,9 @@ def c128_roofline(plan, n, ms, double_float, peaks):
 
 def section_c128(n, gates, steps=3):
     """The benchmark circuit in complex128 through StatevectorSim's default
-    complex128 path (double-float tile sweeps), timed over `steps` runs after a
+    complex128 path (fixed-point blocks on the tensor cores, under the key
+    "double_float" of the arithmetic setting that selects it; double-float tile
+    sweeps below 17 qubits), timed over `steps` runs after a
     warm-up, with its roofline; its final state against the float64 kernels'."""
     import torch
     from qaravan_gb300 import StatevectorSim, _lib

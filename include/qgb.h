@@ -223,7 +223,11 @@ enum {
     QGB_CALL_ROWS = 2,  /* qgb_op_action_unitary                              */
     QGB_CALL_SCALED = 3, /* qgb_op_action_scaled by trace[1]                  */
     QGB_CALL_TRACE = 4, /* qgb_dm_trace_factor on n / 2 sites, start = `link` */
-    QGB_CALL_SWEEP = 5  /* qgb_apply_sweep with `sweep`                       */
+    QGB_CALL_SWEEP = 5, /* qgb_apply_sweep with `sweep`                       */
+    QGB_CALL_FIXED = 6  /* a unitary complex128 block of 5 sites, n >= 12, in fixed point on
+                           the tensor cores: 50 bits relative to the largest amplitude of
+                           each group; else, with qgb_set_c128_arith(0) or
+                           qgb_set_dense_impl(0), as QGB_CALL_OP */
 };
 typedef struct {
     int32_t kind;
@@ -332,7 +336,7 @@ int qgb_dm_batch_run(const void* table, size_t table_bytes, int ncirc, int npass
 /* Arithmetic of complex128 tile sweeps (qgb_apply_sweep): 1 (default) =
  * double-float -- each float64 component carried as a pair of floats (48
  * significant bits) inside the tile, FP32 instructions only, the state in HBM
- * still complex128 -- 0 = float64 kernels. Process-wide; QGB_C128_ARITH=fp64
+ * still complex128 -- 0 = float64 kernels, QGB_CALL_FIXED included. Process-wide; QGB_C128_ARITH=fp64
  * selects 0 at start-up. No reference counterpart: the reference's numpy
  * complex128 op_action (tensorQ/statevector_sim.py:124-140) has one arithmetic. */
 int qgb_set_c128_arith(int mode);

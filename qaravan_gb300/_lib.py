@@ -69,7 +69,7 @@ class AdjointSweep(C.Structure):
     ]
 
 
-QGB_CALL_OP, QGB_CALL_CHAIN, QGB_CALL_ROWS, QGB_CALL_SCALED, QGB_CALL_TRACE, QGB_CALL_SWEEP = range(6)
+QGB_CALL_OP, QGB_CALL_CHAIN, QGB_CALL_ROWS, QGB_CALL_SCALED, QGB_CALL_TRACE, QGB_CALL_SWEEP, QGB_CALL_FIXED = range(7)
 
 
 class Call(C.Structure):

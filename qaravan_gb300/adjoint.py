@@ -90,8 +90,7 @@ class _Runner:
                                device_fusion=True)
         else:
             plan = compile_ops(ops, n, mode=self.sim.mode, width=self.sim.fusion_width, tile_bits=self.sim.tile_bits,
-                               low_bits=self.sim.low_bits, max_sweep_k=kcap, itemsize=isz, device_fusion=True, pack=True,
-                               pad=self.sim._pad())
+                               low_bits=self.sim.low_bits, max_sweep_k=kcap, itemsize=isz, device_fusion=True, pack=True)
         self.sim.initialize_state()  # |0..0>, a bitstring or a given array (copied), as the simulator starts
         psi = self.sim.state.detach().reshape(-1)
         self.sim.state = None  # psi is the only reference: no extra state-sized buffer
@@ -194,7 +193,7 @@ _REV_CACHE: dict = {}
 
 def _tile_bits(dtype):
     """Tile of the adjoint sweeps: state and co-state double-buffered in shared
-    memory (4 x 2^m amplitudes: 64 KiB at m = 11 for complex64, three CTAs per
+    memory (4 x 2^m amplitudes: 64 KiB at m = 11 for complex64, two CTAs per
     SM, the fastest of m = 10-12 measured on 64 sets of 20 qubits; 128 KiB at
     m = 11 for complex128)."""
     return 11

@@ -37,7 +37,7 @@ import torch
 SV_CANDIDATES = {
     torch.complex64: [("fused", 6, 14), ("fused", 5, 14), ("fused", 4, 14), ("tcsweep", 5, 13), ("sweep", 4, 14),
                       ("sweep", 3, 12)],
-    torch.complex128: [("sweep", 3, 13), ("sweep", 2, 13), ("sweep", 4, 12), ("fused", 5, 13), ("fused", 3, 13),
+    torch.complex128: [("sweep", 3, 13), ("sweep", 2, 13), ("sweep", 4, 12), ("fixed", 5, 13), ("fused", 3, 13),
                        ("fused", 2, 13)],
 }
 TRAJ_CANDIDATES = {torch.complex64: [11, 12, 13, 14], torch.complex128: [11, 12, 13]}
@@ -115,7 +115,7 @@ def default_sv(n, dtype):
         return ("fused", 6, 14) if tc else ("sweep", 4, 14)
     # depth-20 brickwork, 5-qubit blocks in fixed point on the tensor cores against double-float tile
     # sweeps: 16 qubits 593 / 552 us, 17 qubits 595 / 1015 us, 20 qubits 1.51 / 3.51 ms
-    return ("fused", 5, 13) if n >= 17 and fixed_point() else ("sweep", 3, 13)
+    return ("fixed", 5, 13) if n >= 17 and fixed_point() else ("sweep", 3, 13)
 
 
 def fixed_point() -> bool:

@@ -50,6 +50,7 @@ class DenseStep:
     mat: int  # index into the plan's matrix list
     unitary: bool = False  # the block is unitary (every op in it is): its launch may restore group norms
     whole: bool = False  # density matrices: the ops applied up to this step form whole channels (no half gate)
+    fixed: bool = False  # complex128: a unitary 5-bit block that may run in fixed point on the tensor cores
 
 
 @dataclass
@@ -510,7 +511,7 @@ def _remember_plan(key, plan):
 
 
 def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, max_sweep_k=5, itemsize=8,
-                device_fusion=False, pack=False, pad=0):
+                device_fusion=False, pack=False):
     """Compile an op sequence (with ``None`` marking a renormalisation point)
     into a :class:`Plan`.
 
@@ -522,12 +523,17 @@ def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, 
     of shared memory. ``device_fusion``: block matrices are left as
     :class:`Recipe` objects for the executor to compose on the GPU. ``pack``
     (dense passes of device-fused blocks): the blocks of :func:`fuse_frontier`,
-    run from either end, when they are fewer; every block of fewer than ``pad`` bits
-    widened to ``pad`` (identity on the lowest free bits) -- fewer passes, the ops in another of their
-    valid orders. The kernel that ``pad`` serves takes unitary blocks of that width: a segment with
-    another op or a wider one runs as 3-bit blocks in tile sweeps.
+    run from either end, when they are fewer -- fewer passes, the ops in another of their valid orders.
+    ``"fixed"`` (complex128, at least 12 bits, device fusion): such blocks of 5 bits, narrower ones
+    widened with the identity on the lowest free bits, marked for the fixed-point kernel; it takes
+    unitary blocks, so a segment with another op or a wider one runs as 3-bit blocks in tile sweeps.
     """
     tile_bits = min(tile_bits, 14 if itemsize <= 8 else 13)
+    pad = 0
+    if mode == "fixed" and itemsize > 8 and nbits >= 12 and device_fusion:
+        mode, width, pad, pack = "fused", 5, 5, True
+    elif mode == "fixed":
+        mode, width = "sweep", 3
     # unitarity of every op with a matrix, batched once (the plan key, trace checks and fusion use it)
     mops = [o for o in ops if o is not None and o.kind != "pauli_mix"]
     ucache = dict(zip(map(id, mops), unitary_flags(mops))) if mops else {}
@@ -606,9 +612,9 @@ def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, 
                         for b in reversed(fuse_frontier(seg[::-1], w))]
                 sym = min(sym, fuse_frontier(seg, w), back, key=len)  # the first of the shortest
                 for b in sym:
-                    if padded and len(b.bits) < min(pad, nbits):
+                    if padded and len(b.bits) < pad:
                         free = [x for x in range(nbits) if x not in b.bits]
-                        b.bits = sorted(b.bits + free[:min(pad, nbits) - len(b.bits)], reverse=True)
+                        b.bits = sorted(b.bits + free[:pad - len(b.bits)], reverse=True)
             blocks = [Block(b.bits, Recipe(list(b.bits), [(base + i, list(seg[i].bits)) for i in b.ops]), b.n_ops)
                       for b in sym]
             bflags = [all(uflags[i] for i in b.ops) for b in sym]
@@ -623,7 +629,7 @@ def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, 
             continue
         if mode == "tcsweep" or (mode == "fused" and (padded or not pad)) or w > max_sweep_k or tile_bits <= 0:
             for b, u, w_ in zip(blocks, bflags, wflags):
-                plan.steps.append(DenseStep(list(b.bits), plan.add_matrix(b.matrix), u, w_))
+                plan.steps.append(DenseStep(list(b.bits), plan.add_matrix(b.matrix), u, w_, padded))
             continue
         for L, high, taken in plan_sweeps(blocks, nbits, tile_bits, low_bits):
             tpos = {b: b for b in range(L)}

@@ -291,7 +291,7 @@ int apply_dense_bits(void* sv, int dtype, int nbits, const int* in_bits, const i
                                     pass);
         if (rc != QGB_EDECLINE) return rc;
     }
-    if (dtype == QGB_C128 && pass.unitary && c128_arith() == 1) {
+    if (dtype == QGB_C128 && pass.fixed && c128_arith() == 1) {
         const int rc = try_dense_oz(sv, op, nbits, a.sorted, in_bits, out_bits, k, batch, st, pass);
         if (rc != QGB_EDECLINE) return rc;
     }
@@ -368,7 +368,7 @@ extern "C" int qgb_run_calls(void* sv, int dtype, int n, const qgb_call* calls, 
     for (int i = 0; i < ncalls; ++i) {
         const qgb_call& c = calls[i];
         const char* op = static_cast<const char*>(mats) + c.mat * int64_t(esz);
-        if (c.kind <= QGB_CALL_SCALED && c.mat < 0) return set_error(QGB_EINVAL, "call %d: negative matrix offset", i);
+        if ((c.kind <= QGB_CALL_SCALED || c.kind == QGB_CALL_FIXED) && c.mat < 0) return set_error(QGB_EINVAL, "call %d: negative matrix offset", i);
         if (c.kind == QGB_CALL_CHAIN && (!chain || c.link < 0 || c.first < 0))
             return set_error(QGB_EINVAL, "call %d: norm chain buffer missing, negative link or epoch", i);
         if ((c.kind == QGB_CALL_SCALED || c.kind == QGB_CALL_TRACE) && !trace)
@@ -384,6 +384,7 @@ extern "C" int qgb_run_calls(void* sv, int dtype, int n, const qgb_call* calls, 
                 pass.first = c.first;
                 break;
             case QGB_CALL_ROWS: pass.unitary = 1; break;
+            case QGB_CALL_FIXED: pass.fixed = 1; break;
             case QGB_CALL_SCALED: pass.scale = trace + 1; break;
             default: break;
         }
@@ -391,6 +392,7 @@ extern "C" int qgb_run_calls(void* sv, int dtype, int n, const qgb_call* calls, 
             case QGB_CALL_OP:
             case QGB_CALL_CHAIN:
             case QGB_CALL_ROWS:
+            case QGB_CALL_FIXED:
             case QGB_CALL_SCALED:
                 rc = op_action(sv, dtype, n, c.sites, c.k, op, 0, 1, 0, stream, pass);
                 break;

@@ -359,7 +359,7 @@ int oz_status_read_clear() {
 // errors relative to the row are errors relative to the result.
 int try_dense_oz(void* sv, const void* op, int nbits, const int* sorted, const int* in_bits, const int* out_bits, int k,
                  int64_t batch, cudaStream_t st, const DensePass& pass) {
-    if (k != kOzK || nbits < kOzTileBits || batch != 1 || !pass.unitary || pass.scale) return QGB_EDECLINE;
+    if (k != kOzK || nbits < kOzTileBits || batch != 1 || !pass.fixed || pass.scale) return QGB_EDECLINE;
     if (qgb_get_dense_impl() == 0) return QGB_EDECLINE;
     OzArgs a{};
     int nt = 0, ng = 0, ti = 0;

@@ -205,6 +205,7 @@ struct DensePass {
     int first = 0;                  //   passes of its first epoch (0: as many as of the others)
     const double* scale = nullptr;  // device factor of the operator (unitary = 0)
     int reverse = 0;                // tiles in descending order
+    int fixed = 0;                  // complex128: a unitary block that may run in fixed point (dense_oz.cu)
 };
 int try_dense_tc(void* sv, const void* op, int nbits, const int* sorted, const int* in_bits, const int* out_bits,
                  int k, int64_t op_stride, int64_t batch, int64_t sv_stride, cudaStream_t st, const DensePass& pass);

@@ -127,7 +127,7 @@ class Executor:
                 nb = plan.nbits
                 sites = [nb - 1 - b for b in s.bits]
                 self._steps.append(("dense", _lib.int_array(sites), len(sites), offs[s.mat], s.unitary, s.whole,
-                                    tc_eligible(self.code, nb, len(sites))))
+                                    tc_eligible(self.code, nb, len(sites)), s.fixed))
             elif isinstance(s, SweepStep):
                 sw = _lib.Sweep()
                 sw.low_bits = s.low_bits
@@ -267,7 +267,7 @@ class Executor:
                 e0 = torch.cuda.Event(enable_timing=True)
                 e0.record()
             if s[0] == "dense" and tchain:
-                _, sites, k, off, unitary, whole, on_tc = s
+                _, sites, k, off, unitary, whole, on_tc = s[:7]
                 if on_tc and t_pending:
                     _lib.check(L.qgb_op_action_scaled(ptr, self.code, nb, sites, k, mptr + off * self.itemsize,
                                                       tptr + 8, st), "op_action")
@@ -285,7 +285,12 @@ class Executor:
                 _, sites, k, off, unitary = s[:5]
                 # per-vector matrices (mat_stride) need not be unitary: only the plan's own are flagged
                 mode = _NORM_RESTORE if (unitary and mats is self.mats) else "off"
-                if mode == "chain" and batch == 1:
+                if s[7] and batch == 1 and mats is self.mats:
+                    call = _lib.Call(kind=_lib.QGB_CALL_FIXED, k=k, mat=off)
+                    for j in range(k):
+                        call.sites[j] = sites[j]
+                    _lib.check(L.qgb_run_calls(ptr, self.code, nb, C.byref(call), 1, mptr, None, None, st), "op_action")
+                elif mode == "chain" and batch == 1:
                     if getattr(self, "_chain", None) is None:
                         self._chain = torch.zeros(6, dtype=torch.float64, device=self.device)
                     _lib.check(L.qgb_op_action_unitary_chain(ptr, self.code, nb, sites, k, mptr + off * self.itemsize,
@@ -293,8 +298,7 @@ class Executor:
                                "op_action")
                     link += 1
                 else:
-                    c128 = unitary and mats is self.mats and self.code == _lib.QGB_C128  # fixed-point blocks
-                    fn = L.qgb_op_action if mode == "off" and not c128 else L.qgb_op_action_unitary
+                    fn = L.qgb_op_action if mode == "off" else L.qgb_op_action_unitary
                     _lib.check(fn(ptr, self.code, nb, sites, k, mptr + off * self.itemsize,
                                   mat_stride if mat_stride else 0, batch, stride, st), "op_action")
                     link = 0
@@ -356,8 +360,7 @@ class Executor:
         entries and trace measurements that ``run`` takes step by step. The norm
         chain knows its length here: its first epoch is cut so that the chain's last
         pass opens an epoch and corrects the drift of every pass but its own, and
-        unitary blocks on the CUDA cores, which do not drift, leave it running. Unitary
-        complex128 blocks are marked in every mode: the mark picks the kernel, no factor."""
+        unitary blocks on the CUDA cores, which do not drift, leave it running."""
         calls, chains, t_since, t_pending = [], [[]], 0, False
         if tchain:
             calls.append((_lib.QGB_CALL_TRACE, None, 0, 1, 0, None))
@@ -366,8 +369,10 @@ class Executor:
                 calls.append((_lib.QGB_CALL_SWEEP, None, 0, 0, 0, s[1]))
                 chains.append([])
                 continue
-            _, sites, k, off, unitary, whole, on_tc = s
-            if tchain:
+            _, sites, k, off, unitary, whole, on_tc, fixed = s
+            if fixed:
+                calls.append((_lib.QGB_CALL_FIXED, sites, k, 0, off, None))
+            elif tchain:
                 scaled = on_tc and t_pending
                 calls.append((_lib.QGB_CALL_SCALED if scaled else _lib.QGB_CALL_OP, sites, k, 0, off, None))
                 t_pending = t_pending and not scaled
@@ -378,7 +383,7 @@ class Executor:
             elif unitary and mode == "chain" and on_tc:
                 chains[-1].append(len(calls))
                 calls.append((_lib.QGB_CALL_CHAIN, sites, k, len(chains[-1]) - 1, off, None))
-            elif unitary and (mode != "off" or self.code == _lib.QGB_C128):
+            elif unitary and mode != "off":
                 calls.append((_lib.QGB_CALL_ROWS, sites, k, 0, off, None))
             else:
                 calls.append((_lib.QGB_CALL_OP, sites, k, 0, off, None))

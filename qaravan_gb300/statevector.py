@@ -108,7 +108,8 @@ class StatevectorSim:
         if mode == "auto":
             from . import autotune
             a_mode, a_width, a_tile = autotune.choose_sv(circ.num_sites, dtype)
-            mode = a_mode
+            # the fixed-point blocks are 5 qubits wide: another width asked for is a sweep's
+            mode = "sweep" if a_mode == "fixed" and fusion_width not in (None, a_width) else a_mode
             fusion_width = a_width if fusion_width is None else fusion_width
             tile_bits = a_tile if tile_bits is None else tile_bits
         if fusion_width is None:
@@ -141,13 +142,6 @@ class StatevectorSim:
         else:
             raise ValueError("init_state must be a NumPy array, Torch tensor, or a bitstring")
 
-    def _pad(self):
-        """Width every fused block is widened to: complex128 blocks of 5 qubits run in
-        fixed point on the tensor cores (at least 12 qubits), narrower ones on the FP64 pipe."""
-        from . import autotune
-        return 5 if (self.dtype == torch.complex128 and self.mode == "fused" and self.fusion_width == 5
-                     and self.num_sites >= 12 and autotune.fixed_point()) else 0
-
     def compile(self):
         if self._exec is None:
             seq = circuit_ops(self.circ, build=True, nm=self.nm)
@@ -155,8 +149,7 @@ class StatevectorSim:
             kcap = 5 if self.dtype == torch.complex64 else 4
             plan = compile_ops(ops, self.num_sites, mode=self.mode, width=self.fusion_width,
                                tile_bits=self.tile_bits, low_bits=self.low_bits, max_sweep_k=kcap,
-                               itemsize=torch.empty(0, dtype=self.dtype).element_size(), device_fusion=True, pack=True,
-                               pad=self._pad())
+                               itemsize=torch.empty(0, dtype=self.dtype).element_size(), device_fusion=True, pack=True)
             self._exec = Executor(plan, self.dtype, self.device)
         return self._exec
 

@@ -7,6 +7,8 @@ others, and whole circuits on the default path.
 Tolerance: components are kept to 2^-50 of their row's largest, the operator to
 2^-51 of its largest entry, so one block's error is below
 64 (2^-50 + 2^-51) max|row| max|w| < 9e-14 max|row| (typically 1e-15)."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -35,8 +37,11 @@ def _run(v, m, sites, n):
     st = torch.from_numpy(v.copy()).cuda()
     op = torch.from_numpy(np.ascontiguousarray(m)).cuda()
     L = _lib.lib()
-    _lib.check(L.qgb_op_action_unitary(st.data_ptr(), 1, n, _lib.int_array(sites), len(sites), op.data_ptr(), 0, 1, 0,
-                                       _lib.stream_ptr(st.device)), "op_action")
+    call = _lib.Call(kind=_lib.QGB_CALL_FIXED, k=len(sites), mat=0)
+    for j, q in enumerate(sites):
+        call.sites[j] = q
+    _lib.check(L.qgb_run_calls(st.data_ptr(), 1, n, ctypes.byref(call), 1, op.data_ptr(), None, None,
+                               _lib.stream_ptr(st.device)), "run_calls")
     _lib.check(L.qgb_check_status(None))
     return st.cpu().numpy()
 
@@ -102,7 +107,7 @@ def test_default_complex128_path(n, depth):
     from qaravan_gb300 import StatevectorSim, workloads
     gates = workloads.brickwork_gates(n, depth, 5)
     sim = StatevectorSim(workloads.brickwork_circuit(n, depth, 5), dtype=torch.complex128)
-    assert (sim.mode, sim.fusion_width) == ("fused", 5)
+    assert (sim.mode, sim.fusion_width) == ("fixed", 5)
     assert all(len(s.bits) == 5 for s in sim.compile().plan.steps)
     assert np.max(np.abs(sim.get_statevector().cpu().numpy() - ref.run_sv(gates, n))) < 1e-13
 
@@ -135,3 +140,31 @@ def test_same_kernel_with_the_norm_off():
     finally:
         engine.set_norm_restore("chain")
     assert torch.equal(a, b)
+
+
+def test_other_entries_keep_their_arithmetic():
+    """Blocks asked for as fused, the unitary entry of the C ABI and another width run as before."""
+    from qaravan_gb300 import StatevectorSim, _lib, workloads
+    n, rng = 17, np.random.default_rng(4)
+    circ = workloads.brickwork_circuit(n, 1, 5)
+    assert not any(s.fixed for s in StatevectorSim(circ, dtype=torch.complex128, mode="fused", fusion_width=5).compile().plan.steps)
+    assert StatevectorSim(circ, dtype=torch.complex128, fusion_width=4).mode == "sweep"
+    v = rng.standard_normal(2 ** 12) + 1j * rng.standard_normal(2 ** 12)
+    m = workloads.haar_unitary(32, rng)
+    st, op = torch.from_numpy(v.copy()).cuda(), torch.from_numpy(m.copy()).cuda()
+    L, sites = _lib.lib(), [0, 1, 2, 3, 4]
+    _lib.check(L.qgb_op_action_unitary(st.data_ptr(), 1, 12, _lib.int_array(sites), 5, op.data_ptr(), 0, 1, 0,
+                                       _lib.stream_ptr(st.device)), "op_action")
+    # float64 sums of 64 products: far below the fixed-point kernel's 2^-50 of the row
+    err = np.abs(st.cpu().numpy() - _apply(v, m, sites, 12))
+    assert np.max(err) < 128 * 2.0 ** -53 * np.max(np.abs(v))
+
+
+def test_steps_one_by_one():
+    """A plan run step by step (with events) gives the one-call run's state."""
+    from qaravan_gb300 import StatevectorSim, workloads
+    sim = StatevectorSim(workloads.brickwork_circuit(17, 1, 5), dtype=torch.complex128)
+    want = sim.run().reshape(-1).clone()
+    sim.initialize_state()
+    sim.compile().run(sim.state, events=[])
+    assert torch.equal(sim.state.reshape(-1), want)

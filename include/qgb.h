@@ -160,7 +160,8 @@ int qgb_fma_probe(int precision, int iters, int blocks_per_sm, void* out, void* 
 
 /* Replaces op_action (tensorQ/statevector_sim.py:124-140) as called by
  * StatevectorSim.apply_gate (:50-52): sv <- op on sites indices[0..k).
- * `op` is a device pointer to the 2^k x 2^k matrix in the state's dtype.
+ * `op` is a device pointer to the 2^k x 2^k matrix in the state's dtype; it must
+ * not overlap the states (so in every entry below that takes operators).
  * batch > 1 applies to `batch` states spaced sv_stride elements apart, each
  * with its own matrix spaced op_stride elements apart (0 = shared matrix). */
 int qgb_op_action(void* sv, int dtype, int n, const int* indices, int k, const void* op,
@@ -244,7 +245,9 @@ typedef struct {
 /* The calls of a plan in order, each as its own entry point would run it on the
  * vector `sv` of n bits (one host call per plan instead of one per launch).
  * Passes over the whole vector alternate between ascending and descending tile
- * order, so that a pass begins with what the previous one left in L2. `chain`
+ * order, so that a pass begins with what the previous one left in L2. A tensor-core
+ * pass that follows another one may read its matrix while that one runs: `mats`
+ * must not overlap sv, chain or trace. `chain`
  * (6 doubles) and `trace` (3 doubles) may be null when no call uses them.
  * Stops at the first failing call. Replaces the per-gate loop of BaseSim.run
  * (core/base_sim.py:30-53). */

@@ -285,6 +285,7 @@ int apply_dense_bits(void* sv, int dtype, int nbits, const int* in_bits, const i
             return check_launch("norm chain reset");
         pass.unitary = 1;
         pass.chain = nullptr;
+        pass.early = 0;
     }
     if (dtype == QGB_C64) {
         const int rc = try_dense_tc(sv, op, nbits, a.sorted, in_bits, out_bits, k, op_stride, batch, sv_stride, st,
@@ -365,6 +366,7 @@ extern "C" int qgb_run_calls(void* sv, int dtype, int n, const qgb_call* calls, 
     if ((reinterpret_cast<uintptr_t>(chain) | reinterpret_cast<uintptr_t>(trace)) % sizeof(double))
         return set_error(QGB_EINVAL, "chain or trace buffer not 8-byte aligned");
     int passes = 0;  // over the whole vector
+    int tensor = 0;  // the call before was one launch on the tensor cores
     for (int i = 0; i < ncalls; ++i) {
         const qgb_call& c = calls[i];
         const char* op = static_cast<const char*>(mats) + c.mat * int64_t(esz);
@@ -376,6 +378,9 @@ extern "C" int qgb_run_calls(void* sv, int dtype, int n, const qgb_call* calls, 
         int rc;
         DensePass pass;
         pass.reverse = passes++ & 1;
+        pass.early = tensor;
+        pass.tensor = &tensor;
+        tensor = 0;
         switch (c.kind) {
             case QGB_CALL_CHAIN:
                 pass.unitary = 2;

@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) dense_oz_kernel(double2* __rest
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
-    // the state is touched from here on (see dense_tc_kernel)
+    // the state is touched from here on; the operator was read before (see dense_tc_kernel)
     tc_grid_wait();
     tc_grid_next();
 
@@ -401,8 +401,9 @@ int try_dense_oz(void* sv, const void* op, int nbits, const int* sorted, const i
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = a.tiles <= 1024 ? 1 : 0;  // while the state fits L2, as dense_tc_kernel
+    cfg.numAttrs = pass.early && a.tiles <= 1024 ? 1 : 0;  // while the state fits L2, as dense_tc_kernel
     cudaLaunchKernelEx(&cfg, dense_oz_kernel, (double2*)sv, (const double2*)op, a);
+    if (pass.tensor) *pass.tensor = 1;
     return check_launch("dense_oz kernel");
 }
 

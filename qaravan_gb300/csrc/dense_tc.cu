@@ -101,9 +101,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) dense_tc_kernel(float2* __restr
     const int q = warp & 3, h = (warp >> 2) & 1;
     // Programmatic dependent launch: this grid may start while the previous pass still runs, its
     // operator built and its tensor memory claimed by the time that pass has finished (64 tiles of
-    // 19 qubits: 11.7 -> 8.8 us a pass). Nothing that a previous kernel may write -- the state, the chain, the
-    // factor -- is touched before tc_grid_wait, and the next grid is let in only after it, so
-    // that everything before the previous pass (the kernel that wrote the operator) is complete.
+    // 19 qubits: 11.7 -> 8.8 us a pass). Nothing that the previous pass may write -- the state, the chain, the
+    // factor -- is touched before tc_grid_wait; the operator is, so the launch before this one must
+    // not have written it. DensePass::early holds that: only a pass that follows another tensor-core
+    // pass of its plan starts early, and that one lets this grid in only after its own tc_grid_wait,
+    // when everything before it (the kernel that wrote the operator) is complete and visible.
     const bool scalars = (MODE == 0 && (a.scale != nullptr || a.chain != nullptr)) || (MODE == 2 && a.c_head);
     if (scalars) {
         tc_grid_wait();
@@ -598,7 +600,7 @@ int dense_impl() {
 }
 
 template <int K, int MODE>
-int launch_tc(float2* sv, const float2* op, const TcArgs& a, cudaStream_t st) {
+int launch_tc(float2* sv, const float2* op, const TcArgs& a, cudaStream_t st, const qgb_host::DensePass& pass) {
     using G = TcGeom<K>;
     static int per_sm = 0;
     if (per_sm == 0) {
@@ -623,8 +625,9 @@ int launch_tc(float2* sv, const float2* op, const TcArgs& a, cudaStream_t st) {
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = a.tiles <= kPdlTiles ? 1 : 0;
+    cfg.numAttrs = pass.early && a.tiles <= kPdlTiles ? 1 : 0;
     cudaLaunchKernelEx(&cfg, dense_tc_kernel<K, MODE>, sv, op, a);
+    if (pass.tensor) *pass.tensor = 1;
     return qgb_host::check_launch("dense_tc kernel");
 }
 
@@ -751,7 +754,9 @@ int try_dense_tc(void* sv, const void* op, int nbits, const int* sorted, const i
     a.reverse = pass.reverse && a.tiles <= kReverseTiles;
     float2* s = static_cast<float2*>(sv);
     const float2* m = static_cast<const float2*>(op);
+    DensePass run = pass;
     if (unitary == 2) {
+        if (pass.link == 0) run.early = 0;  // (the launch before is the reset of the chain)
         // epochs of kChainEpoch passes: the first corrects (and starts the chain), the
         // last measures its output; the passes between run without norm control
         if (pass.link == 0 && cudaMemsetAsync(chain, 0, 6 * sizeof(double), st) != cudaSuccess)
@@ -771,18 +776,18 @@ int try_dense_tc(void* sv, const void* op, int nbits, const int* sorted, const i
         // the correction into the matrix only
         if ((a.c_head && e == 0) || a.c_tail) {
             switch (k) {
-                case 4: return launch_tc<4, 2>(s, m, a, st);
-                case 5: return launch_tc<5, 2>(s, m, a, st);
-                default: return launch_tc<6, 2>(s, m, a, st);
+                case 4: return launch_tc<4, 2>(s, m, a, st, run);
+                case 5: return launch_tc<5, 2>(s, m, a, st, run);
+                default: return launch_tc<6, 2>(s, m, a, st, run);
             }
         }
         if (!a.c_head) a.chain = nullptr;  // a pass inside an epoch: no chain work at all
         unitary = 0;
     }
     switch (k) {
-        case 4: return unitary ? launch_tc<4, 1>(s, m, a, st) : launch_tc<4, 0>(s, m, a, st);
-        case 5: return unitary ? launch_tc<5, 1>(s, m, a, st) : launch_tc<5, 0>(s, m, a, st);
-        default: return unitary ? launch_tc<6, 1>(s, m, a, st) : launch_tc<6, 0>(s, m, a, st);
+        case 4: return unitary ? launch_tc<4, 1>(s, m, a, st, run) : launch_tc<4, 0>(s, m, a, st, run);
+        case 5: return unitary ? launch_tc<5, 1>(s, m, a, st, run) : launch_tc<5, 0>(s, m, a, st, run);
+        default: return unitary ? launch_tc<6, 1>(s, m, a, st, run) : launch_tc<6, 0>(s, m, a, st, run);
     }
 }
 

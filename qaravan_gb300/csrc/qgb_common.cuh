@@ -205,6 +205,9 @@ struct DensePass {
     int first = 0;                  //   passes of its first epoch (0: as many as of the others)
     const double* scale = nullptr;  // device factor of the operator (unitary = 0)
     int reverse = 0;                // tiles in descending order
+    int early = 0;                  // the launch before this one in the stream is a tensor-core pass of the same
+                                    //   plan, so that this one may start before it has finished
+    int* tensor = nullptr;          // set to 1 when the pass was launched on the tensor cores
     int fixed = 0;                  // complex128: a unitary block that may run in fixed point (dense_oz.cu)
 };
 int try_dense_tc(void* sv, const void* op, int nbits, const int* sorted, const int* in_bits, const int* out_bits,

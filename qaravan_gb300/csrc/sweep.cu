@@ -55,12 +55,7 @@ __global__ void __launch_bounds__(kLdstMaxThreads) sweep_ldst_kernel(cplx<T>* __
     const uint32_t lmask = (1u << L) - 1;
     constexpr uint32_t per16 = 16 / sizeof(C);  // amplitudes per 16-byte copy
     const uint64_t total = uint64_t(a.batch) * a.tiles;
-    auto base_of = [&](uint64_t w) -> uint64_t {
-        const uint64_t b = w / a.tiles, o = w - b * a.tiles;
-        uint64_t base = uint64_t(b) * uint64_t(a.sv_stride);
-        for (int j = 0; j < a.n_outer; ++j) base |= ((o >> j) & 1ull) << a.outer_bits[j];
-        return base;  // batch offset plus the scattered tile index (disjoint bits)
-    };
+    auto base_of = [&](uint64_t w) -> uint64_t { return sweep_tile_base(w, a); };
     auto load_async = [&](uint64_t w, C* dst) {
         const uint64_t base = base_of(w);
         for (uint32_t e = per16 * threadIdx.x; e < (1u << m); e += per16 * blockDim.x)

@@ -191,16 +191,14 @@ __global__ void __launch_bounds__(kClThreads, 1)
     const uint32_t part = 1u << ml;
     A* tile = reinterpret_cast<A*>(smem_raw);  // two copies
     A* msh = tile + 2 * size_t(part);          // kClMats matrix entries
-    const uint64_t bt = w / a.tiles, ot = w - bt * a.tiles;
-    uint64_t gbase = bt * uint64_t(a.sv_stride);
-    for (int j = 0; j < a.n_outer; ++j) gbase |= ((ot >> j) & 1ull) << a.outer_bits[j];
-    const cplx<T>* mb = mats + int64_t(bt) * a.mat_stride;
+    const uint64_t gbase = sweep_tile_base(w, a);
+    const cplx<T>* mb = mats + int64_t(w / a.tiles) * a.mat_stride;
     auto offset = [&](uint32_t e) {  // global offset of this part's amplitude e
         const uint32_t u = (rank << ml) | e;
         uint64_t o = u & ((1u << L) - 1u);
         const uint32_t h = u >> L;
         for (int j = 0; j < H; ++j) o |= uint64_t((h >> j) & 1u) << a.sw.high_bits[j];
-        return gbase | o;
+        return gbase + o;  // (the part's bits are disjoint from the tile's, not from the vector's start)
     };
     if (int(threadIdx.x) < nops) {
         ClOp o;

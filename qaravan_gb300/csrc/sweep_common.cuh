@@ -16,6 +16,15 @@ struct SweepArgs {
     uint64_t tiles;  // tiles per vector
 };
 
+// Element offset of work item w's tile: the start of its vector plus the tile's place at the outer
+// bits. Added, never ORed: a batch's stride need not be a multiple of 2^n.
+__device__ __forceinline__ uint64_t sweep_tile_base(uint64_t w, const SweepArgs& a) {
+    const uint64_t b = w / a.tiles, o = w - b * a.tiles;
+    uint64_t tile = 0;
+    for (int j = 0; j < a.n_outer; ++j) tile |= ((o >> j) & 1ull) << a.outer_bits[j];
+    return b * uint64_t(a.sv_stride) + tile;
+}
+
 constexpr int kStageK = 4;  // ops with 3 <= k <= 4 stage their matrix in shared memory
 
 template <int KMAX> __host__ __device__ constexpr int stage_elems() { return KMAX >= 3 ? (1 << (2 * (KMAX < kStageK ? KMAX : kStageK))) : 0; }

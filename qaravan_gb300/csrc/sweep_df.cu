@@ -109,12 +109,7 @@ __global__ void __launch_bounds__(kDfMaxThreads) sweep_df_kernel(double2* __rest
     __syncthreads();
     const uint32_t lmask = (1u << L) - 1;
     const uint64_t total = uint64_t(a.batch) * a.tiles;
-    auto base_of = [&](uint64_t w) -> uint64_t {
-        const uint64_t b = w / a.tiles, o = w - b * a.tiles;
-        uint64_t base = uint64_t(b) * uint64_t(a.sv_stride);
-        for (int j = 0; j < a.n_outer; ++j) base |= ((o >> j) & 1ull) << a.outer_bits[j];
-        return base;
-    };
+    auto base_of = [&](uint64_t w) -> uint64_t { return sweep_tile_base(w, a); };
     auto load_async = [&](uint64_t w, dfc* dst) {
         const uint64_t base = base_of(w);
         for (uint32_t e = threadIdx.x; e < (1u << m); e += blockDim.x)

@@ -83,10 +83,7 @@ __global__ void __maxnreg__(120) sweep_tma_kernel(const __grid_constant__ CUtens
     uint64_t* done = bars + kMaxBuffers;
 
     auto row0_of = [&](uint64_t w) -> uint64_t {
-        const uint64_t b = w / a.tiles, o = w - b * a.tiles;
-        uint64_t base = 0;
-        for (int j = 0; j < a.n_outer; ++j) base |= ((o >> j) & 1ull) << a.outer_bits[j];
-        return ((b * uint64_t(a.sv_stride) + base) * uint64_t(g.W)) >> 4;
+        return (sweep_tile_base(w, a) * uint64_t(g.W)) >> 4;
     };
 
     if (warp == 0) {

@@ -226,8 +226,12 @@ enum {
     QGB_CALL_TRACE = 4, /* qgb_dm_trace_factor on n / 2 sites, start = `link` */
     QGB_CALL_SWEEP = 5, /* qgb_apply_sweep with `sweep`                       */
     QGB_CALL_FIXED = 6  /* a unitary complex128 block of 5 sites, n >= 12, in fixed point on
-                           the tensor cores: 50 bits relative to the largest amplitude of
-                           each group; else, with qgb_set_c128_arith(0) or
+                           the tensor cores: 50 bits relative to the largest amplitude M of
+                           each group. An output i is left to it only where
+                           sum_j |U_ij| |x_j| >= M / 32 is certain (M / 128 in a group of at
+                           most 8 amplitudes, all within 1/8 of M) and formed in double-float
+                           elsewhere, so that its error is relative to that sum, below 2^-38
+                           of it at worst. Else, with qgb_set_c128_arith(0) or
                            qgb_set_dense_impl(0), as QGB_CALL_OP */
 };
 typedef struct {

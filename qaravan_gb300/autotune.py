@@ -20,7 +20,8 @@ seeded workload of that size the first time the size is seen and caches the
 fastest; otherwise it returns the defaults measured on GB300 (complex64
 statevectors: 6-qubit fused blocks on the tensor cores from 13 qubits, else
 4-qubit blocks in one tile sweep; complex128: 5-qubit blocks in fixed point on the
-tensor cores from 17 qubits, else 3-qubit blocks in 13-bit tile sweeps;
+tensor cores from 17 qubits where the circuit spreads amplitudes, else 3-qubit
+blocks in 13-bit tile sweeps;
 trajectories: 13-bit tiles for complex64, 12 for complex128). The cache is a
 JSON file at ``$QGB_AUTOTUNE_CACHE`` (default
 ``~/.cache/qaravan_gb300/autotune.json``). ``select`` is the decision rule
@@ -114,7 +115,8 @@ def default_sv(n, dtype):
         tc = n >= 13 and _lib.lib().qgb_get_dense_impl() >= 1
         return ("fused", 6, 14) if tc else ("sweep", 4, 14)
     # depth-20 brickwork, 5-qubit blocks in fixed point on the tensor cores against double-float tile
-    # sweeps: 16 qubits 593 / 552 us, 17 qubits 595 / 1015 us, 20 qubits 1.51 / 3.51 ms
+    # sweeps: 17 qubits 0.80 / 1.00 ms, 20 qubits 1.89 / 3.49 ms, 16 qubits no faster (circuits that
+    # spread amplitudes less keep the sweeps, compiler._FIXED_SPREAD)
     return ("fixed", 5, 13) if n >= 17 and fixed_point() else ("sweep", 3, 13)
 
 

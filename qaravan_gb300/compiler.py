@@ -431,6 +431,39 @@ def unitary_flags(ops, tol=1e-6):
     return flags
 
 
+def spreading(mats, tol=2 ** 0.5 / 8):
+    """log2 of how many rows a column of each matrix reaches on average, counting the
+    entries of at least 1/8: 1 for a one-site gate that mixes its two states, 0 for a
+    phase, a permutation or a rotation by a small angle, 2 for a Haar pair gate."""
+    out = [0.0] * len(mats)
+    by_dim: dict = {}
+    for i, m in enumerate(mats):
+        by_dim.setdefault(m.shape[0], []).append(i)
+    for d, idx in by_dim.items():
+        m = np.stack([np.asarray(mats[i]) for i in idx])
+        big = (np.abs(m.real) + np.abs(m.imag) >= tol).reshape(len(idx), -1).sum(axis=1)
+        for i, s in zip(idx, np.log2(np.maximum(big / d, 1.0)).tolist()):
+            out[i] = s
+    return out
+
+
+# The fixed-point kernel keeps a group's 32 amplitudes relative to the largest and computes an output
+# again in double-float where the block draws it from small ones only (csrc/dense_oz.cu): phases,
+# permutations and small rotations are computed twice. Its segments spread amplitudes over at least this
+# share of the bits their ops touch, from 19 bits and below. Milliseconds against tile sweeps, from |0..0>
+# and from a random state: 24 qubits, small Trotter steps (share 0) 19.6 / 18.6 and 30.7 / 20.3, Fourier
+# transform (0.1) 8.5 / 11.7 and 13.3 / 13.4, rotations with CNOTs (0.2) 12.4 / 17.0 and 11.6 / 18.7, one-site
+# Haar gates with CNOTs (0.5) 6.1 / 12.4 and 7.4 / 14.1, Haar pairs (0.96) 7.8 / 18.6 and 9.9 / 20.3; 18
+# qubits, 0.5: 0.29 / 0.25 and 0.30 / 0.34, Haar pairs 0.40 / 0.36 and 0.37 / 0.47; 17 qubits, 0.5: 0.30 / 0.22
+# and 0.27 / 0.28, Haar pairs 0.33 / 0.33 and 0.31 / 0.39.
+_FIXED_SPREAD, _FIXED_SPREAD_SMALL, _FIXED_SMALL = 0.15, 0.75, 18
+
+
+def _spreads(seg, nbits):
+    share = _FIXED_SPREAD_SMALL if nbits <= _FIXED_SMALL else _FIXED_SPREAD
+    return sum(spreading([np.asarray(o.matrix) for o in seg])) >= share * sum(len(o.bits) for o in seg)
+
+
 def trace_preserving(op):
     """Whether an op on vec(rho) keeps Tr rho for every rho: a half of a unitary
     gate (unitary on its bits; the other half is its conjugate) or a channel
@@ -526,7 +559,8 @@ def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, 
     run from either end, when they are fewer -- fewer passes, the ops in another of their valid orders.
     ``"fixed"`` (complex128, at least 12 bits, device fusion): such blocks of 5 bits, narrower ones
     widened with the identity on the lowest free bits, marked for the fixed-point kernel; it takes
-    unitary blocks, so a segment with another op or a wider one runs as 3-bit blocks in tile sweeps.
+    unitary blocks, so a segment with another op or a wider one runs as 3-bit blocks in tile sweeps,
+    and so does one whose ops spread amplitudes too little for it (``_FIXED_SPREAD``).
     """
     tile_bits = min(tile_bits, 14 if itemsize <= 8 else 13)
     pad = 0
@@ -562,16 +596,7 @@ def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, 
             pending_loss |= not tp
         trace_kept = not pending_loss
         tp_flags = tuple(tp_list)
-    key = None
-    if device_fusion and mode != "gate" and ops and not any(o is not None and o.kind == "pauli_mix" for o in ops):
-        flags = [ucache[id(o)] for o in ops if o is not None]
-        key = (nbits, mode, width, tile_bits, low_bits, max_sweep_k, itemsize, pack, pad,
-               tuple(None if o is None else tuple(o.bits) for o in ops), tuple(flags), tuple(_pair_offsets(ops)),
-               tp_flags)
-        plan = _cached_plan(key, ops)
-        if plan is not None:
-            return plan
-    plan = Plan(nbits=nbits, n_gates=sum(1 for o in ops if o is not None), trace_kept=trace_kept)
+    # per segment, whether its blocks may go to the fixed-point kernel
     segments, cur = [], []
     for o in ops:
         if o is None or o.kind == "pauli_mix":
@@ -581,7 +606,19 @@ def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, 
         else:
             cur.append(o)
     segments.append(cur)
-    for seg in segments:
+    fixed_segs = tuple(bool(pad) and isinstance(seg, list) and len(seg) > 0 and max(len(o.bits) for o in seg) <= pad
+                       and all(ucache[id(o)] for o in seg) and _spreads(seg, nbits) for seg in segments)
+    key = None
+    if device_fusion and mode != "gate" and ops and not any(o is not None and o.kind == "pauli_mix" for o in ops):
+        flags = [ucache[id(o)] for o in ops if o is not None]
+        key = (nbits, mode, width, tile_bits, low_bits, max_sweep_k, itemsize, pack, pad,
+               tuple(None if o is None else tuple(o.bits) for o in ops), tuple(flags), tuple(_pair_offsets(ops)),
+               tp_flags, fixed_segs)
+        plan = _cached_plan(key, ops)
+        if plan is not None:
+            return plan
+    plan = Plan(nbits=nbits, n_gates=sum(1 for o in ops if o is not None), trace_kept=trace_kept)
+    for seg, padded in zip(segments, fixed_segs):
         if seg is None:
             plan.steps.append(NormalizeStep())
             continue
@@ -600,7 +637,6 @@ def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, 
         tcs = (mode == "tcsweep" and nbits >= 14 and max(len(o.bits) for o in seg) <= 5
                and not any(o.pair is not None or o.kind == "channel" for o in seg))
         widest = max(len(o.bits) for o in seg)
-        padded = bool(pad) and mode == "fused" and widest <= pad and all(uflags)
         w = 5 if tcs else max(width if padded or not pad else 3, widest)
         if device_fusion:
             base = len(plan.op_matrices)

@@ -28,17 +28,31 @@
 // 1.1e-15 to 1.5e-15 of the norm per block, and 7.1e-15 after a 24-qubit circuit of depth 5 where
 // the double-float sweeps leave 4.9e-14.
 //
+// Small amplitudes. An error relative to the row's largest component M is worse than
+// double-float's, which is relative to B_i = sum_j |U_ij| |x_j| of the output, wherever
+// B_i is much smaller than M: phases, permutations, small rotations beside a large
+// amplitude. So an output is left to the products only when B_i >= M / 32 is certain
+// (one product |U_ij| |x_j| of M / 32, or four of M / 128, by bit masks of the entries of
+// at least 1/16, 1/8, 1/4 and of the components within 1, 2, 3 binades of M), or, in a row of at most
+// 8 components that all lie within 3 binades, when one product of M / 128 is (what is
+// rounded is then as large as what is summed). The other outputs are formed in
+// double-float from the staged tile, the products with nonzero entries of the block only,
+// as the tile sweeps form them (sweep_df.cu), while the MMAs run. The certificate costs 6 % of a
+// pass; recomputed outputs, in passes that meet product-like rows, up to four times the pass: 25
+// qubits depth 8 17.8 ms without either, 18.9 with the certificate, 22.1 in all.
+//
 // Data path per CTA (one per SM, 16 warps): a tile is 4096 amplitudes (64 KB: the 5
 // target bits and the 7 lowest others), copied by cp.async one tile ahead; four
 // warps share a lane quarter's rows, 8 components each; digits go to shared memory
 // as K-major core matrices (96 KB), where both operands are read by the MMAs; results
 // come back through that space for coalesced stores, or go straight to memory where a thread's
 // rows are runs of 128 bytes (no target among the three lowest bits: 19.2 to 17.8 ms at 25 qubits).
-// What bounds it: the integer instructions that split and reassemble (about 9000 of 13000 cycles a
-// tile); the products (4100 cycles, the first half overlapped with nothing) come next, memory last:
-// the seven accumulators fill tensor memory, so two tiles cannot be in flight.
-// Measured, brickwork against the double-float sweeps: 17 qubits depth 20 1015 to 595 us, 20 qubits
-// depth 20 3.51 to 1.51 ms, 22 qubits depth 8 6.25 to 2.12 ms, 25 qubits depth 8 48.6 to 17.8 ms.
+// What bounds it: the integer instructions that split and reassemble; the products (4100 cycles a
+// tile, the first half overlapped with nothing) come next, memory last: the seven accumulators fill
+// tensor memory, so two tiles cannot be in flight.
+// Measured, brickwork against the double-float sweeps: 17 qubits depth 20 1.00 to 0.80 ms, 20 qubits
+// depth 20 3.49 to 1.89 ms, 22 qubits depth 8 6.20 to 2.79 ms, 25 qubits depth 8 48.4 to 22.1 ms.
+#include "sweep_df.cuh"
 #include "tc_common.cuh"
 
 namespace qgb {
@@ -54,7 +68,8 @@ constexpr int kOzXBytes = 128 * kOzR * 2;       // one digit of 128 rows
 constexpr int kOzHalf = kOzR / 2;               // output columns of half the components
 constexpr int kOzWRows = kOzSums * kOzHalf;     // B rows of a half: the digits one after the other, then zeros
 constexpr int kOzWBytes = kOzWRows * kOzR * 2;  // the operator's digits for one half
-constexpr size_t kOzSmem = size_t(kOzDigits) * kOzXBytes + 2 * kOzWBytes + sizeof(double2) * kOzTile + 128;
+constexpr size_t kOzSmem = size_t(kOzDigits) * kOzXBytes + 2 * kOzWBytes + sizeof(double2) * kOzTile +
+                           sizeof(double2) * kOzThreads + 128;
 // kind::f16, fp32 accumulator, K-major fp16 operands, M = 128, N columns
 __host__ __device__ constexpr uint32_t oz_idesc(int n) {
     return (1u << 4) | (uint32_t(n >> 3) << 17) | (uint32_t(128 >> 4) << 24);
@@ -70,6 +85,10 @@ struct OzArgs {
     int reverse;
     int direct;                  // no target among the three lowest bits: rows are written straight from registers
 };
+
+// The certificate (see above): this many products of entries of at least 1/16 and components of at least 1/8
+// of the row's largest (2 binades); one where the row has at most 8 components, all that large.
+constexpr int kOzNear = 2, kOzCount = 4, kOzSparse = 8;
 
 // 16-byte element swizzle of the staged tile (linear over XOR).
 __host__ __device__ __forceinline__ uint32_t oz_swz(uint32_t e) { return e ^ (((e >> 3) ^ (e >> 6) ^ (e >> 9)) & 7u); }
@@ -136,6 +155,41 @@ __device__ __forceinline__ void oz_mma(uint32_t d, uint64_t a, uint64_t b, uint3
         : "memory");
 }
 
+// The outputs of one row in `unsure` (bit c: output 8 h + c) in double-float, as the tile sweeps form
+// them: the products with the nonzero entries of the block's row, in order. Called by whole warps, a row
+// per lane; tile: the staged tile in double-float, scaled by 2^(896 - bias) a row; urow: the warp's 32 entries.
+__device__ __noinline__ void oz_redo(double2 (&v)[8], uint32_t unsure, int bias, const double2* __restrict__ op,
+                                     const dfc* tile, uint32_t row, const uint32_t* toff, dfc* urow, const OzArgs& a,
+                                     int h, int lane) {
+    const double scale = __hiloint2double((bias + 127) << 20, 0);  // 2^(bias - 896)
+    uint32_t todo = __reduce_or_sync(0xffffffffu, unsure);
+    while (todo) {
+        const int c = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const double2 u = op[a.perm_out[8 * h + c] * kOzD + a.perm_in[lane]];
+        dfc m;
+        df_split(u.x, m.rh, m.rl);
+        df_split(u.y, m.ih, m.il);
+        urow[lane] = m;
+        uint32_t nz = __ballot_sync(0xffffffffu, u.x != 0.0 || u.y != 0.0);
+        __syncwarp();
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
+        dfc w = {0.f, 0.f, 0.f, 0.f}, y = w;
+        while (nz) {  // an entry's loads ahead of the previous one's product
+            const int j = __ffs(nz) - 1;
+            nz &= nz - 1;
+            const dfc wj = urow[j], yj = tile[row ^ toff[j]];
+            dfc_mac(s, w, y);
+            w = wj;
+            y = yj;
+        }
+        dfc_mac(s, w, y);
+        __syncwarp();
+        const dfc r = dfc_finish(s);
+        v[c] = make_double2(df_join(r.rh, r.rl) * scale, df_join(r.ih, r.il) * scale);
+    }
+}
+
 __global__ void __launch_bounds__(kOzThreads, 1) dense_oz_kernel(double2* __restrict__ sv, const double2* __restrict__ op,
                                                                  const __grid_constant__ OzArgs a) {
     extern __shared__ unsigned char oz_smem_raw[];
@@ -143,16 +197,21 @@ __global__ void __launch_bounds__(kOzThreads, 1) dense_oz_kernel(double2* __rest
     unsigned char* W = base;                                // [half][b_off(digit * 32 + n, k, kOzWRows)]
     unsigned char* X = W + 2 * kOzWBytes;                   // [digit][b_off(row, k, 128)]
     double2* tile = reinterpret_cast<double2*>(X + kOzDigits * kOzXBytes);
+    dfc* urow = reinterpret_cast<dfc*>(tile + kOzTile) + (threadIdx.x & ~31u);  // the warp's row of the block (oz_redo)
     double2* out = reinterpret_cast<double2*>(X);           // the results, once the MMAs have read the digits
     __shared__ __align__(8) uint64_t done[2];  // the accumulators of a half are complete
     __shared__ uint32_t tmem_slot;
-    __shared__ int wexp, row_exp[4][128];
+    __shared__ int wexp;
+    __shared__ uint32_t row_exp[4][128];               // a thread's largest exponent and how far below it its components are
+    __shared__ __align__(16) uint32_t heavy[3][kOzD];  // bit j: entry (i, j) of the block is at least 1/16, 1/8, 1/4, memory order
+    __shared__ uint32_t toff[kOzD];                    // component -> its offset in the staged tile
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int q = warp & 3, h = warp >> 2;  // lane quarter, quarter of the components
     const int rown = 32 * q + lane;
 
     // ---- operator digits
     if (tid == 0) wexp = 0;
+    if (tid < 3 * kOzD) heavy[tid / kOzD][tid % kOzD] = 0;
     __syncthreads();
     {
         double2 v[2];
@@ -162,6 +221,10 @@ __global__ void __launch_bounds__(kOzThreads, 1) dense_oz_kernel(double2* __rest
             const int w = tid + t * kOzThreads, i = w & 31, j = w >> 5;
             v[t] = op[a.perm_out[i] * kOzD + a.perm_in[j]];
             e = max(e, max((__double2hiint(v[t].x) >> 20) & 0x7ff, (__double2hiint(v[t].y) >> 20) & 0x7ff));
+            const float a1 = fabsf(float(v[t].x)) + fabsf(float(v[t].y));  // up to sqrt(2) times the entry
+#pragma unroll
+            for (int l = 0; l < 3; ++l)
+                if (a1 >= 0.08838835f * float(1 << l)) atomicOr(&heavy[l][i], 1u << j);  // sqrt(2) / 16, ..
         }
         atomicMax(&wexp, e);
         __syncthreads();
@@ -221,6 +284,12 @@ __global__ void __launch_bounds__(kOzThreads, 1) dense_oz_kernel(double2* __rest
     for (int j = 0; j < 7; ++j) su |= uint32_t((rown >> j) & 1) << a.pos_g[j];
     su |= uint32_t(h & 1) << a.pos_t[3] | uint32_t(h >> 1) << a.pos_t[4];
     su = oz_swz(su);
+    if (tid < kOzD) {
+        uint32_t o = 0;
+#pragma unroll
+        for (int j = 0; j < kOzK; ++j) o |= uint32_t((tid >> j) & 1) << a.pos_t[j];
+        toff[tid] = oz_swz(o);
+    }
     const uint32_t t1 = oz_swz(1u << a.pos_t[0]), t2 = oz_swz(1u << a.pos_t[1]), t4 = oz_swz(1u << a.pos_t[2]);
     auto at = [&](int c) { return su ^ (c & 1 ? t1 : 0u) ^ (c & 2 ? t2 : 0u) ^ (c & 4 ? t4 : 0u); };
     uint64_t gr = 0;  // and their global offsets
@@ -238,15 +307,55 @@ __global__ void __launch_bounds__(kOzThreads, 1) dense_oz_kernel(double2* __rest
         if (__syncthreads_or(fail)) break;
         double2 v[8];
         int e = 0;
+        {
+            int ec[8];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            v[c] = tile[at(c)];
-            e = max(e, max((__double2hiint(v[c].x) >> 20) & 0x7ff, (__double2hiint(v[c].y) >> 20) & 0x7ff));
+            for (int c = 0; c < 8; ++c) {
+                v[c] = tile[at(c)];
+                ec[c] = max((__double2hiint(v[c].x) >> 20) & 0x7ff, (__double2hiint(v[c].y) >> 20) & 0x7ff);
+                e = max(e, ec[c]);
+            }
+            uint32_t code = uint32_t(e) << 16;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const uint32_t d = uint32_t(min(e - ec[c], 3));
+                code |= (d & 1u) << c | (d >> 1) << (8 + c);
+                if (ec[c] > 0 && d == 3) code |= 1u << 31;
+            }
+            row_exp[h][rown] = code;
         }
-        row_exp[h][rown] = e;
-        __syncthreads();  // (and the tile's space is free)
-        if (k + 1 < ntiles) load(t0 + (k + 1) * step);
-        e = max(max(row_exp[0][rown], row_exp[1][rown]), max(row_exp[2][rown], row_exp[3][rown]));
+        __syncthreads();
+        uint32_t unsure = 0;  // bit c: this thread's output c is not certified
+        {
+            uint32_t code[4], near[3] = {0, 0, 0};  // bit j: component j of the row is at least 1/2, 1/4, 1/8 of the largest
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                code[p] = row_exp[p][rown];
+                e = max(e, int((code[p] >> 16) & 0x7ffu));
+            }
+            bool rest = false;  // the row has other components
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                const int ep = int((code[p] >> 16) & 0x7ffu), left = kOzNear - (e - ep);  // binades below that still count
+                const uint32_t d0 = code[p], d1 = code[p] >> 8, three = ~(d0 & d1);
+                const uint32_t upto[3] = {~(d0 | d1), ~d1, three};  // components at most 0, 1, 2 binades below the thread's largest
+#pragma unroll
+                for (int l = 0; l < 3; ++l) {
+                    const int b = left - (2 - l);
+                    near[l] |= ((b < 0 ? 0u : b == 0 ? upto[0] : b == 1 ? upto[1] : upto[2]) & 0xffu) << (8 * p);
+                }
+                rest |= ep > 0 && ((code[p] >> 31) != 0 || (three & ~(near[2] >> (8 * p)) & 0xffu) != 0);
+            }
+            // B >= M / 32: one product of 1/32, or kOzCount of 1/128 (sparse rows: see above)
+            const int want = !rest && __popc(near[2]) <= kOzSparse ? 1 : kOzCount;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const uint32_t h16 = heavy[0][8 * h + c], h8 = heavy[1][8 * h + c], h4 = heavy[2][8 * h + c];
+                const uint32_t one = (h16 & near[0]) | (h8 & near[1]) | (h4 & near[2]);
+                unsure |= uint32_t(one == 0 && __popc(near[2] & h16) < want) << c;
+            }
+            if (e == 0 || e == 0x7ff || we == 0x7ff) unsure = 0;  // zeros, and rows that become NaN
+        }
 #pragma unroll
         for (int c0 = 0; c0 < 8; c0 += 4) {  // 4 components: 8 fp16 of one core-matrix row
             uint32_t w[kOzDigits][4];
@@ -263,7 +372,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) dense_oz_kernel(double2* __rest
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         tc_fence_before();
-        __syncthreads();
+        const bool redo = __syncthreads_or(unsure);
         tc_fence_after();
         if (warp == 0) {
             if (lane == 0) {
@@ -283,6 +392,24 @@ __global__ void __launch_bounds__(kOzThreads, 1) dense_oz_kernel(double2* __rest
             }
             __syncwarp();
         }
+        if (redo) {  // (every thread has read its components: the tile is converted in place)
+            const int bias = max(e - 127, 1);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                dfc y;
+                df_split(v[c].x, y.rh, y.rl, bias);
+                df_split(v[c].y, y.ih, y.il, bias);
+                reinterpret_cast<dfc*>(tile)[at(c)] = y;
+            }
+            __syncthreads();
+            double2 w[8];  // (the callee's argument lives in memory; v stays in registers)
+            oz_redo(w, unsure, bias, op, reinterpret_cast<const dfc*>(tile), su ^ (h & 1 ? toff[8] : 0u) ^ (h & 2 ? toff[16] : 0u),
+                    toff, urow, a, h, lane);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) v[c] = w[c];
+            __syncthreads();
+        }
+        if (k + 1 < ntiles) load(t0 + (k + 1) * step);  // the tile's space is free
         if (!tc_wait_bounded(tc_smem_u32(&done[h >> 1]), uint32_t(k & 1))) {
             fail = true;
             if (lane == 0) atomicExch(&g_oz_status, 1);
@@ -309,7 +436,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) dense_oz_kernel(double2* __rest
                     x[s] = r[s][2 * c];
                     y[s] = r[s][2 * c + 1];
                 }
-                v[c0 + c] = make_double2(oz_join(x, ey), oz_join(y, ey));
+                if (!((unsure >> (c0 + c)) & 1u)) v[c0 + c] = make_double2(oz_join(x, ey), oz_join(y, ey));
                 if (bad)
                     v[c0 + c] = make_double2(__longlong_as_double(0x7ff8000000000000ll), __longlong_as_double(0x7ff8000000000000ll));
             }

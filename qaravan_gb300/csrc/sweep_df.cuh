@@ -10,13 +10,14 @@ struct dfc {  // one complex128 amplitude as two double-float numbers: 16 bytes,
     float rh, rl, ih, il;
 };
 
-__device__ __forceinline__ void df_split(double x, float& h, float& l) {
+// x 2^(896 - bias) as a pair of floats (bias >= 1).
+__device__ __forceinline__ void df_split(double x, float& h, float& l, int bias = 896) {
     const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(x));
     const uint32_t hw = uint32_t(b >> 32), lw = uint32_t(b);
     const uint32_t sign = hw & 0x80000000u;
     const int E = int((hw >> 20) & 0x7ffu);
-    const int ef = E - 896;  // the float's biased exponent (1023 - 127 = 896)
-    if (ef <= 0) {           // zero, and every |x| < 2^-126
+    const int ef = E - bias;  // the float's biased exponent (1023 - 127 = 896)
+    if (ef <= 0) {            // zero, and every |x| < 2^(bias - 1022)
         h = 0.f;
         l = 0.f;
         return;
@@ -33,7 +34,7 @@ __device__ __forceinline__ void df_split(double x, float& h, float& l) {
         lsign ^= 0x80000000u;
     }
     const int lz = __clz(r);
-    const int el = E - lz - 917;  // biased exponent of r's leading bit: (31 - lz) + (E - 1075) + 127
+    const int el = ef - lz - 21;  // biased exponent of r's leading bit: (31 - lz) + (E - 1075) + bias - 769
     if (r == 0u || el <= 0) {
         l = 0.f;
         return;

@@ -103,8 +103,10 @@ class StatevectorSim:
         # complex64 -> dense fused blocks, one HBM pass each, 6-qubit blocks on the tensor cores
         # from 13 qubits up (half the passes of 4-qubit blocks at the same speed per pass, fastest
         # measured on the 28-qubit brickwork), 4-qubit blocks in one tile sweep below; complex128 ->
-        # 5-qubit blocks in fixed point on the tensor cores from 17 qubits up, below 3-qubit blocks
-        # grouped into tile sweeps (arithmetic dominates, so fewer passes win))
+        # 5-qubit blocks in fixed point on the tensor cores from 17 qubits up where the circuit
+        # spreads amplitudes (outputs that a block draws from small amplitudes only are formed in
+        # double-float), else 3-qubit blocks grouped into tile sweeps (arithmetic dominates, so
+        # fewer passes win))
         if mode == "auto":
             from . import autotune
             a_mode, a_width, a_tile = autotune.choose_sv(circ.num_sites, dtype)

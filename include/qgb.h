@@ -589,6 +589,18 @@ void qgb_philox_uniform(uint32_t event, uint32_t traj, uint32_t stream, uint64_t
 
 /* ---- batches of small uneven circuits ------------------------------------ */
 
+/* Fusion of a circuit's ops into blocks of at most `width` bits (host; no counterpart
+ * in the reference, which applies gate by gate, core/base_sim.py:30-53): op i acts on
+ * bits[begin[i] .. begin[i + 1]); the blocks are a linear extension of the ops' order.
+ * method 0: an op joins the latest block it depends on where it fits; 1: every block is
+ * the best of the sets that grow from the ops that are ready; 2: the fewest blocks of 0,
+ * 1 and 1 from the circuit's end, the first of these on ties. Block j: ops
+ * out_ops[out_begin[j] .. out_begin[j + 1]) in order, on the bits
+ * out_bits[j * width ..][0 .. out_nbits[j]), descending. The arrays hold nops (out_begin:
+ * nops + 1) blocks. Returns the number of blocks or an error code. */
+int qgb_plan_blocks(int method, const int32_t* begin, const int32_t* bits, int nops, int width, int32_t* out_ops,
+                    int32_t* out_begin, int32_t* out_bits, int32_t* out_nbits);
+
 /* Layout sizes of the two device tables qgb_fuse_blocks reads:
  *   block (qgb_fuse_block_bytes() bytes): int64 out (element offset of the
  *     block's 2^k x 2^k row-major matrix in `out`), int32 k (<= 6), int32

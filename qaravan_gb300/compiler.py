@@ -28,10 +28,13 @@ site ``q`` is bit ``n-1-q``.
 from __future__ import annotations
 
 import functools
+import itertools
+import os
 from dataclasses import dataclass, field
 
 import numpy as np
 
+from . import _lib
 from ._lib import QGB_SWEEP_MAX_HIGH, QGB_SWEEP_MAX_OPS, QGB_SWEEP_MAX_TILE_BITS
 
 
@@ -214,41 +217,34 @@ class SymBlock:
         return len(self.ops)
 
 
+def _native_blocks(method, ops, width):
+    """``qgb_plan_blocks`` on objects with ``bits``."""
+    N = len(ops)
+    if not N:
+        return []
+    begin = np.zeros(N + 1, dtype=np.int32)
+    np.cumsum([len(op.bits) for op in ops], out=begin[1:])
+    wide = int(np.max(np.diff(begin)))
+    if wide > width:
+        raise ValueError(f"op on {wide} bits exceeds fusion width {width}")
+    bits = np.fromiter(itertools.chain.from_iterable(op.bits for op in ops), dtype=np.int32, count=int(begin[N]))
+    order, starts = np.empty(N, dtype=np.int32), np.empty(N + 1, dtype=np.int32)
+    sets, sizes = np.empty((N, width), dtype=np.int32), np.empty(N, dtype=np.int32)
+    if not os.path.exists(_lib._build.LIB):
+        _lib._build.build()
+    n = _lib.lib().qgb_plan_blocks(method, begin.ctypes.data, bits.ctypes.data, N, width, order.ctypes.data,
+                                   starts.ctypes.data, sets.ctypes.data, sizes.ctypes.data)
+    if n < 0:
+        _lib.check(n, "plan_blocks")
+    order, starts, sets, sizes = order.tolist(), starts[:n + 1].tolist(), sets[:n].tolist(), sizes[:n].tolist()
+    return [SymBlock(sets[j][:sizes[j]], order[starts[j]:starts[j + 1]]) for j in range(n)]
+
+
 def fuse_symbolic(ops, width):
     """The decisions of :func:`fuse` without the matrix products: blocks of at
     most ``width`` bits, each with the indices of its ops in application order
     (an absorbed earlier block's ops go in front: it is applied first)."""
-    blocks: list = []
-    last: dict = {}
-    for oi, op in enumerate(ops):
-        bits = list(op.bits)
-        if len(bits) > width:
-            raise ValueError(f"op on {len(bits)} bits exceeds fusion width {width}")
-        deps = [last[b] for b in bits if b in last]
-        cand = max(deps) if deps else None
-        if cand is not None and blocks[cand] is not None and len(_union(blocks[cand].bits, bits)) <= width:
-            blk = blocks[cand]
-            u = sorted(_union(blk.bits, bits), reverse=True)
-            blk.ops.append(oi)
-            blk.bits = u
-            for b in bits:
-                last[b] = cand
-            for j in sorted({d for d in deps if d != cand}, reverse=True):
-                bj = blocks[j]
-                if bj is None or not set(bj.bits) <= set(u):
-                    continue
-                if any(blocks[i] is not None and set(blocks[i].bits) & set(bj.bits) for i in range(j + 1, cand)):
-                    continue
-                blk.ops = bj.ops + blk.ops
-                blocks[j] = None
-                for b in bj.bits:
-                    if last.get(b) == j:
-                        last[b] = cand
-            continue
-        blocks.append(SymBlock(sorted(bits, reverse=True) if len(bits) > 1 else list(bits), [oi]))
-        for b in bits:
-            last[b] = len(blocks) - 1
-    return [b for b in blocks if b is not None]
+    return _native_blocks(0, ops, width)
 
 
 def fuse_frontier(ops, width):
@@ -259,96 +255,13 @@ def fuse_frontier(ops, width):
     brickwork circuit is then a rhombus of 9 two-qubit gates on 6 bits, where the
     order-driven :func:`fuse_symbolic` leaves staircases of 7 or 8. Same result type;
     the blocks are a linear extension of the ops' order."""
-    N = len(ops)
-    obits = [tuple(op.bits) for op in ops]
-    queue: dict = {}  # bit -> its ops in order
-    for i, bits in enumerate(obits):
-        if len(bits) > width:
-            raise ValueError(f"op on {len(bits)} bits exceeds fusion width {width}")
-        for b in bits:
-            queue.setdefault(b, []).append(i)
-    for qb in queue.values():
-        qb.append(-1)  # no further op
-    head = dict.fromkeys(queue, 0)
-    weight = [1.0 if len(b) > 1 else 1e-3 for b in obits]
+    return _native_blocks(1, ops, width)
 
-    def take(bits, pos, got):
-        """Continues the in-order application on ``bits`` from ``pos`` (updated);
-        appends the ops taken to ``got`` and returns their weight."""
-        total, work = 0.0, list(bits)
-        while work:
-            b = work.pop()
-            while True:
-                i = queue[b][pos[b]]
-                if i < 0:
-                    break
-                ib = obits[i]
-                ok = True
-                for y in ib:
-                    if y not in pos or queue[y][pos[y]] != i:
-                        ok = False
-                        break
-                if not ok:
-                    break
-                got.append(i)
-                total += weight[i]
-                for y in ib:
-                    pos[y] += 1
-                    if y != b and y not in work:
-                        work.append(y)
-        return total
 
-    def grow(start):
-        pos = {b: head[b] for b in obits[start]}
-        got: list = []
-        total = take(obits[start], pos, got)
-        seen = set(pos)
-        while len(pos) < width:
-            best = None
-            tried = set()
-            for b in sorted(pos):
-                i = queue[b][pos[b]]
-                if i < 0:
-                    continue
-                ext = tuple(sorted(y for y in obits[i] if y not in pos))
-                if not ext or len(pos) + len(ext) > width or ext in tried:
-                    continue
-                tried.add(ext)
-                seen.update(ext)
-                p2 = dict(pos)
-                for y in ext:
-                    p2[y] = head[y]
-                g2: list = []
-                gain = take(list(p2), p2, g2) / len(ext)
-                if best is None or gain > best[0]:
-                    best = (gain, p2, g2)
-            if best is None:
-                break
-            total += best[0] * (len(best[1]) - len(pos))
-            pos = best[1]
-            got += best[2]
-        return total, pos, got, seen
-
-    cache: dict = {}  # start op -> its grown set, while nothing it looked at has moved
-    blocks, done = [], 0
-    while done < N:
-        best = None
-        for b in queue:
-            i = queue[b][head[b]]
-            if i < 0 or obits[i][0] != b or any(queue[y][head[y]] != i for y in obits[i]):
-                continue
-            hit = cache.get(i)
-            if hit is None:
-                hit = cache[i] = grow(i)
-            if best is None or hit[0] > best[0]:
-                best = hit
-        _, pos, got, _ = best
-        blocks.append(SymBlock(sorted(pos, reverse=True), got))
-        done += len(got)
-        head.update(pos)
-        moved = set(pos)
-        cache = {i: hit for i, hit in cache.items() if not (hit[3] & moved)}
-    return blocks
+def fuse_fewest(ops, width):
+    """The fewest blocks of :func:`fuse_symbolic`, :func:`fuse_frontier` and the latter
+    from the circuit's end; the first of these on ties."""
+    return _native_blocks(2, ops, width)
 
 
 def recipe_matrix(recipe, op_matrices):
@@ -556,7 +469,7 @@ def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, 
     of shared memory. ``device_fusion``: block matrices are left as
     :class:`Recipe` objects for the executor to compose on the GPU. ``pack``
     (dense passes of device-fused blocks): the blocks of :func:`fuse_frontier`,
-    run from either end, when they are fewer -- fewer passes, the ops in another of their valid orders.
+    run from either end, when they are fewer (:func:`fuse_fewest`) -- fewer passes, the ops in another of their valid orders.
     ``"fixed"`` (complex128, at least 12 bits, device fusion): such blocks of 5 bits, narrower ones
     widened with the identity on the lowest free bits, marked for the fixed-point kernel; it takes
     unitary blocks, so a segment with another op or a wider one runs as 3-bit blocks in tile sweeps,
@@ -641,14 +554,10 @@ def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, 
         if device_fusion:
             base = len(plan.op_matrices)
             plan.op_matrices.extend(np.ascontiguousarray(o.matrix, dtype=np.complex128) for o in seg)
-            sym = fuse_symbolic(seg, w)
-            if pack and mode == "fused" and (padded or not pad):
-                n = len(seg)
-                back = [SymBlock(b.bits, [n - 1 - i for i in reversed(b.ops)])
-                        for b in reversed(fuse_frontier(seg[::-1], w))]
-                sym = min(sym, fuse_frontier(seg, w), back, key=len)  # the first of the shortest
+            sym = (fuse_fewest if pack and mode == "fused" and (padded or not pad) else fuse_symbolic)(seg, w)
+            if padded:
                 for b in sym:
-                    if padded and len(b.bits) < pad:
+                    if len(b.bits) < pad:
                         free = [x for x in range(nbits) if x not in b.bits]
                         b.bits = sorted(b.bits + free[:pad - len(b.bits)], reverse=True)
             blocks = [Block(b.bits, Recipe(list(b.bits), [(base + i, list(seg[i].bits)) for i in b.ops]), b.n_ops)

@@ -72,6 +72,8 @@ def set_norm_restore(mode="chain"):
 
 
 _FUSE_BLOCK = np.dtype([("out", "<i8"), ("k", "<i4"), ("op_begin", "<i4"), ("op_end", "<i4"), ("pad", "<i4")])
+_CALL = np.dtype([("kind", "<i4"), ("k", "<i4"), ("sites", "<i4", (_lib.QGB_MAX_K,)), ("link", "<i4"),
+                  ("first", "<i4"), ("mat", "<i8"), ("sweep", "<u8")])  # qgb_call
 _FUSE_ENTRY = np.dtype([("k", "<i4"), ("pos", "<i4", (6,)), ("pad", "<i4"), ("mat", "<i8")])
 
 
@@ -127,7 +129,8 @@ class Executor:
                 nb = plan.nbits
                 sites = [nb - 1 - b for b in s.bits]
                 self._steps.append(("dense", _lib.int_array(sites), len(sites), offs[s.mat], s.unitary, s.whole,
-                                    tc_eligible(self.code, nb, len(sites)), s.fixed))
+                                    tc_eligible(self.code, nb, len(sites)), s.fixed,
+                                    tuple(sites + [0] * (_lib.QGB_MAX_K - len(sites)))))
             elif isinstance(s, SweepStep):
                 sw = _lib.Sweep()
                 sw.low_bits = s.low_bits
@@ -362,14 +365,15 @@ class Executor:
         pass opens an epoch and corrects the drift of every pass but its own, and
         unitary blocks on the CUDA cores, which do not drift, leave it running."""
         calls, chains, t_since, t_pending = [], [[]], 0, False
+        none = (0,) * _lib.QGB_MAX_K
         if tchain:
-            calls.append((_lib.QGB_CALL_TRACE, None, 0, 1, 0, None))
+            calls.append((_lib.QGB_CALL_TRACE, none, 0, 1, 0, None))
         for s in self._steps:
             if s[0] == "sweep":
-                calls.append((_lib.QGB_CALL_SWEEP, None, 0, 0, 0, s[1]))
+                calls.append((_lib.QGB_CALL_SWEEP, none, 0, 0, 0, s[1]))
                 chains.append([])
                 continue
-            _, sites, k, off, unitary, whole, on_tc, fixed = s
+            _, _, k, off, unitary, whole, on_tc, fixed, sites = s
             if fixed:
                 calls.append((_lib.QGB_CALL_FIXED, sites, k, 0, off, None))
             elif tchain:
@@ -378,7 +382,7 @@ class Executor:
                 t_pending = t_pending and not scaled
                 t_since += int(on_tc)
                 if whole and t_since >= _TRACE_EPOCH:
-                    calls.append((_lib.QGB_CALL_TRACE, None, 0, 0, 0, None))
+                    calls.append((_lib.QGB_CALL_TRACE, none, 0, 0, 0, None))
                     t_since, t_pending = 0, True
             elif unitary and mode == "chain" and on_tc:
                 chains[-1].append(len(calls))
@@ -389,33 +393,29 @@ class Executor:
                 calls.append((_lib.QGB_CALL_OP, sites, k, 0, off, None))
                 if not unitary:
                     chains.append([])
-        arr = (_lib.Call * max(len(calls), 1))()
-        for c, (kind, sites, k, link, off, sweep) in zip(arr, calls):
-            c.kind, c.k, c.link, c.mat = kind, k, link, off
-            for j in range(k):
-                c.sites[j] = sites[j]
-            if sweep is not None:
-                c.sweep = C.pointer(sweep)
+        first = [0] * len(calls)
         for chain in chains:
             for i in chain:
-                arr[i].first = (len(chain) - 1) % _CHAIN_EPOCH
-        return arr, len(calls)
+                first[i] = (len(chain) - 1) % _CHAIN_EPOCH
+        arr = np.array([(kind, k, sites, link, f, off, 0 if sweep is None else C.addressof(sweep))
+                        for (kind, sites, k, link, off, sweep), f in zip(calls, first)], dtype=_CALL)
+        return arr, arr.ctypes.data_as(C.POINTER(_lib.Call)), len(calls), any(chains)
 
     def _run_calls(self, state, L, ptr, st):
         tchain = self._trace_chained()
         key = (_NORM_RESTORE, tchain)
         hit = self._calls.get(key)
         if hit is None:
-            if L.qgb_call_bytes() != C.sizeof(_lib.Call):
+            if L.qgb_call_bytes() != _CALL.itemsize:
                 raise _lib.QgbError("call table layout mismatch with the library")
             hit = self._calls[key] = self._call_list(*key)
-        arr, count = hit
+        _, arr, count, chained = hit  # (the table points into the sweeps of self._steps)
         chain = trace = None
         if tchain:
             if getattr(self, "_tchain", None) is None:
                 self._tchain = torch.zeros(4, dtype=torch.float64, device=self.device)
             trace = self._tchain.data_ptr()
-        elif _NORM_RESTORE == "chain":
+        elif chained:
             if getattr(self, "_chain", None) is None:
                 self._chain = torch.zeros(6, dtype=torch.float64, device=self.device)
             chain = self._chain.data_ptr()

@@ -71,6 +71,11 @@ int sm_count() {
     return cached;
 }
 
+int current_device() {
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 ? dev & 63 : 0;
+}
+
 }  // namespace qgb_host
 
 extern "C" int qgb_abi_version(void) { return QGB_ABI_VERSION; }

@@ -516,8 +516,9 @@ int try_dense_oz(void* sv, const void* op, int nbits, const int* sorted, const i
     a.tiles = uint64_t(1) << (nbits - kOzTileBits);
     a.direct = a.pos_t[0] >= 3;
     a.reverse = pass.reverse && a.tiles <= 4096;  // states of up to 256 MB, as dense_tc_kernel
-    if (cudaFuncSetAttribute(dense_oz_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kOzSmem)) != cudaSuccess)
-        return check_launch("dense_oz attribute");
+    static std::atomic<uint64_t> done{0};
+    const int rc = allow_smem(dense_oz_kernel, kOzSmem, done, "dense_oz attribute");
+    if (rc) return rc;
     const uint64_t cap = uint64_t(sm_count());
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned(a.tiles < cap ? a.tiles : cap));

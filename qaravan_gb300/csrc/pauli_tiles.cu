@@ -625,11 +625,12 @@ int expect_impl(const void* sv, int n, const PauliTerm* terms, int nterms, int64
                             sizeof(double) * size_t(a.nterms) * kPtWarps;
         constexpr int most = int(2 * sizeof(double2) * (size_t(1) << kPtM) +
                                  kPtMaxTerms * (sizeof(double) * kPtThreads + sizeof(double) * kPtWarps));
-        if (cudaFuncSetAttribute(pauli_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess)
-            return check_launch("pauli tiles attribute");
+        static std::atomic<uint64_t> done{0};
+        int rc = allow_smem(pauli_tile_kernel, most, done, "pauli tiles attribute");
+        if (rc) return rc;
         pauli_tile_kernel<<<dim3(unsigned(bx), unsigned(batch)), kPtThreads, smem, st>>>((const double2*)sv, a, nterms,
                                                                                          partials);
-        const int rc = check_launch("pauli tiles");
+        rc = check_launch("pauli tiles");
         if (rc) return rc;
     }
     *nblk = int(bx);
@@ -645,14 +646,14 @@ int apply_impl(const void* sv, void* out, int n, const PauliTerm* terms, int nte
         a.accumulate = first ? 0 : 1;
         first = false;
         const size_t smem = 2 * sizeof(double2) * (size_t(1) << a.m);
-        if (cudaFuncSetAttribute(pauli_tile_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(2 * sizeof(double2) << kPtM)) != cudaSuccess)
-            return check_launch("pauli apply attribute");
+        static std::atomic<uint64_t> done{0};
+        int rc = allow_smem(pauli_tile_apply_kernel, 2 * sizeof(double2) << kPtM, done, "pauli apply attribute");
+        if (rc) return rc;
         uint64_t bx = (uint64_t(sm_count()) * 12 + uint64_t(batch) - 1) / uint64_t(batch);
         bx = std::min<uint64_t>(std::max<uint64_t>(bx, 1), a.tiles);
         pauli_tile_apply_kernel<<<dim3(unsigned(bx), unsigned(batch)), kPtThreads, smem, st>>>(
             (const double2*)sv, (double2*)out, a);
-        const int rc = check_launch("pauli apply tiles");
+        rc = check_launch("pauli apply tiles");
         if (rc) return rc;
     }
     return QGB_OK;

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/qgb.h"
 
 namespace qgb {
@@ -194,6 +196,17 @@ namespace qgb_host {
 int set_error(int code, const char* fmt, ...);
 int check_launch(const char* what);
 int sm_count();
+int current_device();  // 0 .. 63
+// Dynamic shared memory of a kernel instance, asked for once per device: `done` is the instance's own.
+template <typename F>
+int allow_smem(F* kern, size_t bytes, std::atomic<uint64_t>& done, const char* what) {
+    const uint64_t bit = uint64_t(1) << current_device();
+    if (done.load(std::memory_order_relaxed) & bit) return QGB_OK;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)) != cudaSuccess)
+        return check_launch(what);
+    done.fetch_or(bit, std::memory_order_relaxed);
+    return QGB_OK;
+}
 // Internal status (never returned through the C ABI): a specialised kernel
 // declines an op, and the caller runs the general kernel instead.
 constexpr int QGB_EDECLINE = 1000;

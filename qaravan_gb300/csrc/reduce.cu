@@ -937,9 +937,9 @@ int launch_diag(const void* sv, int n, int64_t stride, const PauliGroup& g, int 
     constexpr size_t most = sizeof(double) * NT * kRedThreads;
     const uint64_t per = (uint64_t(1) << n) / (uint64_t(red_blocks(n)) * kRedThreads) + 1;
     const size_t smem = per >= kChunk * kChunk ? most : 0;
-    if (cudaFuncSetAttribute(pauli_diag_kernel<NT, uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most)) !=
-        cudaSuccess)
-        return check_launch("pauli diagonal attribute");
+    static std::atomic<uint64_t> done{0};
+    const int rc = allow_smem(pauli_diag_kernel<NT, uint32_t>, most, done, "pauli diagonal attribute");
+    if (rc) return rc;
     pauli_diag_kernel<NT, uint32_t><<<dim3(red_blocks(n), unsigned(batch)), kRedThreads, smem, st>>>(
         (const float2*)sv, n, stride, g, nslots, partials);
     return check_launch("pauli diagonal terms");

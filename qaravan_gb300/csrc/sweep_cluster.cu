@@ -285,11 +285,15 @@ int launch_cluster(void* sv, const void* mats, const SweepArgs& a, int rbits, cu
     const int m = a.sw.low_bits + a.sw.n_high;
     const size_t smem = sizeof(typename ClAmp<T>::type) * ((size_t(2) << (m - rbits)) + kClMats);
     auto kern = sweep_cluster_kernel<T, KMAX>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kClSmem) != cudaSuccess)
-        return qgb_host::check_launch("cluster sweep attribute");
-    // (set always: clusters of up to 8 do not need it)
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-        return qgb_host::check_launch("cluster sweep attribute");
+    static std::atomic<uint64_t> done{0}, wide{0};
+    const int rc = qgb_host::allow_smem(kern, kClSmem, done, "cluster sweep attribute");
+    if (rc) return rc;
+    const uint64_t bit = uint64_t(1) << qgb_host::current_device();
+    if (!(wide.load(std::memory_order_relaxed) & bit)) {  // (clusters of up to 8 do not need it)
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+            return qgb_host::check_launch("cluster sweep attribute");
+        wide.fetch_or(bit, std::memory_order_relaxed);
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned((uint64_t(a.batch) * a.tiles) << rbits));
     cfg.blockDim = dim3(kClThreads);

@@ -280,22 +280,64 @@ using namespace qgb;
 
 namespace {
 
+// How many clusters of 2^r CTAs, an SM each, the device runs at a time (0: none, or not known), asked once per
+// kernel instance and device.
 template <typename T, int KMAX>
-int launch_cluster(void* sv, const void* mats, const SweepArgs& a, int rbits, cudaStream_t st) {
-    const int m = a.sw.low_bits + a.sw.n_high;
-    const size_t smem = sizeof(typename ClAmp<T>::type) * ((size_t(2) << (m - rbits)) + kClMats);
+int cluster_room(int r) {
     auto kern = sweep_cluster_kernel<T, KMAX>;
-    static std::atomic<uint64_t> done{0}, wide{0};
+    static std::atomic<int> known[64][kClMaxRankBits + 1];  // 1 + the answer
+    std::atomic<int>& k = known[qgb_host::current_device()][r];
+    const int hit = k.load(std::memory_order_relaxed);
+    if (hit > 0) return hit - 1;
+    int n = 0;
+    if (r == 0) {
+        n = qgb_host::sm_count();
+    } else if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kClSmem) == cudaSuccess &&
+               cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1u << r);
+        cfg.blockDim = dim3(kClThreads);
+        cfg.dynamicSmemBytes = kClSmem;  // one CTA an SM
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = 1u << r;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) n = 0;
+    }
+    if (n <= 0) {
+        n = 0;
+        cudaGetLastError();  // a size that this device does not take is no error of the caller's
+    }
+    k.store(1 + n, std::memory_order_relaxed);
+    return n;
+}
+
+template <typename T, int KMAX>
+int launch_cluster(void* sv, const void* mats, const SweepArgs& a, cudaStream_t st) {
+    const int m = a.sw.low_bits + a.sw.n_high;
+    const uint64_t total = uint64_t(a.batch) * a.tiles;
+    // One wave: as many CTAs per tile as leave every cluster an SM per CTA (152 SMs hold 7, 15, 36 and
+    // 76 clusters of 16, 8, 4 and 2 CTAs; one too many costs a second wave: 17 qubits complex128,
+    // 16 tiles: 8 CTAs 1228 us, 4 CTAs 943 us), each with at least 128 amplitudes
+    // (9 qubits complex128: 128 of 4 CTAs 78 us, 256 of 2 CTAs 92 us).
+    if (total > uint64_t(cluster_room<T, KMAX>(0))) return qgb_host::QGB_EDECLINE;
+    int rbits = 0;
+    while (rbits < kClMaxRankBits && m - (rbits + 1) >= 7 && total <= uint64_t(cluster_room<T, KMAX>(rbits + 1))) ++rbits;
+    // float32 rows are cheap enough for one CTA to keep up on large parts (20-qubit sweeps of 13-bit
+    // tiles: 518 us with 2 CTAs a tile, 467 us with one CTA of sweep.cu; 12 bits alone 177 against
+    // 133 us, 11 bits 104 against 113 us); double-float rows are not (2 CTAs 1.8x faster)
+    if (sizeof(T) == 4 && rbits < 2 && m - rbits > 11) return qgb_host::QGB_EDECLINE;
+    const size_t smem = sizeof(typename ClAmp<T>::type) * ((size_t(2) << (m - rbits)) + kClMats);
+    if (smem > size_t(kClSmem)) return qgb_host::QGB_EDECLINE;  // the tile twice
+    auto kern = sweep_cluster_kernel<T, KMAX>;
+    static std::atomic<uint64_t> done{0};
     const int rc = qgb_host::allow_smem(kern, kClSmem, done, "cluster sweep attribute");
     if (rc) return rc;
-    const uint64_t bit = uint64_t(1) << qgb_host::current_device();
-    if (!(wide.load(std::memory_order_relaxed) & bit)) {  // (clusters of up to 8 do not need it)
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-            return qgb_host::check_launch("cluster sweep attribute");
-        wide.fetch_or(bit, std::memory_order_relaxed);
-    }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(unsigned((uint64_t(a.batch) * a.tiles) << rbits));
+    cfg.gridDim = dim3(unsigned(total << rbits));
     cfg.blockDim = dim3(kClThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -306,8 +348,11 @@ int launch_cluster(void* sv, const void* mats, const SweepArgs& a, int rbits, cu
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, kern, (cplx<T>*)sv, (const cplx<T>*)mats, a, rbits) != cudaSuccess)
-        return qgb_host::check_launch("cluster sweep");
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, (cplx<T>*)sv, (const cplx<T>*)mats, a, rbits);
+    if (e == cudaErrorInvalidClusterSize || e == cudaErrorLaunchOutOfResources) {  // nothing was launched
+        cudaGetLastError();
+        return qgb_host::QGB_EDECLINE;
+    }
     return qgb_host::check_launch("cluster sweep");
 }
 
@@ -316,33 +361,17 @@ int launch_cluster(void* sv, const void* mats, const SweepArgs& a, int rbits, cu
 namespace qgb_host {
 
 int launch_sweep_cluster(int dtype, void* sv, const void* mats, const SweepArgs& a, int kmax, cudaStream_t st) {
-    const int m = a.sw.low_bits + a.sw.n_high;
-    const uint64_t total = uint64_t(a.batch) * a.tiles;
-    if (total > 152) return QGB_EDECLINE;
-    // One wave: as many CTAs per tile as leave every cluster an SM per CTA (152 SMs in GPCs of at
-    // most 20 hold 7, 15, 36 and 76 clusters of 16, 8, 4 and 2 CTAs; one too many costs a second
-    // wave: 17 qubits complex128, 16 tiles: 8 CTAs 1228 us, 4 CTAs 943 us), each with at least 128
-    // amplitudes (9 qubits complex128: 128 of 4 CTAs 78 us, 256 of 2 CTAs 92 us).
-    static const int room[5] = {152, 76, 36, 15, 7};
-    int rbits = 0;
-    while (rbits < kClMaxRankBits && total <= uint64_t(room[rbits + 1]) && m - (rbits + 1) >= 7) ++rbits;
-    // float32 rows are cheap enough for one CTA to keep up on large parts (20-qubit sweeps of 13-bit
-    // tiles: 518 us with 2 CTAs a tile, 467 us with one CTA of sweep.cu; 12 bits alone 177 against
-    // 133 us, 11 bits 104 against 113 us); double-float rows are not (2 CTAs 1.8x faster)
-    if (dtype == QGB_C64 && rbits < 2 && m - rbits > 11) return QGB_EDECLINE;
-    const size_t amp = dtype == QGB_C64 ? sizeof(float2) : sizeof(dfc);
-    if (amp * ((size_t(2) << (m - rbits)) + kClMats) > size_t(kClSmem)) return QGB_EDECLINE;  // the tile twice
     if (dtype == QGB_C64) switch (kmax) {
         case 1:
-        case 2: return launch_cluster<float, 2>(sv, mats, a, rbits, st);
-        case 3: return launch_cluster<float, 3>(sv, mats, a, rbits, st);
-        case 4: return launch_cluster<float, 4>(sv, mats, a, rbits, st);
-        case 5: return launch_cluster<float, 5>(sv, mats, a, rbits, st);
+        case 2: return launch_cluster<float, 2>(sv, mats, a, st);
+        case 3: return launch_cluster<float, 3>(sv, mats, a, st);
+        case 4: return launch_cluster<float, 4>(sv, mats, a, st);
+        case 5: return launch_cluster<float, 5>(sv, mats, a, st);
     } else switch (kmax) {
         case 1:
-        case 2: return launch_cluster<double, 2>(sv, mats, a, rbits, st);
-        case 3: return launch_cluster<double, 3>(sv, mats, a, rbits, st);
-        case 4: return launch_cluster<double, 4>(sv, mats, a, rbits, st);
+        case 2: return launch_cluster<double, 2>(sv, mats, a, st);
+        case 3: return launch_cluster<double, 3>(sv, mats, a, st);
+        case 4: return launch_cluster<double, 4>(sv, mats, a, st);
     }
     return QGB_EDECLINE;
 }

@@ -395,8 +395,11 @@ class ParamGate(Gate):
         # While the matrix is still the one built from those angles the rebuild
         # would recompute the same values, so the copy shares it instead.
         if self.built_from_angles():
-            g = object.__new__(type(self))  # as copy.copy, without its dispatch (5 us a gate)
-            g.__dict__.update(self.__dict__)
+            if type(self) in _PLAIN_GATES:
+                g = object.__new__(type(self))  # as copy.copy, without its dispatch (5 us a gate)
+                g.__dict__.update(self.__dict__)
+            else:  # a class from elsewhere may have slots or its own way of being copied
+                g = copy.copy(self)
             g.indices = list(self.indices)
             return g
         return type(self)(self.indices, *self.angles)
@@ -532,6 +535,10 @@ class Givens(ParamGate):
 
     def solve_angles(self):
         return (np.arccos(self.matrix[1, 1]) * 2,)  # core/param_gates.py:185-187
+
+
+# the classes above: their instances are their __dict__ (ParamGate.shallow_copy)
+_PLAIN_GATES = frozenset({RX, RY, RZ, RXX, RYY, RZZ, XYCoupling, HeisenbergCoupling, CPhase, U, Givens})
 
 
 def kak_unitary(params):

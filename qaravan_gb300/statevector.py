@@ -110,10 +110,13 @@ class StatevectorSim:
         if mode == "auto":
             from . import autotune
             a_mode, a_width, a_tile = autotune.choose_sv(circ.num_sites, dtype)
-            # the fixed-point blocks are 5 qubits wide: another width asked for is a sweep's
-            mode = "sweep" if a_mode == "fixed" and fusion_width not in (None, a_width) else a_mode
+            mode = a_mode
             fusion_width = a_width if fusion_width is None else fusion_width
             tile_bits = a_tile if tile_bits is None else tile_bits
+        if mode == "fixed":
+            # the fixed-point blocks are 5 qubits wide: another width asked for is a sweep's
+            fusion_width = 5 if fusion_width is None else fusion_width
+            mode = "fixed" if fusion_width == 5 else "sweep"
         if fusion_width is None:
             if dtype == torch.complex64:
                 fusion_width = 6 if circ.num_sites >= 13 and _lib.lib().qgb_get_dense_impl() >= 1 else 4

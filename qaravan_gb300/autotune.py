@@ -139,6 +139,8 @@ def default_sweep(nbits, dtype):
 
 def choose_sv(n, dtype=torch.complex64):
     c = cached("sv", n, dtype)
+    if c is not None and c[0] == "fixed" and not fixed_point():
+        c = default_sv(n, dtype)  # (the entry holds no arithmetic: measured with the blocks, used without)
     if c is not None:
         return c
     if enabled():
@@ -191,6 +193,8 @@ def tune_sv(n, dtype=torch.complex64, depth=4, reps=3, measure=None):
 
         def measure(c):
             mode, width, tile = c
+            if mode == "fixed" and not fixed_point():
+                return None
             try:
                 ex = StatevectorSim(circ, dtype=dtype, mode=mode, fusion_width=width, tile_bits=tile).compile()
             except Exception:

@@ -115,8 +115,12 @@ class StatevectorSim:
             tile_bits = a_tile if tile_bits is None else tile_bits
         if mode == "fixed":
             # the fixed-point blocks are 5 qubits wide: another width asked for is a sweep's
+            from . import autotune
             fusion_width = 5 if fusion_width is None else fusion_width
-            mode = "fixed" if fusion_width == 5 else "sweep"
+            if fusion_width != 5:
+                mode = "sweep"
+            elif not autotune.fixed_point():  # switched off: 5-qubit float64 blocks would run in their place
+                mode, fusion_width = "sweep", 3
         if fusion_width is None:
             if dtype == torch.complex64:
                 fusion_width = 6 if circ.num_sites >= 13 and _lib.lib().qgb_get_dense_impl() >= 1 else 4

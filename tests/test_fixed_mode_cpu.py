@@ -24,3 +24,20 @@ def _sim(n=17, **kw):
 def test_width_asked_for(width, want):
     assert _sim(mode="fixed", fusion_width=width) == want
     assert _sim(fusion_width=width) == want
+
+
+@pytest.mark.parametrize("switch", ["arithmetic", "tensor cores"])
+def test_blocks_switched_off(switch):
+    """A remembered choice, the default and the mode by name: sweeps, not 5-qubit float64 blocks."""
+    L = _lib.lib()
+    autotune.store("sv", 17, torch.complex128, ("fixed", 5, 13), [])
+    assert _sim() == ("fixed", 5)
+    impl = L.qgb_get_dense_impl()
+    _lib.check(L.qgb_set_c128_arith(0) if switch == "arithmetic" else L.qgb_set_dense_impl(0))
+    try:
+        assert autotune.choose_sv(17, torch.complex128) == ("sweep", 3, 13)
+        assert _sim() == _sim(mode="fixed") == _sim(18) == ("sweep", 3)
+    finally:
+        _lib.check(L.qgb_set_c128_arith(1))
+        _lib.check(L.qgb_set_dense_impl(impl))
+    assert _sim() == ("fixed", 5)

@@ -216,8 +216,9 @@ def fma_peaks():
 
 
 def c128_roofline(plan, n, ms, double_float, peaks):
-    """Roofline of a complex128 plan: dense passes (5-qubit blocks in fixed point on
-    the tensor cores) against the HBM copy rate; sweeps with float64 kernels against the measured
+    """Roofline of a complex128 plan: 5-qubit blocks in fixed point on the tensor cores are
+    bound by the integer instructions that split and reassemble numbers, so their share of the HBM
+    copy rate is information; sweeps with float64 kernels against the measured
     FP64 FMA rate (8 flops per complex multiply-add); double-float kernels
     against the measured FP32 rate, counting the FP32 pipe's work -- one
     double-float complex multiply-add is 4 real terms of 1 multiply, 3 FMAs and
@@ -226,12 +227,12 @@ def c128_roofline(plan, n, ms, double_float, peaks):
     from qaravan_gb300.compiler import plan_flops
     flops64 = plan_flops(plan)[1] * 2 ** n  # 8 per complex multiply-add
     out = {"tflops_fp64_equivalent": round(flops64 / (ms / 1e3) / 1e12, 3)}
-    if plan.steps and all(type(s).__name__ == "DenseStep" and len(s.bits) == 5 for s in plan.steps):
+    if double_float and plan.steps and all(getattr(s, "fixed", False) for s in plan.steps):
         peak, kind = _peaks()
         achieved = 2 * 16 * 2 ** n * len(plan.steps) / (ms / 1e3) / 1e9
-        out["arithmetic"] = "fixed point, 9-bit digits on the tensor cores"
-        out["roofline"] = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-                           "frac": round(achieved / peak, 3), "peak_source": f"hbm_gbs of {kind}"}
+        out["arithmetic"] = "fixed point, 9-bit digits on the tensor cores; double-float where that is less accurate"
+        out["roofline"] = {"bound": "integer instructions", "hbm_gbs": round(achieved, 1), "hbm_peak": peak,
+                           "hbm_frac": round(achieved / peak, 3), "peak_source": f"hbm_gbs of {kind}"}
     elif double_float:
         achieved = 2 * 48 * (flops64 / 8) / (ms / 1e3) / 1e12
         out["roofline"] = {"bound": "fp32", "achieved": round(achieved, 2), "peak": peaks["fp32_tflops"],
@@ -247,11 +248,10 @@ def c128_roofline(plan, n, ms, double_float, peaks):
 
 
 def section_c128(n, gates, steps=3):
-    """The benchmark circuit in complex128 through StatevectorSim's default
-    complex128 path (fixed-point blocks on the tensor cores, under the key
-    "double_float" of the arithmetic setting that selects it; double-float tile
-    sweeps below 17 qubits), timed over `steps` runs after a
-    warm-up, with its roofline; its final state against the float64 kernels'."""
+    """The benchmark circuit in complex128 through StatevectorSim: its default path
+    ("default": fixed-point blocks on the tensor cores, tile sweeps below 17 qubits), double-float
+    tile sweeps ("double_float") and the float64 kernels ("float64"), timed over `steps`
+    runs after a warm-up, each with its roofline; final states against the float64 kernels'."""
     import torch
     from qaravan_gb300 import StatevectorSim, _lib
     from qaravan_gb300.circuits import Circuit
@@ -260,9 +260,10 @@ def section_c128(n, gates, steps=3):
     code = _lib.dtype_code(torch.complex128)
     out = {}
     states = {}
-    for arith, name in ((1, "double_float"), (0, "float64")):
+    sweeps = {"mode": "sweep", "fusion_width": 3, "tile_bits": 13}
+    for arith, name, kw in ((1, "default", {}), (1, "double_float", sweeps), (0, "float64", sweeps)):
         _lib.check(L.qgb_set_c128_arith(arith))
-        ex = StatevectorSim(circ, dtype=torch.complex128).compile()
+        ex = StatevectorSim(circ, dtype=torch.complex128, **kw).compile()
         st = torch.empty(2 ** n, dtype=torch.complex128, device="cuda")
 
         def step():
@@ -275,12 +276,14 @@ def section_c128(n, gates, steps=3):
         states[name] = st
         del ex
     _lib.check(L.qgb_set_c128_arith(1))
-    d = (states["double_float"] - states["float64"]).abs()
-    out["max_abs_amplitude_diff_double_float_vs_float64"] = float(d.max().item())
     out["max_abs_amplitude"] = float(states["float64"].abs().max().item())
-    out["norm_error_double_float"] = float(abs(torch.linalg.vector_norm(states["double_float"]).item() - 1.0))
-    out["speedup_double_float_vs_float64"] = round(out["float64"]["ms"] / out["double_float"]["ms"], 2)
-    del states, d
+    for name in ("default", "double_float"):
+        d = (states[name] - states["float64"]).abs()
+        out[f"max_abs_amplitude_diff_{name}_vs_float64"] = float(d.max().item())
+        out[f"norm_error_{name}"] = float(abs(torch.linalg.vector_norm(states[name]).item() - 1.0))
+        out[f"speedup_{name}_vs_float64"] = round(out["float64"]["ms"] / out[name]["ms"], 2)
+        del d
+    del states
     torch.cuda.empty_cache()
     return out
 

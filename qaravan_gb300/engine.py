@@ -35,10 +35,13 @@ _NORM_RESTORE = _NORM_MODES.get(os.environ.get("QGB_NORM_RESTORE", "chain"), "ch
 
 # Complex64 density matrices on the tensor cores keep their trace by a trace
 # chain: the trace is measured (qgb_dm_trace_factor) where the ops applied so
-# far are whole channels, at most every _TRACE_EPOCH tensor-core passes, and the
+# far are whole channels, every _TRACE_EPOCH or more tensor-core passes, and the
 # next tensor-core pass multiplies its matrix by reference / measured trace
-# (qgb_op_action_scaled). QGB_TRACE_CHAIN=0 or set_trace_chain(False) turns it off.
-_TRACE_EPOCH = 4
+# (qgb_op_action_scaled). The last measurement is _TRACE_TAIL passes before the end where the
+# plan allows: small entries lose more than large ones, so a state whose trace has just
+# been restored is too large in norm (13 sites, depth 10: 1 pass behind, trace short by 0.6e-7, norm
+# 4.2e-7 too large; 4 passes, 4.5e-7 and 1.4e-7). QGB_TRACE_CHAIN=0 or set_trace_chain(False) turns it off.
+_TRACE_EPOCH, _TRACE_TAIL = 4, 2
 _TRACE_CHAIN = os.environ.get("QGB_TRACE_CHAIN", "1") not in ("0", "off")
 
 
@@ -46,6 +49,34 @@ def set_trace_chain(on=True):
     """Process-wide trace chain of complex64 density matrices (default on)."""
     global _TRACE_CHAIN
     _TRACE_CHAIN = bool(on)
+
+
+def trace_cuts(steps):
+    """Where the trace chain measures: steps after which the ops applied are whole
+    channels, each at least ``_TRACE_EPOCH`` tensor-core passes after the one before,
+    and the first so much later that, in every stretch between renormalisations,
+    ``_TRACE_TAIL`` passes follow the last. ``steps``: the executor's (kind, .., whole, on
+    tensor cores)."""
+    cuts, begin = set(), 0
+    for end in [i for i, s in enumerate(steps) if s[0] == "normalize"] + [len(steps)]:
+        passes = [(i, s[5], int(s[6])) for i, s in enumerate(steps[begin:end], begin) if s[0] == "dense"]
+        best = None
+        for lead in range(_TRACE_EPOCH, 2 * _TRACE_EPOCH):
+            got, since, need = [], 0, lead
+            for i, whole, tc in passes:
+                since += tc
+                if whole and since >= need:
+                    got.append(i)
+                    since, need = 0, _TRACE_EPOCH
+            if got and since == 0:  # nothing behind it takes the factor
+                got.pop()
+                since = _TRACE_EPOCH
+            off = abs(since - _TRACE_TAIL) if got else len(passes)
+            if best is None or off < best[0]:
+                best = (off, got)
+        cuts.update(best[1])
+        begin = end + 1
+    return cuts
 
 
 def tc_eligible(code, nbits, k, batch=1):
@@ -162,6 +193,7 @@ class Executor:
                     raise NotImplementedError("Pauli channels of more than 128 terms")
                 strings = "".join(t[1].lower() for t in s.terms).encode()
                 self._steps.append(("pauli_mix", strings, _lib.double_array([t[0] for t in s.terms]), len(s.terms)))
+        self._cuts = trace_cuts(self._steps)
         self._calls: dict = {}  # (norm mode, trace chain) -> the plan's launches for qgb_run_calls
         self.scratch = Scratch(self.device)
         self.norm = torch.empty(1, dtype=torch.float64, device=self.device)
@@ -264,8 +296,8 @@ class Executor:
             tptr = self._tchain.data_ptr()
             _lib.check(L.qgb_dm_trace_factor(ptr, self.code, nb // 2, tptr, 1, st), "dm_trace_factor")
             launches += 1
-            t_since, t_pending = 0, False  # tensor-core passes since the last measurement; a factor waits
-        for s in self._steps:
+            t_pending = False  # a factor waits
+        for i, s in enumerate(self._steps):
             if events is not None and s[0] != "normalize":
                 e0 = torch.cuda.Event(enable_timing=True)
                 e0.record()
@@ -279,11 +311,10 @@ class Executor:
                     _lib.check(L.qgb_op_action(ptr, self.code, nb, sites, k, mptr + off * self.itemsize, 0, 1, 0,
                                                st), "op_action")
                 launches += 1
-                t_since += int(on_tc)
-                if whole and t_since >= _TRACE_EPOCH:
+                if i in self._cuts:
                     _lib.check(L.qgb_dm_trace_factor(ptr, self.code, nb // 2, tptr, 0, st), "dm_trace_factor")
                     launches += 1
-                    t_since, t_pending = 0, True
+                    t_pending = True
             elif s[0] == "dense":
                 _, sites, k, off, unitary = s[:5]
                 # per-vector matrices (mat_stride) need not be unitary: only the plan's own are flagged
@@ -344,7 +375,7 @@ class Executor:
                 if tchain:  # the trace is 1 again: a new reference
                     _lib.check(L.qgb_dm_trace_factor(ptr, self.code, nb // 2, tptr, 1, st), "dm_trace_factor")
                     launches += 1
-                    t_since, t_pending = 0, False
+                    t_pending = False
             if events is not None and s[0] != "normalize":
                 e1 = torch.cuda.Event(enable_timing=True)
                 e1.record()
@@ -364,11 +395,11 @@ class Executor:
         chain knows its length here: its first epoch is cut so that the chain's last
         pass opens an epoch and corrects the drift of every pass but its own, and
         unitary blocks on the CUDA cores, which do not drift, leave it running."""
-        calls, chains, t_since, t_pending = [], [[]], 0, False
+        calls, chains, t_pending = [], [[]], False
         none = (0,) * _lib.QGB_MAX_K
         if tchain:
             calls.append((_lib.QGB_CALL_TRACE, none, 0, 1, 0, None))
-        for s in self._steps:
+        for i, s in enumerate(self._steps):
             if s[0] == "sweep":
                 calls.append((_lib.QGB_CALL_SWEEP, none, 0, 0, 0, s[1]))
                 chains.append([])
@@ -380,10 +411,9 @@ class Executor:
                 scaled = on_tc and t_pending
                 calls.append((_lib.QGB_CALL_SCALED if scaled else _lib.QGB_CALL_OP, sites, k, 0, off, None))
                 t_pending = t_pending and not scaled
-                t_since += int(on_tc)
-                if whole and t_since >= _TRACE_EPOCH:
+                if i in self._cuts:
                     calls.append((_lib.QGB_CALL_TRACE, none, 0, 0, 0, None))
-                    t_since, t_pending = 0, True
+                    t_pending = True
             elif unitary and mode == "chain" and on_tc:
                 chains[-1].append(len(calls))
                 calls.append((_lib.QGB_CALL_CHAIN, sites, k, len(chains[-1]) - 1, off, None))

@@ -239,7 +239,7 @@ typedef struct {
     int32_t k;                  /* op calls: width                                */
     int32_t sites[QGB_MAX_K];   /* op calls: sites, as qgb_op_action's indices    */
     int32_t link;
-    int32_t first;              /* chain calls: passes of the chain's first epoch (0: 4), so
+    int32_t first;              /* chain calls: passes of the chain's first epoch (0: qgb_chain_epoch()), so
                                    that a caller who knows the chain's length can let its last
                                    pass open an epoch and correct the norm once more         */
     int64_t mat;                /* op calls: element offset of the matrix in mats */
@@ -258,7 +258,7 @@ typedef struct {
 int qgb_run_calls(void* sv, int dtype, int n, const qgb_call* calls, int ncalls, const void* mats, double* chain,
                   double* trace, void* stream);
 size_t qgb_call_bytes(void);
-
+int qgb_chain_epoch(void); /* passes of a norm chain's epoch */
 
 /* A fused pass (several gates per read+write of the state), planned by the
  * host compiler from a Circuit's gate list (core/base_sim.py:30-53 loop). */

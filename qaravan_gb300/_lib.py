@@ -101,6 +101,7 @@ SIGNATURES = {
     "qgb_op_action_scaled": (C.c_int, [_vp, _i, _i, _ip, _i, _vp, _vp, _vp]),
     "qgb_run_calls": (C.c_int, [_vp, _i, _i, C.POINTER(Call), _i, _vp, _vp, _vp, _vp]),
     "qgb_call_bytes": (C.c_size_t, []),
+    "qgb_chain_epoch": (C.c_int, []),
     "qgb_plan_blocks": (C.c_int, [_i, _vp, _vp, _i, _i, _vp, _vp, _vp, _vp]),
     "qgb_dm_trace_factor": (C.c_int, [_vp, _i, _i, _vp, _i, _vp]),
     "qgb_apply_sweep": (C.c_int, [_vp, _i, _i, C.POINTER(Sweep), _vp, _i64, _i64, _i64, _vp]),

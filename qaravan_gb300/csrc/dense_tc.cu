@@ -793,6 +793,8 @@ int try_dense_tc(void* sv, const void* op, int nbits, const int* sorted, const i
 
 }  // namespace qgb_host
 
+extern "C" int qgb_chain_epoch(void) { return kChainEpoch; }
+
 extern "C" int qgb_set_dense_impl(int mode) { return qgb_host::set_dense_impl(mode); }
 
 extern "C" int qgb_get_dense_impl(void) { return dense_impl(); }

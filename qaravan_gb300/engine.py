@@ -29,7 +29,6 @@ from .compiler import DenseStep, NormalizeStep, PauliMixStep, Plan, Recipe, Swee
 # pass (qgb_op_action_unitary; also what batches use under "chain"), ~10 % of the
 # kernel's speed. "off": neither. QGB_NORM_RESTORE=chain|row|0 or set_norm_restore().
 _NORM_MODES = {"1": "chain", "chain": "chain", "row": "row", "0": "off", "off": "off"}
-_CHAIN_EPOCH = 4  # passes per epoch of the norm chain (the library's)
 _NORM_RESTORE = _NORM_MODES.get(os.environ.get("QGB_NORM_RESTORE", "chain"), "chain")
 
 
@@ -424,9 +423,10 @@ class Executor:
                 if not unitary:
                     chains.append([])
         first = [0] * len(calls)
-        for chain in chains:
+        for chain in filter(None, chains):
+            lead = (len(chain) - 1) % _lib.lib().qgb_chain_epoch()
             for i in chain:
-                first[i] = (len(chain) - 1) % _CHAIN_EPOCH
+                first[i] = lead
         arr = np.array([(kind, k, sites, link, f, off, 0 if sweep is None else C.addressof(sweep))
                         for (kind, sites, k, link, off, sweep), f in zip(calls, first)], dtype=_CALL)
         return arr, arr.ctypes.data_as(C.POINTER(_lib.Call)), len(calls), any(chains)

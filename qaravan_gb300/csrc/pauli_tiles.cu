@@ -569,23 +569,28 @@ Plan make_plan(int n, const PauliTerm* terms, int nterms, uint64_t stride, bool 
     const int L = n <= kPtM ? m : kPtLow;
     const int H = m - L;
     const uint64_t low = (uint64_t(1) << L) - 1;
+    for (int t = 0; t < nterms; ++t)
+        if (__builtin_popcountll(terms[t].x & ~low) > H) return plan;  // an X mask wider than a tile
     std::vector<int> left(nterms);
     for (int t = 0; t < nterms; ++t) left[t] = t;
     // masks in ascending order of their top bit, so that neighbouring bits share a pass
     std::stable_sort(left.begin(), left.end(), [&](int p, int q) { return terms[p].x < terms[q].x; });
-    while (!left.empty()) {
+    // (a full pass stops looking: what it passed over goes in front of the rest)
+    for (size_t at = 0; at < left.size();) {
         uint64_t high = 0;
-        std::vector<int> taken, rest;
-        for (int t : left) {
-            const uint64_t need = high | (terms[t].x & ~low);
-            if (int(taken.size()) < kPtMaxTerms && __builtin_popcountll(need) <= H) {
+        std::vector<int> taken, over;
+        size_t i = at;
+        for (; i < left.size() && int(taken.size()) < kPtMaxTerms; ++i) {
+            const uint64_t need = high | (terms[left[i]].x & ~low);
+            if (__builtin_popcountll(need) <= H) {
                 high = need;
-                taken.push_back(t);
+                taken.push_back(left[i]);
             } else {
-                rest.push_back(t);
+                over.push_back(left[i]);
             }
         }
-        if (taken.empty()) return Plan{};  // an X mask wider than a tile
+        at = i - over.size();
+        std::copy(over.begin(), over.end(), left.begin() + int64_t(at));
         for (int b = L; b < n && __builtin_popcountll(high) < H; ++b) high |= uint64_t(1) << b;
         plan.passes.emplace_back();
         PtArgs& a = plan.passes.back();
@@ -608,7 +613,6 @@ Plan make_plan(int n, const PauliTerm* terms, int nterms, uint64_t stride, bool 
             }
         }
         if (!build_pass(a, taken, terms, expect)) return Plan{};
-        left = rest;
     }
     return plan;
 }

@@ -21,7 +21,8 @@
 // each per 16 amplitudes.
 //
 // Measured (Ising terms, one state): 25 qubits 9.82 -> 7.12 ms, 17 qubits 230 ->
-// 129 us, 8 qubits 50 -> 35 us against one pass per X mask.
+// 129 us, 8 qubits 50 -> 35 us against one pass per X mask. Where the general
+// kernels (reduce.cu) are the faster ones, see expect_pays and apply_pays.
 //
 // What bounds it: the FP64 pipe (two multiply-adds per pair and term, four adds
 // per amplitude for the diagonal). All sums run in a fixed order, so results are
@@ -668,15 +669,39 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) % 16) == 
 // complex128 only: the complex64 kernels (reduce.cu) add float32 products in an
 // order that fixes every bit of their float64 results, which callers compare
 // between runs and builds; complex128 results move at the 1e-16 level only.
-// From 5 bits up (two threads of 16 amplitudes): 35 us against 50 us of one
-// launch per mask at 8 qubits, 7.1 against 9.8 ms at 25.
+// From 5 bits up (two threads of 16 amplitudes).
 bool eligible(const void* sv, int dtype, int n) { return dtype == QGB_C128 && n >= 5 && aligned16(sv); }
+
+// Expectation values. Up to 11 bits one tile takes a pass of at most 44 terms, 57 us whatever its masks; the
+// general kernel takes a launch for every run of up to 32 terms on one mask, 6 to 28 us at 8 bits. So at
+// 9 bits and below sums of many terms a mask stay there (us, tiles / general: 8 bits, 1 term a mask 59 / 71, 4
+// 123 / 105, 8 184 / 152, 32 331 / 219; 9 bits, 16 341 / 435, 32 333 / 271; 10 bits, 32 345 / 382; 14 bits,
+// 1 110 / 162, 32 600 / 1071).
+bool expect_pays(int n, const PauliTerm* terms, int nterms) {
+    if (n > 9) return true;
+    int runs = 0;
+    for (int t = 0, k = 0; t < nterms; ++t, ++k)
+        if (t == 0 || terms[t].x != terms[t - 1].x || k == 32) {
+            ++runs;
+            k = 0;
+        }
+    return n < 9 ? nterms < 4 * runs : nterms < 24 * runs;
+}
+
+// Applied sums. The general kernel is one launch that reads the state once a term, through the caches: a state
+// in L1 or L2 costs it little, and it reads and writes `out` once. Tiles pay from 20 bits, and
+// where all terms are diagonal, one pass for 44 of them, from 16 (us, tiles / general: Ising terms 12 bits 48 / 11,
+// 17 bits 60 / 33, 20 bits 231 / 238, 22 bits 817 / 1010; 128 diagonal terms 14 bits 44 / 41, 17 bits
+// 44 / 115, 20 bits 101 / 788; 128 dense terms 12 bits 376 / 48).
+bool apply_pays(int n, const PauliTerm* terms, int nterms) {
+    return n >= 20 || (n >= 16 && std::all_of(terms, terms + nterms, [](const PauliTerm& t) { return t.x == 0; }));
+}
 
 }  // namespace
 
 int pauli_tiles_expect(const void* sv, int dtype, int n, const PauliTerm* terms, int nterms, int64_t batch,
                        int64_t stride, int max_blocks, double* partials, int* nblk, cudaStream_t st) {
-    if (!eligible(sv, dtype, n)) return QGB_EDECLINE;
+    if (!eligible(sv, dtype, n) || !expect_pays(n, terms, nterms)) return QGB_EDECLINE;
     try {
         return expect_impl(sv, n, terms, nterms, batch, stride, max_blocks, partials, nblk, st);
     } catch (const std::exception&) {  // no memory for the plan: nothing has been launched
@@ -686,7 +711,7 @@ int pauli_tiles_expect(const void* sv, int dtype, int n, const PauliTerm* terms,
 
 int pauli_tiles_apply(const void* sv, void* out, int dtype, int n, const PauliTerm* terms, int nterms, int64_t batch,
                       int64_t stride, cudaStream_t st) {
-    if (!eligible(sv, dtype, n) || !aligned16(out)) return QGB_EDECLINE;
+    if (!eligible(sv, dtype, n) || !aligned16(out) || !apply_pays(n, terms, nterms)) return QGB_EDECLINE;
     try {
         return apply_impl(sv, out, n, terms, nterms, batch, stride, st);
     } catch (const std::exception&) {

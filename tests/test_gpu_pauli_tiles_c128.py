@@ -69,3 +69,36 @@ def test_many_passes(n, count, wide):
     many = pauli_expectations(psi, n, terms).cpu().numpy()
     single = np.array([pauli_expectations(psi, n, [t]).cpu().numpy()[0] for t in terms])
     assert np.max(np.abs(many - single)) < 1e-13
+
+
+def _times(psi, n, s):
+    """P psi for a Pauli string, site 0 most significant."""
+    idx = np.arange(2 ** n)
+    src = idx ^ sum(1 << (n - 1 - q) for q, c in enumerate(s) if c in "xy")
+    out = psi[src]
+    for q, c in enumerate(s):
+        b = (src >> (n - 1 - q)) & 1
+        if c == "z":
+            out = out * (1 - 2 * b)
+        elif c == "y":  # Y|0> = i|1>, Y|1> = -i|0>
+            out = out * np.where(b == 0, 1j, -1j)
+    return out
+
+
+@pytest.mark.parametrize("n,kind", [(15, "diagonal"), (16, "diagonal"), (17, "diagonal"), (19, "chain"), (20, "chain"),
+                                    (21, "chain"), (20, "one")])
+def test_applied_on_both_sides_of_the_rule(n, kind):
+    """The tile form from 20 qubits (16 for diagonal sums), in several passes that add to `out`, and the
+    general kernel below: at most two roundings a term and amplitude, 2^-53 each, in either."""
+    rng = np.random.default_rng(n)
+    if kind == "diagonal":
+        terms = [(float(rng.uniform(-1, 1)), "".join(rng.choice(list("iz"), n))) for _ in range(100)]
+    elif kind == "one":
+        terms = [(0.7, "i" * (n - 3) + "yxz")]
+    else:
+        terms = [(float(rng.uniform(-1, 1)), "i" * q + p + "i" * (n - q - len(p))) for p in ("z", "yy", "xz")
+                 for q in range(0, n - len(p) + 1, 2)]
+    v = rng.standard_normal(2 ** n) + 1j * rng.standard_normal(2 ** n)
+    want = sum(c * _times(v, n, s) for c, s in terms)
+    got = _apply(torch.from_numpy(v).cuda(), n, terms)
+    assert np.max(np.abs(got - want)) < 4 * len(terms) * 2.0 ** -53 * np.max(np.abs(v))

@@ -330,6 +330,9 @@ int launch_cluster(void* sv, const void* mats, const SweepArgs& a, cudaStream_t 
     // tiles: 518 us with 2 CTAs a tile, 467 us with one CTA of sweep.cu; 12 bits alone 177 against
     // 133 us, 11 bits 104 against 113 us); double-float rows are not (2 CTAs 1.8x faster)
     if (sizeof(T) == 4 && rbits < 2 && m - rbits > 11) return qgb_host::QGB_EDECLINE;
+    // and so are ops of at most two qubits on small tiles (here / one CTA of sweep.cu: 4 bits 13 / 10 us, 8 bits
+    // 25 / 18, 10 bits 35 / 30, 11 bits 40 / 41, 12 bits 51 / 66; of three qubits 8 bits 17 / 25)
+    if (sizeof(T) == 4 && KMAX <= 2 && m <= 10) return qgb_host::QGB_EDECLINE;
     const size_t smem = sizeof(typename ClAmp<T>::type) * ((size_t(2) << (m - rbits)) + kClMats);
     if (smem > size_t(kClSmem)) return qgb_host::QGB_EDECLINE;  // the tile twice
     auto kern = sweep_cluster_kernel<T, KMAX>;

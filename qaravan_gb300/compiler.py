@@ -377,6 +377,23 @@ def _spreads(seg, nbits):
     return sum(spreading([np.asarray(o.matrix) for o in seg])) >= share * sum(len(o.bits) for o in seg)
 
 
+# A fixed-point pass costs the same whatever its block holds, and more where the block is narrower than 5
+# bits (outputs drawn from few amplitudes); a tile sweep's op costs by its rows. A segment takes the passes
+# when its 3-bit blocks have at least this many rows in all for each of its 5-bit blocks, the narrower ones
+# counted twice: up to 18 bits, 19 bits, more. Milliseconds against sweeps from a random state: 25 qubits, one
+# pair gate (2 rows a block) 0.96 / 0.60, 30 pairs (4.6) 5.5 / 4.5, pair layers 1 (2) 11.7 / 3.9, 2 (16) 3.4 / 6.4,
+# 3 (7) 7.1 / 9.2, 6 (14) 10.1 / 18.6; 20 qubits, 3 layers (6.2) 0.28 / 0.29, 2 layers (15) 0.14 / 0.19; 19 qubits,
+# 3 layers (7.2) 0.16 / 0.15, 2 layers (12) 0.10 / 0.11; 18 qubits, 3 layers (6.3) 0.14 / 0.09, 2 layers (11.3)
+# 0.09 / 0.06, 4 (15) 0.12 / 0.11, 6 (14) 0.17 / 0.17; 17 qubits, 2 layers (16) 0.06 / 0.06, 3 (7.4) 0.12 / 0.08.
+_FIXED_ROWS = (11.0, 9.0, 6.0)
+
+
+def _rows_pay(fixed, sweep, nbits):
+    rows = sum(2 ** len(b.bits) for b in sweep)
+    passes = sum(1 if len(b.bits) >= 5 else 2 for b in fixed)
+    return rows >= _FIXED_ROWS[0 if nbits <= _FIXED_SMALL else 1 if nbits == _FIXED_SMALL + 1 else 2] * passes
+
+
 def trace_preserving(op):
     """Whether an op on vec(rho) keeps Tr rho for every rho: a half of a unitary
     gate (unitary on its bits; the other half is its conjugate) or a channel
@@ -473,7 +490,8 @@ def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, 
     ``"fixed"`` (complex128, at least 12 bits, device fusion): such blocks of 5 bits, narrower ones
     widened with the identity on the lowest free bits, marked for the fixed-point kernel; it takes
     unitary blocks, so a segment with another op or a wider one runs as 3-bit blocks in tile sweeps,
-    and so does one whose ops spread amplitudes too little for it (``_FIXED_SPREAD``).
+    and so does one whose ops spread amplitudes too little for it (``_FIXED_SPREAD``) or are too few for its
+    passes (``_FIXED_ROWS``).
     """
     tile_bits = min(tile_bits, 14 if itemsize <= 8 else 13)
     pad = 0
@@ -555,6 +573,10 @@ def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, 
             base = len(plan.op_matrices)
             plan.op_matrices.extend(np.ascontiguousarray(o.matrix, dtype=np.complex128) for o in seg)
             sym = (fuse_fewest if pack and mode == "fused" and (padded or not pad) else fuse_symbolic)(seg, w)
+            if padded:
+                narrow = fuse_symbolic(seg, max(3, widest))
+                if not _rows_pay(sym, narrow, nbits):
+                    padded, w, sym = False, max(3, widest), narrow
             if padded:
                 for b in sym:
                     if len(b.bits) < pad:

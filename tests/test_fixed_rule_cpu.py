@@ -44,6 +44,24 @@ def test_routes(n, make, kind):
         assert all(s.fixed and len(s.bits) == 5 for s in plan.steps)
 
 
+def _pairs(n, layers):
+    rng = np.random.default_rng(7)
+    return Circuit([Gate("u", [q, q + 1], workloads.haar_unitary(4, rng)) for j in range(layers)
+                    for q in range(j % 2, n - 1, 2)], n=n)
+
+
+@pytest.mark.parametrize("n,layers,kind", [(17, 1, SweepStep), (17, 2, DenseStep), (17, 3, SweepStep), (18, 3, SweepStep),
+                                           (18, 6, DenseStep), (19, 2, DenseStep), (20, 1, SweepStep),
+                                           (20, 2, DenseStep), (25, 1, SweepStep), (25, 3, DenseStep)])
+def test_too_few_ops_for_the_passes(n, layers, kind):
+    assert all(type(s) is kind for s in _plan(_pairs(n, layers), n).steps)
+
+
+def test_one_gate():
+    g = Circuit([Gate("u", [3, 4], workloads.haar_unitary(4, np.random.default_rng(0)))], n=20)
+    assert [type(s) for s in _plan(g, 20).steps] == [SweepStep]
+
+
 def test_segments_are_judged_by_themselves():
     """A reset cuts the circuit: Haar gates on one side, phases on the other."""
     n, rng = 17, np.random.default_rng(2)

@@ -327,15 +327,18 @@ def plan_sweeps(blocks, nbits, tile_bits, low_bits=None, max_high=QGB_SWEEP_MAX_
 
 # ------------------------------------------------------------------- plans
 
-def unitary_flags(ops, tol=1e-6):
-    """Whether each op's matrix is unitary (max |M^H M - I| < tol), batched by size."""
-    flags = [False] * len(ops)
+def _stacks(mats):
+    """The matrices by size: ``[(indices, complex128 stack)]``."""
     by_dim: dict = {}
-    for i, o in enumerate(ops):
-        m = np.asarray(o.matrix)
+    for i, m in enumerate(mats):
         by_dim.setdefault(m.shape[0], []).append(i)
-    for d, idx in by_dim.items():
-        m = np.stack([np.asarray(ops[i].matrix, dtype=np.complex128) for i in idx])
+    return [(idx, np.stack([np.asarray(mats[i], dtype=np.complex128) for i in idx])) for idx in by_dim.values()]
+
+
+def _unitary_of(stacks, count, tol):
+    flags = [False] * count
+    for idx, m in stacks:
+        d = m.shape[-1]
         gram = np.matmul(m.conj().transpose(0, 2, 1), m)
         gram[:, np.arange(d), np.arange(d)] -= 1
         err = np.abs(gram).reshape(len(idx), -1).max(axis=1)
@@ -344,20 +347,25 @@ def unitary_flags(ops, tol=1e-6):
     return flags
 
 
-def spreading(mats, tol=2 ** 0.5 / 8):
+def unitary_flags(ops, tol=1e-6):
+    """Whether each op's matrix is unitary (max |M^H M - I| < tol), batched by size."""
+    return _unitary_of(_stacks([np.asarray(o.matrix) for o in ops]), len(ops), tol)
+
+
+def _spread_of(stacks, count):
+    out = [0.0] * count
+    for idx, m in stacks:
+        big = (np.abs(m.real) + np.abs(m.imag) >= 2 ** 0.5 / 8).reshape(len(idx), -1).sum(axis=1)
+        for i, s in zip(idx, np.log2(np.maximum(big / m.shape[-1], 1.0)).tolist()):
+            out[i] = s
+    return out
+
+
+def spreading(mats):
     """log2 of how many rows a column of each matrix reaches on average, counting the
     entries of at least 1/8: 1 for a one-site gate that mixes its two states, 0 for a
     phase, a permutation or a rotation by a small angle, 2 for a Haar pair gate."""
-    out = [0.0] * len(mats)
-    by_dim: dict = {}
-    for i, m in enumerate(mats):
-        by_dim.setdefault(m.shape[0], []).append(i)
-    for d, idx in by_dim.items():
-        m = np.stack([np.asarray(mats[i]) for i in idx])
-        big = (np.abs(m.real) + np.abs(m.imag) >= tol).reshape(len(idx), -1).sum(axis=1)
-        for i, s in zip(idx, np.log2(np.maximum(big / d, 1.0)).tolist()):
-            out[i] = s
-    return out
+    return _spread_of(_stacks([np.asarray(m) for m in mats]), len(mats))
 
 
 # The fixed-point kernel keeps a group's 32 amplitudes relative to the largest and computes an output
@@ -372,9 +380,9 @@ def spreading(mats, tol=2 ** 0.5 / 8):
 _FIXED_SPREAD, _FIXED_SPREAD_SMALL, _FIXED_SMALL = 0.15, 0.75, 18
 
 
-def _spreads(seg, nbits):
+def _spreads(seg, spread, nbits):
     share = _FIXED_SPREAD_SMALL if nbits <= _FIXED_SMALL else _FIXED_SPREAD
-    return sum(spreading([np.asarray(o.matrix) for o in seg])) >= share * sum(len(o.bits) for o in seg)
+    return sum(spread[id(o)] for o in seg) >= share * sum(len(o.bits) for o in seg)
 
 
 # A fixed-point pass costs the same whatever its block holds, and more where the block is narrower than 5
@@ -501,7 +509,9 @@ def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, 
         mode, width = "sweep", 3
     # unitarity of every op with a matrix, batched once (the plan key, trace checks and fusion use it)
     mops = [o for o in ops if o is not None and o.kind != "pauli_mix"]
-    ucache = dict(zip(map(id, mops), unitary_flags(mops))) if mops else {}
+    stacks = _stacks([np.asarray(o.matrix) for o in mops])
+    ucache = dict(zip(map(id, mops), _unitary_of(stacks, len(mops), 1e-6)))
+    spread = dict(zip(map(id, mops), _spread_of(stacks, len(mops)))) if pad else {}
     # density matrices: does every op keep the trace, or is it followed by a renormalisation?
     dm = any(o is not None and (o.pair is not None or o.kind == "channel") for o in ops)
     trace_kept = False
@@ -538,7 +548,7 @@ def compile_ops(ops, nbits, mode="sweep", width=2, tile_bits=13, low_bits=None, 
             cur.append(o)
     segments.append(cur)
     fixed_segs = tuple(bool(pad) and isinstance(seg, list) and len(seg) > 0 and max(len(o.bits) for o in seg) <= pad
-                       and all(ucache[id(o)] for o in seg) and _spreads(seg, nbits) for seg in segments)
+                       and all(ucache[id(o)] for o in seg) and _spreads(seg, spread, nbits) for seg in segments)
     key = None
     if device_fusion and mode != "gate" and ops and not any(o is not None and o.kind == "pauli_mix" for o in ops):
         flags = [ucache[id(o)] for o in ops if o is not None]

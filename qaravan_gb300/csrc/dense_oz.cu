@@ -47,9 +47,10 @@
 // as K-major core matrices (96 KB), where both operands are read by the MMAs; results
 // come back through that space for coalesced stores, or go straight to memory where a thread's
 // rows are runs of 128 bytes (no target among the three lowest bits: 19.2 to 17.8 ms at 25 qubits).
-// What bounds it: the integer instructions that split and reassemble; the products (4100 cycles a
-// tile, the first half overlapped with nothing) come next, memory last: the seven accumulators fill
-// tensor memory, so two tiles cannot be in flight.
+// What bounds it: the integer instructions that split and reassemble (24 qubits: ALU pipe 60 % busy, 2660
+// instructions a warp and tile of 20,100 cycles); the products (tensor pipe 17 %, the first half
+// overlapped with nothing) come next, memory (20 %) last: the seven accumulators fill tensor memory, so
+// two tiles cannot be in flight.
 // Measured, brickwork against the double-float sweeps: 17 qubits depth 20 1.00 to 0.80 ms, 20 qubits
 // depth 20 3.49 to 1.89 ms, 22 qubits depth 8 6.20 to 2.79 ms, 25 qubits depth 8 48.4 to 22.1 ms.
 #include "sweep_df.cuh"

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from qaravan_gb300 import _lib, workloads
-from qaravan_gb300.compiler import Op, fuse_fewest, fuse_frontier, fuse_symbolic
+from qaravan_gb300.compiler import Op, SymBlock, fuse_fewest, fuse_frontier, fuse_symbolic
 from qaravan_gb300.density_matrix import DensityMatrixSim
 from qaravan_gb300.statevector import circuit_ops, gates_to_ops
 

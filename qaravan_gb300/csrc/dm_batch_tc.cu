@@ -657,8 +657,8 @@ extern "C" size_t qgb_dm_batch_table_bytes(int ncirc, int npasses, int64_t nitem
     return table_layout(ncirc, npasses, nitems).total;
 }
 
-extern "C" int qgb_dm_batch_build(void* table, size_t table_bytes, const qgb_dm_circuit* circs, int ncirc,
-                                  const qgb_dm_pass* passes, int npasses, int items_per_pass) {
+static int batch_build(void* table, size_t table_bytes, const qgb_dm_circuit* circs, int ncirc,
+                       const qgb_dm_pass* passes, int npasses, int items_per_pass) {
     using qgb_host::set_error;
     int rc = check_tables(circs, ncirc, passes, npasses, items_per_pass);
     if (rc) return rc;
@@ -732,6 +732,11 @@ extern "C" int qgb_dm_batch_build(void* table, size_t table_bytes, const qgb_dm_
             P[p].tail_items = count[size_t(passes[p].tslot)];
         }
     return w == nitems ? QGB_OK : set_error(QGB_EINVAL, "item count mismatch");
+}
+
+extern "C" int qgb_dm_batch_build(void* table, size_t table_bytes, const qgb_dm_circuit* circs, int ncirc,
+                                  const qgb_dm_pass* passes, int npasses, int items_per_pass) {
+    return qgb_host::guarded([&] { return batch_build(table, table_bytes, circs, ncirc, passes, npasses, items_per_pass); });
 }
 
 extern "C" size_t qgb_dm_batch_work_bytes(int ncirc, int64_t nitems) {

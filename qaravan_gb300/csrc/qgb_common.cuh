@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <exception>
 
 #include "../../include/qgb.h"
 
@@ -206,6 +207,15 @@ int allow_smem(F* kern, size_t bytes, std::atomic<uint64_t>& done, const char* w
         return check_launch(what);
     done.fetch_or(bit, std::memory_order_relaxed);
     return QGB_OK;
+}
+// A C entry's body: host allocations that fail become an error code (nothing has been launched by then).
+template <typename F>
+int guarded(F&& body) {
+    try {
+        return body();
+    } catch (const std::exception&) {
+        return set_error(QGB_EINVAL, "out of host memory");
+    }
 }
 // Internal status (never returned through the C ABI): a specialised kernel
 // declines an op, and the caller runs the general kernel instead.

@@ -1091,15 +1091,19 @@ extern "C" int qgb_inner_product(const void* a, const void* b, int dtype, int n,
 extern "C" int qgb_pauli_expectation(const void* sv, int dtype, int n, const char* paulis, const double* coeff,
                                      int nterms, int64_t batch, int64_t sv_stride, double* out, void* scratch,
                                      size_t scratch_bytes, void* stream) {
-    return pauli_expect_impl(sv, dtype, n, paulis, coeff, nterms, batch, sv_stride, out, scratch, scratch_bytes, false,
-                             (cudaStream_t)stream);
+    return guarded([&] {
+        return pauli_expect_impl(sv, dtype, n, paulis, coeff, nterms, batch, sv_stride, out, scratch, scratch_bytes, false,
+                                 (cudaStream_t)stream);
+    });
 }
 
 extern "C" int qgb_dm_pauli_expectation(const void* rho, int dtype, int n, const char* paulis, const double* coeff,
                                         int nterms, int64_t batch, int64_t rho_stride, double* out, void* scratch,
                                         size_t scratch_bytes, void* stream) {
-    return pauli_expect_impl(rho, dtype, n, paulis, coeff, nterms, batch, rho_stride, out, scratch, scratch_bytes, true,
-                             (cudaStream_t)stream);
+    return guarded([&] {
+        return pauli_expect_impl(rho, dtype, n, paulis, coeff, nterms, batch, rho_stride, out, scratch, scratch_bytes, true,
+                                 (cudaStream_t)stream);
+    });
 }
 
 extern "C" size_t qgb_partial_overlap_scratch_bytes(int n, int k, int64_t batch) {
@@ -1238,8 +1242,8 @@ extern "C" int qgb_dm_trace_factor(const void* rho, int dtype, int n, double* ch
     return check_launch("dm trace factor");
 }
 
-extern "C" int qgb_pauli_apply(const void* sv, void* out, int dtype, int n, const char* paulis, const double* coeff,
-                               int nterms, int64_t batch, int64_t sv_stride, void* stream) {
+static int pauli_apply_impl(const void* sv, void* out, int dtype, int n, const char* paulis, const double* coeff,
+                            int nterms, int64_t batch, int64_t sv_stride, void* stream) {
     int rc = check_common(sv, dtype, n, batch, sv_stride);
     if (rc) return rc;
     if (!out || !coeff) return set_error(QGB_EINVAL, "null pointer");
@@ -1275,8 +1279,13 @@ extern "C" int qgb_pauli_apply(const void* sv, void* out, int dtype, int n, cons
     }
     if (bx > cap) bx = cap;
     dim3 grid((unsigned)bx, (unsigned)batch);
-     pauli_apply_kernel<<<grid, 256, 0, st>>>((const double2*)sv, (double2*)out, sv_stride, a);
+    pauli_apply_kernel<<<grid, 256, 0, st>>>((const double2*)sv, (double2*)out, sv_stride, a);
     return check_launch("pauli apply");
+}
+
+extern "C" int qgb_pauli_apply(const void* sv, void* out, int dtype, int n, const char* paulis, const double* coeff,
+                               int nterms, int64_t batch, int64_t sv_stride, void* stream) {
+    return guarded([&] { return pauli_apply_impl(sv, out, dtype, n, paulis, coeff, nterms, batch, sv_stride, stream); });
 }
 
 namespace {

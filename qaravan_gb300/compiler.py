@@ -28,7 +28,6 @@ site ``q`` is bit ``n-1-q``.
 from __future__ import annotations
 
 import functools
-import itertools
 import os
 from dataclasses import dataclass, field
 
@@ -222,22 +221,28 @@ def _native_blocks(method, ops, width):
     N = len(ops)
     if not N:
         return []
-    begin = np.zeros(N + 1, dtype=np.int32)
-    np.cumsum([len(op.bits) for op in ops], out=begin[1:])
-    wide = int(np.max(np.diff(begin)))
+    begin, bits, wide = [0], [], 0
+    for op in ops:
+        bits.extend(op.bits)
+        begin.append(len(bits))
+        wide = max(wide, begin[-1] - begin[-2])
     if wide > width:
         raise ValueError(f"op on {wide} bits exceeds fusion width {width}")
-    bits = np.fromiter(itertools.chain.from_iterable(op.bits for op in ops), dtype=np.int32, count=int(begin[N]))
-    order, starts = np.empty(N, dtype=np.int32), np.empty(N + 1, dtype=np.int32)
-    sets, sizes = np.empty((N, width), dtype=np.int32), np.empty(N, dtype=np.int32)
-    if not os.path.exists(_lib._build.LIB):
+    if _lib._lib is None and not os.path.exists(_lib._build.LIB):
         _lib._build.build()
-    n = _lib.lib().qgb_plan_blocks(method, begin.ctypes.data, bits.ctypes.data, N, width, order.ctypes.data,
-                                   starts.ctypes.data, sets.ctypes.data, sizes.ctypes.data)
+    # one buffer: begin | bits | ops | block begins | block bits | block sizes
+    at = np.cumsum([0, N + 1, len(bits), N, N + 1, N * width]).tolist()
+    buf = np.empty(at[-1] + N, dtype=np.int32)
+    buf[:at[1]] = begin
+    buf[at[1]:at[2]] = bits
+    base = buf.ctypes.data
+    n = _lib.lib().qgb_plan_blocks(method, base, base + 4 * at[1], N, width, base + 4 * at[2], base + 4 * at[3],
+                                   base + 4 * at[4], base + 4 * at[5])
     if n < 0:
         _lib.check(n, "plan_blocks")
-    order, starts, sets, sizes = order.tolist(), starts[:n + 1].tolist(), sets[:n].tolist(), sizes[:n].tolist()
-    return [SymBlock(sets[j][:sizes[j]], order[starts[j]:starts[j + 1]]) for j in range(n)]
+    order, starts = buf[at[2]:at[3]].tolist(), buf[at[3]:at[3] + n + 1].tolist()
+    sets, sizes = buf[at[4]:at[4] + n * width].tolist(), buf[at[5]:at[5] + n].tolist()
+    return [SymBlock(sets[j * width:j * width + sizes[j]], order[starts[j]:starts[j + 1]]) for j in range(n)]
 
 
 def fuse_symbolic(ops, width):

@@ -3,7 +3,7 @@
 // No counterpart in the reference, which applies gate by gate (core/base_sim.py:30-53).
 // Native because a new circuit pays for it before its first launch: with the planner in Python a
 // compilation took 14 ms for 28 qubits at depth 20, 23 ms for a noisy 13-site circuit and 327 ms for 5000 random
-// pairs, more than the passes that the frontier blocks save in one run; now 3.4, 3.1 and 38 ms.
+// pairs, more than the passes that the frontier blocks save in one run; now 2.6, 2.6 and 32 ms.
 #include <algorithm>
 #include <cstdint>
 #include <exception>

@@ -227,7 +227,7 @@ def c128_roofline(plan, n, ms, double_float, peaks):
     from qaravan_gb300.compiler import plan_flops
     flops64 = plan_flops(plan)[1] * 2 ** n  # 8 per complex multiply-add
     out = {"tflops_fp64_equivalent": round(flops64 / (ms / 1e3) / 1e12, 3)}
-    if double_float and plan.steps and all(getattr(s, "fixed", False) for s in plan.steps):
+    if double_float and any(getattr(s, "fixed", False) for s in plan.steps):
         peak, kind = _peaks()
         achieved = 2 * 16 * 2 ** n * len(plan.steps) / (ms / 1e3) / 1e9
         out["arithmetic"] = "fixed point, 9-bit digits on the tensor cores; double-float where that is less accurate"

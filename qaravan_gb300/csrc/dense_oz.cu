@@ -38,8 +38,9 @@
 // rounded is then as large as what is summed). The other outputs are formed in
 // double-float from the staged tile, the products with nonzero entries of the block only,
 // as the tile sweeps form them (sweep_df.cu), while the MMAs run. The certificate costs 6 % of a
-// pass; recomputed outputs, in passes that meet product-like rows, up to four times the pass: 25
-// qubits depth 8 17.8 ms without either, 18.9 with the certificate, 22.1 in all.
+// pass; recomputed outputs, in passes that meet product-like rows and in narrow blocks, up to the
+// pass once more: 25 qubits depth 8 17.8 ms without either, 18.9 with the certificate, 22.1 in all
+// (20.3 with the last narrow blocks in a tile sweep, compiler._narrow_tail).
 //
 // Data path per CTA (one per SM, 16 warps): a tile is 4096 amplitudes (64 KB: the 5
 // target bits and the 7 lowest others), copied by cp.async one tile ahead; four
@@ -52,7 +53,7 @@
 // overlapped with nothing) come next, memory (20 %) last: the seven accumulators fill tensor memory, so
 // two tiles cannot be in flight.
 // Measured, brickwork against the double-float sweeps: 17 qubits depth 20 1.00 to 0.80 ms, 20 qubits
-// depth 20 3.49 to 1.89 ms, 22 qubits depth 8 6.20 to 2.79 ms, 25 qubits depth 8 48.4 to 22.1 ms.
+// depth 20 3.49 to 1.89 ms, 22 qubits depth 8 6.20 to 2.79 ms, 25 qubits depth 8 48.4 to 20.3 ms.
 #include "sweep_df.cuh"
 #include "tc_common.cuh"
 

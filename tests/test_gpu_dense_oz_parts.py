@@ -153,3 +153,19 @@ def test_circuits_by_default(kind):
             t = np.moveaxis(t.reshape([2] * n), range(k), g.indices).reshape(-1)
             x, b = (t, b) if what == 0 else (x, t)
     assert np.all(np.abs(got - x).astype(float) <= 6 * BOUND * b)
+
+
+@pytest.mark.parametrize("n,depth", [(19, 4), (20, 20), (22, 3)])
+def test_passes_and_the_sweep_behind_them(n, depth):
+    """Whole circuits with a narrow tail against float64 sweeps: below 1e-13 of the norm (double-float sweeps
+    leave 5e-14 after such circuits, the passes less)."""
+    from qaravan_gb300 import StatevectorSim
+    circ = workloads.brickwork_circuit(n, depth, 3)
+    L = _lib.lib()
+    _lib.check(L.qgb_set_c128_arith(0))
+    try:
+        want = StatevectorSim(circ, dtype=torch.complex128, mode="sweep", fusion_width=3, tile_bits=13).run()
+    finally:
+        _lib.check(L.qgb_set_c128_arith(1))
+    got = StatevectorSim(circ, dtype=torch.complex128).run()
+    assert torch.linalg.vector_norm(got - want).item() < 1e-13
